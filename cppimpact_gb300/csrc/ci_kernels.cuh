@@ -149,44 +149,78 @@ struct Rule<10> {
   }
 };
 
+// Sums of products with their rounding written out (RN): left to the compiler, which product
+// of a sum is fused differs from kernel to kernel, and the step kernels have to give the
+// same bits on the same plan.  RN false leaves it to the compiler (k_step_t10, whose results
+// no other kernel has to reproduce).
+template <bool RN>
+__device__ __forceinline__ float sub2f(float a, float b, float c, float d) {  // a b - c d
+  return RN ? __fmaf_rn(a, b, -__fmul_rn(c, d)) : a * b - c * d;
+}
+template <bool RN>
+__device__ __forceinline__ float dot3f(float a, float b, float c, float d, float e, float f) {
+  return RN ? __fmaf_rn(e, f, __fmaf_rn(a, b, __fmul_rn(c, d))) : a * b + c * d + e * f;
+}
+template <bool RN>
+__device__ __forceinline__ float mulf(float a, float b) {
+  return RN ? __fmul_rn(a, b) : a * b;
+}
+template <bool RN>
+__device__ __forceinline__ float maddf(float a, float b, float c) {  // a b + c
+  return RN ? __fmaf_rn(a, b, c) : a * b + c;
+}
+
 // Cofactor inverse of a 3x3 (row-major), returns det (cf. inv3x3, include/physics.h:38-58).
+template <bool RN = true>
 __device__ __forceinline__ float inv3f(const float* A, float* Ai) {
-  const float c00 = A[4] * A[8] - A[5] * A[7];
-  const float c01 = A[5] * A[6] - A[3] * A[8];
-  const float c02 = A[3] * A[7] - A[4] * A[6];
-  const float det = A[0] * c00 + A[1] * c01 + A[2] * c02;
+  const float c00 = sub2f<RN>(A[4], A[8], A[5], A[7]);
+  const float c01 = sub2f<RN>(A[5], A[6], A[3], A[8]);
+  const float c02 = sub2f<RN>(A[3], A[7], A[4], A[6]);
+  const float det = dot3f<RN>(A[0], c00, A[1], c01, A[2], c02);
   const float r = __frcp_rn(det);
-  Ai[0] = c00 * r;
-  Ai[1] = (A[2] * A[7] - A[1] * A[8]) * r;
-  Ai[2] = (A[1] * A[5] - A[2] * A[4]) * r;
-  Ai[3] = c01 * r;
-  Ai[4] = (A[0] * A[8] - A[2] * A[6]) * r;
-  Ai[5] = (A[2] * A[3] - A[0] * A[5]) * r;
-  Ai[6] = c02 * r;
-  Ai[7] = (A[1] * A[6] - A[0] * A[7]) * r;
-  Ai[8] = (A[0] * A[4] - A[1] * A[3]) * r;
+  Ai[0] = mulf<RN>(c00, r);
+  Ai[1] = mulf<RN>(sub2f<RN>(A[2], A[7], A[1], A[8]), r);
+  Ai[2] = mulf<RN>(sub2f<RN>(A[1], A[5], A[2], A[4]), r);
+  Ai[3] = mulf<RN>(c01, r);
+  Ai[4] = mulf<RN>(sub2f<RN>(A[0], A[8], A[2], A[6]), r);
+  Ai[5] = mulf<RN>(sub2f<RN>(A[2], A[3], A[0], A[5]), r);
+  Ai[6] = mulf<RN>(c02, r);
+  Ai[7] = mulf<RN>(sub2f<RN>(A[1], A[6], A[0], A[7]), r);
+  Ai[8] = mulf<RN>(sub2f<RN>(A[0], A[4], A[1], A[3]), r);
   return det;
+}
+
+// s0 + lambda tr + 2 mu de
+template <bool RN = true>
+__device__ __forceinline__ float trial_axial(const ElemParams& p, float s0, float tr, float de) {
+  return RN ? __fmaf_rn(2.f * p.mu, de, __fmaf_rn(p.lambda, tr, s0))
+            : s0 + p.lambda * tr + 2.f * p.mu * de;
 }
 
 // J2 radial return with linear isotropic hardening (Simo & Hughes 1998, Box 3.1):
 // trial = s + lambda tr(de) I + 2 mu de (engineering shear in de[3..5]); if the
 // deviatoric norm exceeds sqrt(2/3)(sy0 + H epbar), return along the deviator.
+template <bool RN = true>
 __device__ __forceinline__ void j2_return(const ElemParams& p, float s[6], float& epbar) {
-  const float pm = (s[0] + s[1] + s[2]) * (1.0f / 3.0f);
+  const float pm = mulf<RN>(s[0] + s[1] + s[2], 1.0f / 3.0f);
   const float d0 = s[0] - pm, d1 = s[1] - pm, d2 = s[2] - pm;
-  const float nrm2 = d0 * d0 + d1 * d1 + d2 * d2 + 2.f * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
+  const float nrm2 =
+      RN ? __fmaf_rn(2.f, dot3f<true>(s[3], s[3], s[4], s[4], s[5], s[5]),
+                     dot3f<true>(d0, d0, d1, d1, d2, d2))
+         : d0 * d0 + d1 * d1 + d2 * d2 + 2.f * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
   const float nrm = sqrtf(nrm2);
-  const float f = nrm - 0.81649658092772603f * (p.sy0 + p.H * epbar);
+  const float y = maddf<RN>(p.H, epbar, p.sy0);
+  const float f = RN ? __fmaf_rn(-0.81649658092772603f, y, nrm) : nrm - 0.81649658092772603f * y;
   if (f > 0.f) {
-    const float dg = f / (2.f * p.mu + (2.f / 3.f) * p.H);
-    const float sc = 1.f - 2.f * p.mu * dg / nrm;
-    s[0] = d0 * sc + pm;
-    s[1] = d1 * sc + pm;
-    s[2] = d2 * sc + pm;
-    s[3] *= sc;
-    s[4] *= sc;
-    s[5] *= sc;
-    epbar += 0.81649658092772603f * dg;
+    const float dg = f / maddf<RN>(2.f / 3.f, p.H, 2.f * p.mu);
+    const float sc = 1.f - mulf<RN>(2.f * p.mu, dg) / nrm;
+    s[0] = maddf<RN>(d0, sc, pm);
+    s[1] = maddf<RN>(d1, sc, pm);
+    s[2] = maddf<RN>(d2, sc, pm);
+    s[3] = mulf<RN>(s[3], sc);
+    s[4] = mulf<RN>(s[4], sc);
+    s[5] = mulf<RN>(s[5], sc);
+    epbar = maddf<RN>(0.81649658092772603f, dg, epbar);
   }
 }
 
@@ -242,15 +276,15 @@ __device__ __forceinline__ void element_force(const ElemParams& p, const DevStat
     for (int a = 0; a < 3; a++)
 #pragma unroll
       for (int b = 0; b < 3; b++)
-        L[3 * a + b] = Gu[3 * a + 0] * Ji[0 * 3 + b] + Gu[3 * a + 1] * Ji[1 * 3 + b] +
-                       Gu[3 * a + 2] * Ji[2 * 3 + b];
+        L[3 * a + b] = dot3f<true>(Gu[3 * a + 0], Ji[0 * 3 + b], Gu[3 * a + 1], Ji[1 * 3 + b],
+                             Gu[3 * a + 2], Ji[2 * 3 + b]);
     const float de[6] = {L[0], L[4], L[8], L[1] + L[3], L[5] + L[7], L[2] + L[6]};
     const float tr = de[0] + de[1] + de[2];
     float s[6];
     if (MODE == EM_REFCOMPAT) {
-      s[0] = p.lambda * tr + 2.f * p.mu * de[0];
-      s[1] = p.lambda * tr + 2.f * p.mu * de[1];
-      s[2] = p.lambda * tr + 2.f * p.mu * de[2];
+      s[0] = __fmaf_rn(p.lambda, tr, __fmul_rn(2.f * p.mu, de[0]));
+      s[1] = __fmaf_rn(p.lambda, tr, __fmul_rn(2.f * p.mu, de[1]));
+      s[2] = __fmaf_rn(p.lambda, tr, __fmul_rn(2.f * p.mu, de[2]));
       s[3] = p.mu * de[3];
       s[4] = p.mu * de[4];
       s[5] = p.mu * de[5];
@@ -266,12 +300,12 @@ __device__ __forceinline__ void element_force(const ElemParams& p, const DevStat
       const float2 sb = S.sig_b[qi];
       float ep = S.epbar[qi];
       const float s0[6] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y};
-      s[0] = s0[0] + p.lambda * tr + 2.f * p.mu * de[0];
-      s[1] = s0[1] + p.lambda * tr + 2.f * p.mu * de[1];
-      s[2] = s0[2] + p.lambda * tr + 2.f * p.mu * de[2];
-      s[3] = s0[3] + p.mu * de[3];
-      s[4] = s0[4] + p.mu * de[4];
-      s[5] = s0[5] + p.mu * de[5];
+      s[0] = trial_axial(p, s0[0], tr, de[0]);
+      s[1] = trial_axial(p, s0[1], tr, de[1]);
+      s[2] = trial_axial(p, s0[2], tr, de[2]);
+      s[3] = __fmaf_rn(p.mu, de[3], s0[3]);
+      s[4] = __fmaf_rn(p.mu, de[4], s0[4]);
+      s[5] = __fmaf_rn(p.mu, de[5], s0[5]);
       const float ep0 = ep;
       j2_return(p, s, ep);
       S.sig_a[qi] = make_float4(s[0], s[1], s[2], s[3]);
@@ -292,8 +326,8 @@ __device__ __forceinline__ void element_force(const ElemParams& p, const DevStat
     for (int a = 0; a < 3; a++)
 #pragma unroll
       for (int j = 0; j < 3; j++)
-        Pm[3 * a + j] = wd * (Sg[3 * a + 0] * Ji[3 * j + 0] + Sg[3 * a + 1] * Ji[3 * j + 1] +
-                              Sg[3 * a + 2] * Ji[3 * j + 2]);
+        Pm[3 * a + j] = __fmul_rn(wd, dot3f<true>(Sg[3 * a + 0], Ji[3 * j + 0], Sg[3 * a + 1],
+                                            Ji[3 * j + 1], Sg[3 * a + 2], Ji[3 * j + 2]));
 #pragma unroll
     for (int i = 0; i < NPE; i++)
 #pragma unroll
@@ -529,6 +563,26 @@ __device__ __forceinline__ ChunkStep chunk_step(const FusedArgs& A, const ChunkI
   return c;
 }
 
+// The wall: a screen in FP32 at a node's new displacement uf (d0f the rounded distance of
+// its reference position), false only where the node is clear of the plane:
+// |d32 - d| <= 2^-22 (|d0| + |u|_1) for |n_k| <= 1, and 1e-6 (1 + ...) covers it.
+__device__ __forceinline__ bool wall_near(const NodeParams& p, float d0f, const float (&uf)[3]) {
+  const float d32 = __fadd_rn(d0f, __fadd_rn(__fmul_rn(p.nf[0], uf[0]),
+                                  __fadd_rn(__fmul_rn(p.nf[1], uf[1]), __fmul_rn(p.nf[2], uf[2]))));
+  const float margin = 1e-6f * (1.f + fabsf(d0f) + fabsf(uf[0]) + fabsf(uf[1]) + fabsf(uf[2]));
+  return !(d32 > margin);
+}
+
+// Its FP64 distance, and for a penetrating node (d < 0) the push along the normal.
+__device__ __forceinline__ double wall_distance(const NodeParams& p, double d0,
+                                                const double (&un)[3]) {
+  return __fma_rn(p.wall_n[2], un[2], __fma_rn(p.wall_n[1], un[1], __fma_rn(p.wall_n[0], un[0], d0)));
+}
+
+__device__ __forceinline__ double wall_push(const NodeParams& p, double d, float m) {
+  return __ddiv_rn(__dmul_rn(-d, p.wall_k), (double)m);
+}
+
 // One node's central-difference update from its total internal force f.
 // u, v: in S^n, out S^{n+1}; a: the acceleration applied.  Rounding is explicit (no
 // contraction freedom), so every chunk that updates the same boundary node gets the
@@ -551,18 +605,13 @@ __device__ __forceinline__ void node_step(const NodeParams& p, float fx, float f
     un[k] = __fma_rn(p.dt, v[k], u[k]);
     uf[k] = f64_to_f32(un[k]);
   }
-  // |d32 - d| <= 2^-22 (|d0| + |u|_1) for |n_k| <= 1; 1e-6 (1 + ...) covers it
-  const float d32 = __fadd_rn(d0f, __fadd_rn(__fmul_rn(p.nf[0], uf[0]),
-                                  __fadd_rn(__fmul_rn(p.nf[1], uf[1]), __fmul_rn(p.nf[2], uf[2]))));
-  const float margin = 1e-6f * (1.f + fabsf(d0f) + fabsf(uf[0]) + fabsf(uf[1]) + fabsf(uf[2]));
   in_contact = false;
   double ad[3] = {f32_to_f64(a[0]), f32_to_f64(a[1]), f32_to_f64(a[2])};
-  if (!(d32 > margin)) {
-    const double d = __fma_rn(p.wall_n[2], un[2], __fma_rn(p.wall_n[1], un[1],
-                              __fma_rn(p.wall_n[0], un[0], d0[g])));
+  if (wall_near(p, d0f, uf)) {
+    const double d = wall_distance(p, d0[g], un);
     if (d < 0.0) {
       in_contact = true;
-      const double c = __ddiv_rn(__dmul_rn(-d, p.wall_k), (double)m);
+      const double c = wall_push(p, d, m);
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         ad[k] = __fma_rn(c, p.wall_n[k], ad[k]);
@@ -1039,6 +1088,93 @@ __device__ __forceinline__ void tet10_rs_slot(const Tet10QP& t, const float (&Pm
   R[K] = (even ? m0 : m1) + __shfl_xor_sync(0xffffffffu, even ? m1 : m0, 1);
 }
 
+// One Gauss point of a four-lane element (lane q = tid & 3): kinematics from the ten node
+// records, the stress update from the stored stress (s4, s2: xx yy zz xy, yz xz) and
+// plastic strain ep0, which an active lane passes updated to put(), the work terms, and in
+// keep the element force on the nodes this lane owns (q, q + 4 and, for q < 2, q + 8).
+template <int MODE, class Put>
+__device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& t, int q,
+                                           const Tile& T, const int (&ln)[10], bool act, float4 s4,
+                                           float2 s2, float ep0, unsigned* status, float& wint,
+                                           float& wp, float (&keep)[3][3], Put put) {
+  constexpr float W = 1.0f / 24.0f;
+  float2 JG[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) JG[k] = make_float2(0.f, 0.f);
+  tet10_gather<0>(t, T, ln[0], JG);
+  tet10_gather<1>(t, T, ln[1], JG);
+  tet10_gather<2>(t, T, ln[2], JG);
+  tet10_gather<3>(t, T, ln[3], JG);
+  tet10_gather<4>(t, T, ln[4], JG);
+  tet10_gather<5>(t, T, ln[5], JG);
+  tet10_gather<6>(t, T, ln[6], JG);
+  tet10_gather<7>(t, T, ln[7], JG);
+  tet10_gather<8>(t, T, ln[8], JG);
+  tet10_gather<9>(t, T, ln[9], JG);
+  float J[9], Gu[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    J[k] = JG[k].x;
+    Gu[k] = JG[k].y;
+  }
+  float Ji[9];
+  const float detJ = inv3f(J, Ji);
+  if (act && !(detJ > 0.f)) atomicOr(status, (unsigned)ST_DEGENERATE);
+  const float wd = act ? W * detJ : 0.f;
+  float Lg[9];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+      Lg[3 * a + b] = dot3f<true>(Gu[3 * a + 0], Ji[0 * 3 + b], Gu[3 * a + 1], Ji[1 * 3 + b],
+                            Gu[3 * a + 2], Ji[2 * 3 + b]);
+  const float de[6] = {Lg[0], Lg[4], Lg[8], Lg[1] + Lg[3], Lg[5] + Lg[7], Lg[2] + Lg[6]};
+  const float tr = de[0] + de[1] + de[2];
+  const float s0[6] = {s4.x, s4.y, s4.z, s4.w, s2.x, s2.y};
+  float s[6];
+  s[0] = trial_axial(ep, s0[0], tr, de[0]);
+  s[1] = trial_axial(ep, s0[1], tr, de[1]);
+  s[2] = trial_axial(ep, s0[2], tr, de[2]);
+  s[3] = __fmaf_rn(ep.mu, de[3], s0[3]);
+  s[4] = __fmaf_rn(ep.mu, de[4], s0[4]);
+  s[5] = __fmaf_rn(ep.mu, de[5], s0[5]);
+  float epn = ep0;
+  if (MODE == EM_J2) {
+    j2_return(ep, s, epn);
+    if (act) put(make_float4(s[0], s[1], s[2], s[3]), make_float2(s[4], s[5]), epn);
+  }
+  if (ep.accum_energy && act) {
+    float wq = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; k++) wq = fmaf(s0[k] + s[k], de[k], wq);
+    wint = fmaf(0.5f * wd, wq, wint);
+    if (MODE == EM_J2) wp = fmaf(wd * (ep.sy0 + ep.H * epn), epn - ep0, wp);
+  }
+  const float Sg[9] = {s[0], s[3], s[5], s[3], s[1], s[4], s[5], s[4], s[2]};
+  float Pm[9];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      Pm[3 * a + j] = __fmul_rn(wd, dot3f<true>(Sg[3 * a + 0], Ji[3 * j + 0], Sg[3 * a + 1],
+                                          Ji[3 * j + 1], Sg[3 * a + 2], Ji[3 * j + 2]));
+  {
+    float R[9];
+    const bool lo = q < 2, even = (q & 1) == 0;
+    tet10_rs_slot<0>(t, Pm, lo, even, R);
+    tet10_rs_slot<1>(t, Pm, lo, even, R);
+    tet10_rs_slot<2>(t, Pm, lo, even, R);
+    tet10_rs_slot<3>(t, Pm, lo, even, R);
+    tet10_rs_slot<4>(t, Pm, lo, even, R);
+    tet10_rs_slot<5>(t, Pm, lo, even, R);
+    tet10_rs_slot<6>(t, Pm, lo, even, R);
+    tet10_rs_slot<7>(t, Pm, lo, even, R);
+    tet10_rs_slot<8>(t, Pm, lo, even, R);
+#pragma unroll
+    for (int k = 0; k < 9; k++) keep[k / 3][k % 3] = R[k];
+  }
+}
+
 // Element loop of one chunk by the CTA's BS threads (4 lanes per element, colours
 // applied in order between barriers) into the tile's force accumulators; this thread's
 // internal and plastic work in wint, wp.  CG: the stored stress and plastic strain are
@@ -1053,7 +1189,6 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
   const DevPlan& P = A.P;
   const int q = tid & 3;
   const Tet10QP t = tet10_qp(q);
-  constexpr float W = 1.0f / 24.0f;
   const int E = P.E;
   wint = 0.f;
   wp = 0.f;
@@ -1088,86 +1223,13 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
     const int ee = act ? e : ch.elem_begin;
     const size_t qi = (size_t)ee * 4 + q;
     if (!PF) window_loads(w);
-    float2 JG[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) JG[k] = make_float2(0.f, 0.f);
-    tet10_gather<0>(t, T, ln[0], JG);
-    tet10_gather<1>(t, T, ln[1], JG);
-    tet10_gather<2>(t, T, ln[2], JG);
-    tet10_gather<3>(t, T, ln[3], JG);
-    tet10_gather<4>(t, T, ln[4], JG);
-    tet10_gather<5>(t, T, ln[5], JG);
-    tet10_gather<6>(t, T, ln[6], JG);
-    tet10_gather<7>(t, T, ln[7], JG);
-    tet10_gather<8>(t, T, ln[8], JG);
-    tet10_gather<9>(t, T, ln[9], JG);
-    float J[9], Gu[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      J[k] = JG[k].x;
-      Gu[k] = JG[k].y;
-    }
-    float Ji[9];
-    const float detJ = inv3f(J, Ji);
-    if (act && !(detJ > 0.f)) atomicOr(A.status, (unsigned)ST_DEGENERATE);
-    const float wd = act ? W * detJ : 0.f;
-    float Lg[9];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++)
-        Lg[3 * a + b] = Gu[3 * a + 0] * Ji[0 * 3 + b] + Gu[3 * a + 1] * Ji[1 * 3 + b] +
-                        Gu[3 * a + 2] * Ji[2 * 3 + b];
-    const float de[6] = {Lg[0], Lg[4], Lg[8], Lg[1] + Lg[3], Lg[5] + Lg[7], Lg[2] + Lg[6]};
-    const float tr = de[0] + de[1] + de[2];
-    const float s0[6] = {s4.x, s4.y, s4.z, s4.w, s2.x, s2.y};
-    float s[6];
-    s[0] = s0[0] + ep.lambda * tr + 2.f * ep.mu * de[0];
-    s[1] = s0[1] + ep.lambda * tr + 2.f * ep.mu * de[1];
-    s[2] = s0[2] + ep.lambda * tr + 2.f * ep.mu * de[2];
-    s[3] = s0[3] + ep.mu * de[3];
-    s[4] = s0[4] + ep.mu * de[4];
-    s[5] = s0[5] + ep.mu * de[5];
-    float epn = ep0;
-    if (MODE == EM_J2) {
-      j2_return(ep, s, epn);
-      if (act) {
-        A.sig_a[qi] = make_float4(s[0], s[1], s[2], s[3]);
-        A.sig_b[qi] = make_float2(s[4], s[5]);
-        A.epbar[qi] = epn;
-      }
-    }
-    if (ep.accum_energy && act) {
-      float wq = 0.f;
-#pragma unroll
-      for (int k = 0; k < 6; k++) wq = fmaf(s0[k] + s[k], de[k], wq);
-      wint = fmaf(0.5f * wd, wq, wint);
-      if (MODE == EM_J2) wp = fmaf(wd * (ep.sy0 + ep.H * epn), epn - ep0, wp);
-    }
-    const float Sg[9] = {s[0], s[3], s[5], s[3], s[1], s[4], s[5], s[4], s[2]};
-    float Pm[9];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int j = 0; j < 3; j++)
-        Pm[3 * a + j] = wd * (Sg[3 * a + 0] * Ji[3 * j + 0] + Sg[3 * a + 1] * Ji[3 * j + 1] +
-                              Sg[3 * a + 2] * Ji[3 * j + 2]);
     float keep[3][3];
-    {
-      float R[9];
-      const bool lo = q < 2, even = (q & 1) == 0;
-      tet10_rs_slot<0>(t, Pm, lo, even, R);
-      tet10_rs_slot<1>(t, Pm, lo, even, R);
-      tet10_rs_slot<2>(t, Pm, lo, even, R);
-      tet10_rs_slot<3>(t, Pm, lo, even, R);
-      tet10_rs_slot<4>(t, Pm, lo, even, R);
-      tet10_rs_slot<5>(t, Pm, lo, even, R);
-      tet10_rs_slot<6>(t, Pm, lo, even, R);
-      tet10_rs_slot<7>(t, Pm, lo, even, R);
-      tet10_rs_slot<8>(t, Pm, lo, even, R);
-#pragma unroll
-      for (int k = 0; k < 9; k++) keep[k / 3][k % 3] = R[k];
-    }
+    qp10_point<MODE>(ep, t, q, T, ln, act, s4, s2, ep0, A.status, wint, wp, keep,
+                     [&](float4 a4, float2 a2, float epn) {
+                       A.sig_a[qi] = a4;
+                       A.sig_b[qi] = a2;
+                       A.epbar[qi] = epn;
+                     });
     // lane q owns nodes q, q+4 and (for q < 2) q+8
     const int own0 = q == 0 ? ln[0] : q == 1 ? ln[1] : q == 2 ? ln[2] : ln[3];
     const int own1 = q == 0 ? ln[4] : q == 1 ? ln[5] : q == 2 ? ln[6] : ln[7];
@@ -1673,7 +1735,7 @@ __device__ __forceinline__ void tet10_bary_element(const ElemParams& ep, const F
       Gu[3 * a + 2] = Cd[3][a] - Cd[2][a];
     }
     float Ji[9];
-    const float detJ = inv3f(J, Ji);
+    const float detJ = inv3f<false>(J, Ji);
     if (!(detJ > 0.f)) atomicOr(A.status, (unsigned)ST_DEGENERATE);
     const float wd = W * detJ;
     float Lg[9];
@@ -1681,8 +1743,8 @@ __device__ __forceinline__ void tet10_bary_element(const ElemParams& ep, const F
     for (int a = 0; a < 3; a++)
 #pragma unroll
       for (int b = 0; b < 3; b++)
-        Lg[3 * a + b] = Gu[3 * a + 0] * Ji[0 * 3 + b] + Gu[3 * a + 1] * Ji[1 * 3 + b] +
-                        Gu[3 * a + 2] * Ji[2 * 3 + b];
+        Lg[3 * a + b] = dot3f<false>(Gu[3 * a + 0], Ji[0 * 3 + b], Gu[3 * a + 1], Ji[1 * 3 + b],
+                              Gu[3 * a + 2], Ji[2 * 3 + b]);
     const float de[6] = {Lg[0], Lg[4], Lg[8], Lg[1] + Lg[3], Lg[5] + Lg[7], Lg[2] + Lg[6]};
     const float tr = de[0] + de[1] + de[2];
     float s[6];
@@ -1705,14 +1767,14 @@ __device__ __forceinline__ void tet10_bary_element(const ElemParams& ep, const F
       const float2 sb = A.sig_b[qi];
       const float ep0 = A.epbar[qi];
       const float s0[6] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y};
-      s[0] = s0[0] + ep.lambda * tr + 2.f * ep.mu * de[0];
-      s[1] = s0[1] + ep.lambda * tr + 2.f * ep.mu * de[1];
-      s[2] = s0[2] + ep.lambda * tr + 2.f * ep.mu * de[2];
+      s[0] = trial_axial<false>(ep, s0[0], tr, de[0]);
+      s[1] = trial_axial<false>(ep, s0[1], tr, de[1]);
+      s[2] = trial_axial<false>(ep, s0[2], tr, de[2]);
       s[3] = s0[3] + ep.mu * de[3];
       s[4] = s0[4] + ep.mu * de[4];
       s[5] = s0[5] + ep.mu * de[5];
       float epn = ep0;
-      j2_return(ep, s, epn);
+      j2_return<false>(ep, s, epn);
       A.sig_a[qi] = make_float4(s[0], s[1], s[2], s[3]);
       A.sig_b[qi] = make_float2(s[4], s[5]);
       A.epbar[qi] = epn;
@@ -1730,8 +1792,8 @@ __device__ __forceinline__ void tet10_bary_element(const ElemParams& ep, const F
       float Pr[3];  // row c of P
 #pragma unroll
       for (int j = 0; j < 3; j++)
-        Pr[j] = wd * (Sg[3 * c + 0] * Ji[3 * j + 0] + Sg[3 * c + 1] * Ji[3 * j + 1] +
-                      Sg[3 * c + 2] * Ji[3 * j + 2]);
+        Pr[j] = wd * dot3f<false>(Sg[3 * c + 0], Ji[3 * j + 0], Sg[3 * c + 1], Ji[3 * j + 1],
+                           Sg[3 * c + 2], Ji[3 * j + 2]);
       // Q_k = P g_k: Q_0 = P_0, Q_1 = P_1, Q_3 = P_2, Q_2 = -(P_0 + P_1 + P_2)
       const float Q[4] = {Pr[0], Pr[1], -(Pr[0] + Pr[1] + Pr[2]), Pr[2]};
       Sq[0][c] += Q[0];
