@@ -23,6 +23,7 @@
 #include "../../include/cppimpact_gb300.h"
 #include "ci_kernels.cuh"
 #include "ci_plan.h"
+#include "ci_resident.h"
 
 namespace ci {
 int set_last_error(int code, const char* msg);
@@ -102,6 +103,16 @@ struct Group {
   DBuf<ElemParams> inst_ep;
   DBuf<NodeParams> inst_np;
   DBuf<int> inst_nsteps, step_ctr;
+  // resident form of the step (ci_resident.cuh): kernel, entry lists, tagged slots, the
+  // order in which CTAs take chunks with its counter and the abort flag, the next tag
+  ResidentPick res;
+  DBuf<uint32_t> node_ent, node_slots;
+  DBuf<uint16_t> ent;
+  DBuf<int> slots;
+  DBuf<ResidentChunk> rchunks;
+  DBuf<float4> halo;      // [2][S]
+  DBuf<int> order, claim;  // claim[0] counter, claim[1] abort flag
+  unsigned tag = 1;
   ~Group() {
     if (graph) cudaGraphExecDestroy(graph);
     if (stream) cudaStreamDestroy(stream);
@@ -124,6 +135,10 @@ struct ci_batch {
 };
 
 namespace {
+
+// The group runs resident (the tet10 kernel has four lanes per element; the autotuner also
+// tries one, which runs from a graph).
+bool resident(const Group& G) { return G.res.kernel && (G.npe == 4 || G.elem_lanes == 4); }
 
 ElemParams make_ep(const ci_material& m, double dt) {
   ElemParams p{};
@@ -263,6 +278,8 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
     if (src[j] == j) uniq.push_back(j);
   }
   std::vector<Plan> built(n_inst);
+  std::vector<ResidentTables> tab(n_inst);  // of the resident form, if the group can have it
+  const bool may_reside = G.npe == 4 || G.elem_lanes == 4;
   std::vector<std::string> errs(n_inst);
   std::vector<char> ok(n_inst, 0);
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
@@ -274,6 +291,7 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
       ok[j] = build_plan(I.mesh.num_nodes, I.mesh.num_elements, I.mesh.nodes_per_element,
                          I.mesh.xloc, I.mesh.element_nodes, G.chunk_elements, G.chunk_nodes, kDefaultTargetCtas,
                          &built[j], &errs[j]);
+      if (ok[j] && may_reside) resident_tables(built[j], &tab[j]);
     }
   };
   if (n_thr <= 1) {
@@ -315,12 +333,16 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   std::vector<ElemParams> eps;
   std::vector<NodeParams> nps;
   std::vector<int> nsteps;
+  std::vector<int> chunk0;  // first chunk of every instance
+  int most_chunks = 0;      // of one instance
   long long s_off = 0, l_off = 0;
   slot_row.reserve(G.N + 1);
   G.max_steps = 0;
   for (size_t j = 0; j < plans.size(); j++) {
     const Plan& P = *plans[j];
     Inst& T = b->inst[G.insts[j]];
+    chunk0.push_back((int)chunks.size());
+    most_chunks = std::max(most_chunks, P.n_chunks);
     for (ChunkInfo c : P.chunks) {
       c.elem_begin += T.elem_off;
       c.elem_end += T.elem_off;
@@ -408,13 +430,130 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   CB_CUDA(G.step_ctr.alloc(1));
   CB_CUDA(G.peak.alloc(G.insts.size()));
   CB_CUDA(npe == 4 ? configure<4>((int)G.smem) : configure<10>((int)G.smem));
+  // the resident form, where one instance's chunks fit the GPU together
+  G.res = ResidentPick();
+  std::vector<ResidentChunk> rchunks;
+  if (may_reside) {
+    int at = 0;
+    for (size_t j = 0; j < n_inst; j++)
+      for (const ResidentChunk& c : tab[src[j]].chunks) {
+        rchunks.push_back({at, c.n_slots});
+        at += c.n_slots;
+      }
+    CB_CUDA(pick_resident(npe, false, true, chunks, rchunks, 0, most_chunks, b->device, &G.res));
+  }
+  if (G.res.kernel) {
+    ResidentTables all;
+    long long so = 0;
+    for (size_t j = 0; j < n_inst; j++) {
+      const ResidentTables& t = tab[src[j]];
+      all.node_ent.insert(all.node_ent.end(), t.node_ent.begin(), t.node_ent.end());
+      all.node_slots.insert(all.node_slots.end(), t.node_slots.begin(), t.node_slots.end());
+      all.ent.insert(all.ent.end(), t.ent.begin(), t.ent.end());
+      for (int sl : t.slots) all.slots.push_back(sl + (int)so);
+      so += plans[j]->slot_row[plans[j]->N];
+    }
+    // instances with the most work first, so that the last to end are short ones
+    std::vector<int> by(n_inst), order;
+    for (size_t j = 0; j < n_inst; j++) by[j] = (int)j;
+    chunk0.push_back(G.C);
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
+      return (long long)nsteps[x] * plans[x]->E > (long long)nsteps[y] * plans[y]->E;
+    });
+    for (int j : by)
+      for (int c = chunk0[j]; c < chunk0[j + 1]; c++) order.push_back(c);
+    CB_CUDA(G.node_ent.upload(all.node_ent, st));
+    CB_CUDA(G.node_slots.upload(all.node_slots, st));
+    CB_CUDA(G.ent.upload(all.ent, st));
+    CB_CUDA(G.slots.upload(all.slots, st));
+    CB_CUDA(G.rchunks.upload(rchunks, st));
+    CB_CUDA(G.order.upload(order, st));
+    CB_CUDA(G.claim.alloc(2));
+    CB_CUDA(G.halo.alloc(2 * (size_t)G.S));
+    CB_CUDA(cudaMemsetAsync(G.halo.p, 0, sizeof(float4) * 2 * (size_t)G.S, st));
+    G.tag = 1;
+    CB_CUDA(cudaStreamSynchronize(st));
+  }
   CB_CUDA(cudaStreamSynchronize(st));
+  return CI_OK;
+}
+
+// What a resident run records besides the final state: snapshot s is the state after
+// (s + 1) every steps (the last state of an instance that has ended), s < n_snaps.
+struct Snapshots {
+  int every = 0, n_snaps = 0;
+  float* snap = nullptr;
+  float* peak = nullptr;
+};
+
+constexpr int kResidentRound = 1 << 14;  // steps per launch: no chunk waits longer for a CTA
+
+// All instances' steps up to `total` in launches of the resident kernel, in place in
+// buffer A.
+int enqueue_resident(Group& G, int total, const Snapshots& sn) {
+  cudaStream_t st = G.stream;
+  const size_t N = G.N;
+  for (int step0 = 0; step0 < total; step0 += kResidentRound) {
+    const int k = std::min(kResidentRound, total - step0);
+    if (G.tag > ~0u - (unsigned)kResidentRound) {  // every tag used once: start over
+      CB_CUDA(cudaMemsetAsync(G.halo.p, 0, sizeof(float4) * 2 * (size_t)G.S, st));
+      G.tag = 1;
+    }
+    CB_CUDA(cudaMemsetAsync(G.claim.p, 0, 2 * sizeof(int), st));
+    const FusedArgs F = group_args(G, 0);
+    ResidentArgs A{};
+    A.P = F.P;
+    for (int c = 0; c < 3; c++) {
+      A.u[c] = G.ua.p + c * N;
+      A.v[c] = G.va.p + c * N;
+      A.acc[c] = G.acc.p + c * N;
+    }
+    A.halo[0] = G.halo.p;
+    A.halo[1] = G.halo.p + G.S;
+    A.mass = G.mass.p;
+    A.d0 = G.d0.p;
+    A.d0f = G.d0f.p;
+    A.contact = G.contact.p;
+    A.sig_a = G.sig_a.p;
+    A.sig_b = G.sig_b.p;
+    A.epbar = G.epbar.p;
+    A.chunk_work = G.work.p;
+    A.status = G.status.p;
+    A.rchunk = G.rchunks.p;
+    A.slots = G.slots.p;
+    A.node_slots = G.node_slots.p;
+    A.node_ent = G.node_ent.p;
+    A.ent = G.ent.p;
+    A.claim = G.claim.p;
+    A.abort_flag = G.claim.p + 1;
+    A.wait_ns = kFlowWaitNs;
+    A.tag0 = G.tag;
+    A.nsteps = k;
+    A.inst_ep = G.inst_ep.p;
+    A.inst_np = G.inst_np.p;
+    A.inst_nsteps = G.inst_nsteps.p;
+    A.order = G.order.p;
+    A.n_chunks = G.C;
+    A.step0 = step0;
+    A.every = std::max(1, sn.every);
+    A.snap_end = sn.n_snaps == 0               ? 0
+                 : step0 + kResidentRound >= total ? sn.n_snaps
+                                                   : std::min(sn.n_snaps, (step0 + k) / A.every);
+    A.snap_nodes = G.N;
+    A.snap = sn.snap;
+    A.peak = sn.peak;
+    G.tag += (unsigned)k;
+    void* args[] = {&A};
+    CB_CUDA(cudaLaunchCooperativeKernel(G.res.kernel, dim3(std::min(G.res.ctas, G.C)),
+                                        dim3(G.res.threads), args, G.res.smem, st));
+  }
   return CI_OK;
 }
 
 int capture_graph(Group& G) {
   if (G.graph) cudaGraphExecDestroy(G.graph);
   G.graph = nullptr;
+  if (resident(G)) return CI_OK;  // runs without one
   cudaGraph_t g = nullptr;
   CB_CUDA(cudaStreamBeginCapture(G.stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
@@ -494,6 +633,7 @@ int enqueue_run(Group& G, bool launch = true) {
   k_node_init<true><<<(G.N + 255) / 256, 256, 0, st>>>(A, np0, G.inst_np.p, G.node_inst.p,
                                                        G.d0f.p);
   CB_CUDA(cudaGetLastError());
+  if (launch && resident(G)) return enqueue_resident(G, G.max_steps, Snapshots());
   if (launch) {
     // all global steps: max_steps + 1 (the last instance's boundary finalisation)
     const int total = G.max_steps + 1;
@@ -520,9 +660,15 @@ int trial_shape(Group& G, int graphs, cudaEvent_t e0, cudaEvent_t e1, float* ms_
   int rc;
   if ((rc = capture_graph(G))) return rc;
   if ((rc = enqueue_run(G, false))) return rc;
-  CB_CUDA(cudaGraphLaunch(G.graph, G.stream));  // warm-up: uploads the graph
-  CB_CUDA(cudaEventRecord(e0, G.stream));
-  for (int r = 0; r < graphs; r++) CB_CUDA(cudaGraphLaunch(G.graph, G.stream));
+  if (resident(G)) {
+    if ((rc = enqueue_resident(G, kGraphSteps, Snapshots()))) return rc;  // warm-up
+    CB_CUDA(cudaEventRecord(e0, G.stream));
+    if ((rc = enqueue_resident(G, graphs * kGraphSteps, Snapshots()))) return rc;
+  } else {
+    CB_CUDA(cudaGraphLaunch(G.graph, G.stream));  // warm-up: uploads the graph
+    CB_CUDA(cudaEventRecord(e0, G.stream));
+    for (int r = 0; r < graphs; r++) CB_CUDA(cudaGraphLaunch(G.graph, G.stream));
+  }
   CB_CUDA(cudaEventRecord(e1, G.stream));
   CB_CUDA(cudaEventSynchronize(e1));
   float ms = 0.f;
@@ -531,6 +677,7 @@ int trial_shape(Group& G, int graphs, cudaEvent_t e0, cudaEvent_t e1, float* ms_
   CB_CUDA(cudaMemcpy(&st, G.status.p, sizeof(st), cudaMemcpyDeviceToHost));
   if (st & ST_DEGENERATE) return fail(CI_ERR_DEGENERATE, "an element has det J <= 0");
   if (st & ST_NONFINITE) return fail(CI_ERR_NONFINITE, "non-finite nodal state");
+  if (st & ST_FLOW_TIMEOUT) return fail(CI_ERR_CUDA, "a chunk waited longer than its time limit");
   *ms_per_step = ms / (float)(graphs * kGraphSteps);
   return CI_OK;
 }
@@ -742,13 +889,21 @@ int ci_batch_run(ci_batch* b, float* device_ms) {
   // both groups start after ev0 and end before ev1 (device time of the whole batch)
   cudaStream_t s0 = b->g[0] ? b->g[0]->stream : b->g[1]->stream;
   CB_CUDA(cudaEventRecord(b->ev0, s0));
+  std::vector<cudaEvent_t> ends;
   for (int gi = 0; gi < 2; gi++)
     if (b->g[gi]) {
       CB_CUDA(cudaStreamWaitEvent(b->g[gi]->stream, b->ev0, 0));
+      if (gi == 1 && b->g[0] && resident(*b->g[0]) && resident(*b->g[1])) {
+        // one resident group after the other: each wants the whole GPU
+        cudaEvent_t e;
+        CB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ends.push_back(e);
+        CB_CUDA(cudaEventRecord(e, b->g[0]->stream));
+        CB_CUDA(cudaStreamWaitEvent(b->g[1]->stream, e, 0));
+      }
       const int rc = enqueue_run(*b->g[gi]);
       if (rc) return rc;
     }
-  std::vector<cudaEvent_t> ends;
   for (int gi = 0; gi < 2; gi++)
     if (b->g[gi] && b->g[gi]->stream != s0) {
       cudaEvent_t e;
@@ -768,6 +923,7 @@ int ci_batch_run(ci_batch* b, float* device_ms) {
       CB_CUDA(cudaMemcpy(&st, b->g[gi]->status.p, sizeof(st), cudaMemcpyDeviceToHost));
       if (st & ST_DEGENERATE) return fail(CI_ERR_DEGENERATE, "an element has det J <= 0");
       if (st & ST_NONFINITE) return fail(CI_ERR_NONFINITE, "non-finite nodal state");
+      if (st & ST_FLOW_TIMEOUT) return fail(CI_ERR_CUDA, "a chunk waited longer than its time limit");
     }
   b->done = true;
   return CI_OK;
@@ -794,8 +950,8 @@ int ci_batch_get_state(ci_batch* b, int i, double* x, double* v, float* epbar,
   const Inst& T = b->inst[i];
   const Group& G = *b->g[T.group];
   const int N = T.N, E = T.E, nq = G.nq;
-  // final state in buffer A for an even step count, B for an odd one
-  const bool a = (T.nsteps & 1) == 0;
+  // final state in buffer A for an even step count (or a resident run), B for an odd one
+  const bool a = resident(G) || (T.nsteps & 1) == 0;
   std::vector<double> hu(3 * (size_t)N), hv(3 * (size_t)N);
   for (int k = 0; k < 3; k++) {
     CB_CUDA(cudaMemcpy(&hu[(size_t)k * N], (a ? G.ua.p : G.ub.p) + (size_t)k * G.N + T.node_off,
@@ -832,37 +988,49 @@ namespace {
 // tail(G) (kernels on G.stream, captured into the graph); the device time goes to
 // *device_ms.  One element type per batch.
 template <class Tail>
-int run_intervals(ci_batch* b, int every, float* device_ms, const char* what, Tail tail) {
+int run_intervals(ci_batch* b, int every, const Snapshots& sn, float* device_ms, const char* what,
+                  Tail tail) {
   if (b->g[0] && b->g[1])
     return fail(CI_ERR_UNSUPPORTED, std::string(what) + ": one element type per batch");
   CB_CUDA(cudaSetDevice(b->device));
   Group& G = *(b->g[0] ? b->g[0] : b->g[1]);
-  if (G.graph) cudaGraphExecDestroy(G.graph);
-  G.graph = nullptr;
-  cudaGraph_t g = nullptr;
-  CB_CUDA(cudaStreamBeginCapture(G.stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t err = cudaSuccess;
-  for (int i = 0; i < every && err == cudaSuccess; i++) {
-    const FusedArgs F = group_args(G, i);
-    err = G.npe == 4 ? launch_batch<4>(G, F) : launch_batch<10>(G, F);
-  }
-  if (err == cudaSuccess) {
-    k_tick<<<1, 1, 0, G.stream>>>(G.step_ctr.p, every);
-    tail(G);
-    err = cudaGetLastError();
-  }
-  cudaError_t e2 = cudaStreamEndCapture(G.stream, &g);
-  if (err != cudaSuccess || e2 != cudaSuccess)
-    return fail(CI_ERR_CUDA, std::string(what) + " capture: " +
-                                 cudaGetErrorString(err != cudaSuccess ? err : e2));
-  err = cudaGraphInstantiate(&G.graph, g, 0);
-  cudaGraphDestroy(g);
-  if (err != cudaSuccess) return fail(CI_ERR_CUDA, std::string(what) + " graph: " + cudaGetErrorString(err));
-  CB_CUDA(cudaEventRecord(b->ev0, G.stream));
-  // ceil((max_steps + 1) / every) graphs of `every` steps, prepared like a normal run
-  {
-    const int rc = enqueue_run_graph(G, G.max_steps + 1, every);
+  if (resident(G)) {
+    // every instance's last state counts for the snapshots up to the interval that holds
+    // step max_steps
+    CB_CUDA(cudaEventRecord(b->ev0, G.stream));
+    int rc = enqueue_run(G, false);
     if (rc) return rc;
+    Snapshots s = sn;
+    s.n_snaps = std::min(sn.n_snaps, G.max_steps / every + 1);
+    if ((rc = enqueue_resident(G, G.max_steps, s))) return rc;
+  } else {
+    if (G.graph) cudaGraphExecDestroy(G.graph);
+    G.graph = nullptr;
+    cudaGraph_t g = nullptr;
+    CB_CUDA(cudaStreamBeginCapture(G.stream, cudaStreamCaptureModeThreadLocal));
+    cudaError_t err = cudaSuccess;
+    for (int i = 0; i < every && err == cudaSuccess; i++) {
+      const FusedArgs F = group_args(G, i);
+      err = G.npe == 4 ? launch_batch<4>(G, F) : launch_batch<10>(G, F);
+    }
+    if (err == cudaSuccess) {
+      k_tick<<<1, 1, 0, G.stream>>>(G.step_ctr.p, every);
+      tail(G);
+      err = cudaGetLastError();
+    }
+    cudaError_t e2 = cudaStreamEndCapture(G.stream, &g);
+    if (err != cudaSuccess || e2 != cudaSuccess)
+      return fail(CI_ERR_CUDA, std::string(what) + " capture: " +
+                                   cudaGetErrorString(err != cudaSuccess ? err : e2));
+    err = cudaGraphInstantiate(&G.graph, g, 0);
+    cudaGraphDestroy(g);
+    if (err != cudaSuccess) return fail(CI_ERR_CUDA, std::string(what) + " graph: " + cudaGetErrorString(err));
+    CB_CUDA(cudaEventRecord(b->ev0, G.stream));
+    // ceil((max_steps + 1) / every) graphs of `every` steps, prepared like a normal run
+    {
+      const int rc = enqueue_run_graph(G, G.max_steps + 1, every);
+      if (rc) return rc;
+    }
   }
   CB_CUDA(cudaEventRecord(b->ev1, G.stream));
   CB_CUDA(cudaEventSynchronize(b->ev1));
@@ -874,6 +1042,7 @@ int run_intervals(ci_batch* b, int every, float* device_ms, const char* what, Ta
   unsigned int stw = 0;
   CB_CUDA(cudaMemcpy(&stw, G.status.p, sizeof(stw), cudaMemcpyDeviceToHost));
   if (stw & ST_NONFINITE) return fail(CI_ERR_NONFINITE, "non-finite nodal state");
+  if (stw & ST_FLOW_TIMEOUT) return fail(CI_ERR_CUDA, "a chunk waited longer than its time limit");
   b->done = true;
   return CI_OK;
 }
@@ -885,7 +1054,11 @@ extern "C" {
 int ci_batch_run_snapshots(ci_batch* b, int every, float* d_snap, int max_snaps, float* device_ms) {
   if (!b || every <= 0 || (every & 1) || !d_snap || max_snaps <= 0)
     return fail(CI_ERR_INVALID, "ci_batch_run_snapshots: needs an even interval and a buffer");
-  return run_intervals(b, every, device_ms, "ci_batch_run_snapshots", [&](Group& G) {
+  Snapshots sn;
+  sn.every = every;
+  sn.n_snaps = max_snaps;
+  sn.snap = d_snap;
+  return run_intervals(b, every, sn, device_ms, "ci_batch_run_snapshots", [&](Group& G) {
     k_snapshot<<<(G.N + 255) / 256, 256, 0, G.stream>>>(group_args(G, 0), group_args(G, 1),
                                                         G.node_inst.p, G.N, every, d_snap, max_snaps);
   });
@@ -895,7 +1068,11 @@ int ci_batch_run_peaks(ci_batch* b, int every, int max_snaps, float* peak_disp, 
                        float* device_ms) {
   if (!b || every <= 0 || (every & 1) || max_snaps <= 0)
     return fail(CI_ERR_INVALID, "ci_batch_run_peaks: needs an even interval");
-  int rc = run_intervals(b, every, device_ms, "ci_batch_run_peaks", [&](Group& G) {
+  Snapshots sn;
+  sn.every = every;
+  sn.n_snaps = max_snaps;
+  if (b->g[0] || b->g[1]) sn.peak = (b->g[0] ? b->g[0] : b->g[1])->peak.p;
+  int rc = run_intervals(b, every, sn, device_ms, "ci_batch_run_peaks", [&](Group& G) {
     k_snapshot_peak<<<(G.N + 255) / 256, 256, 0, G.stream>>>(group_args(G, 0), group_args(G, 1),
                                                              G.node_inst.p, G.N, every, max_snaps,
                                                              G.peak.p);

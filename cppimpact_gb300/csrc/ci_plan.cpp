@@ -282,6 +282,50 @@ int flow_lists(const Plan& P, std::vector<int>* own_row, std::vector<int>* own_i
   return longest;
 }
 
+void resident_chunks(const Plan& P, std::vector<ResidentChunk>* chunks) {
+  int begin = 0;
+  chunks->clear();
+  for (const ChunkInfo& ch : P.chunks) {
+    int n = 0;
+    for (int l = ch.n_int; l < ch.n_local; l++) {
+      const size_t lb = (size_t)ch.local_begin + l;
+      n += P.local_srow[2 * lb + 1] - P.local_srow[2 * lb];
+    }
+    chunks->push_back({begin, n});
+    begin += n;
+  }
+}
+
+void resident_tables(const Plan& P, ResidentTables* out) {
+  resident_chunks(P, &out->chunks);
+  out->node_ent.assign(P.local_gid.size(), 0u);
+  out->node_slots.assign(P.local_gid.size(), 0u);
+  out->ent.assign((size_t)P.npe * P.E, 0);
+  out->slots.clear();
+  std::vector<int> cur;
+  for (const ChunkInfo& ch : P.chunks) {
+    const int ne = ch.elem_end - ch.elem_begin;
+    cur.assign(ch.n_local + 1, 0);
+    for (int a = 0; a < P.npe; a++)
+      for (int i = 0; i < ne; i++) cur[P.conn_local[(size_t)a * P.E + ch.elem_begin + i] + 1]++;
+    for (int l = 0; l < ch.n_local; l++) {
+      out->node_ent[ch.local_begin + l] = (uint32_t)cur[l] | (uint32_t)cur[l + 1] << 16;
+      cur[l + 1] += cur[l];
+    }
+    uint16_t* e = out->ent.data() + (size_t)P.npe * ch.elem_begin;
+    for (int i = 0; i < ne; i++)
+      for (int a = 0; a < P.npe; a++)
+        e[cur[P.conn_local[(size_t)a * P.E + ch.elem_begin + i]]++] = (uint16_t)(a * ne + i);
+    const size_t begin = out->slots.size();
+    for (int l = ch.n_int; l < ch.n_local; l++) {
+      const size_t lb = (size_t)ch.local_begin + l;
+      const int s0 = P.local_srow[2 * lb], s1 = P.local_srow[2 * lb + 1];
+      out->node_slots[lb] = (uint32_t)(out->slots.size() - begin) | (uint32_t)(s1 - s0) << 16;
+      for (int s = s0; s < s1; s++) out->slots.push_back(s);
+    }
+  }
+}
+
 std::vector<int> flow_order(int C, const std::vector<int>& own_row, const std::vector<int>& own_idx) {
   // symmetric adjacency without self loops
   std::vector<std::vector<int>> adj(C);

@@ -76,6 +76,26 @@ int flow_lists(const Plan& P, std::vector<int>* own_row, std::vector<int>* own_i
 // one block of C tasks back in the claim order.
 std::vector<int> flow_order(int C, const std::vector<int>& own_row, const std::vector<int>& own_idx);
 
+// Tables of the resident step kernels.  Element entries of every local node: node_ent[local
+// entry] = begin | count << 16 into the chunk's part of ent (from npe * elem_begin on), whose
+// values are corner * (elements of the chunk) + element, elements in plan order (that is
+// colour order: a node has one element of a colour).  Slots of a chunk's boundary nodes
+// (local ids from n_int on), each node's in slot order: slots[slot_begin ...];
+// node_slots[local entry] = begin | count << 16 into the chunk's part.
+// Valid where npe * elements and n_slots of every chunk are at most 65535.
+struct ResidentChunk {
+  int slot_begin, n_slots;
+};
+struct ResidentTables {
+  std::vector<uint32_t> node_ent, node_slots;
+  std::vector<uint16_t> ent;
+  std::vector<int> slots;
+  std::vector<ResidentChunk> chunks;
+};
+// The chunks' slot counts only, then everything.
+void resident_chunks(const Plan& P, std::vector<ResidentChunk>* chunks);
+void resident_tables(const Plan& P, ResidentTables* out);
+
 // Host check of the plan invariants (used by tests through ci_plan_verify).
 bool verify_plan(const Plan& p, const int* conn, std::string* err);
 

@@ -1,0 +1,82 @@
+// ci_resident4.cu -- resident step kernels of tet4 meshes (ci_resident.cuh).
+#include <algorithm>
+
+#include "ci_resident.cuh"
+
+namespace ci {
+
+namespace {
+template <int MODE, bool BATCH>
+const void* pick(int threads, bool chip) {
+  if constexpr (BATCH)
+    if (threads == 32 && chip) return resident_fn<4, MODE, 32, true, BATCH>();
+  if (threads == 64 && chip) return resident_fn<4, MODE, 64, true, BATCH>();
+  if (threads == 128 && chip) return resident_fn<4, MODE, 128, true, BATCH>();
+  return nullptr;
+}
+}  // namespace
+
+const void* resident_kernel_tet4(bool refcompat, bool batch, int threads, bool chip) {
+  if (batch) return refcompat ? nullptr : pick<EM_J2, true>(threads, chip);
+  return refcompat ? pick<EM_REFCOMPAT, false>(threads, chip) : pick<EM_J2, false>(threads, chip);
+}
+
+}  // namespace ci
+
+namespace ci {
+
+const void* resident_kernel_tet10(bool refcompat, bool batch, int threads, bool chip);
+
+cudaError_t pick_resident(int npe, bool refcompat, bool batch, const std::vector<ChunkInfo>& chunks,
+                          const std::vector<ResidentChunk>& rchunks, int energy_threads,
+                          int need_ctas, int device, ResidentPick* out) {
+  *out = ResidentPick();
+  int smem_max = 0, sms = 0, coop = 0;
+  cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)))
+    return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) return e;
+  if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device))) return e;
+  if (!coop) return cudaSuccess;
+  const int lanes = npe == 10 ? 4 : 1;
+  int max_lanes = 0;  // threads that an element per thread (a point per thread) fills
+  for (const ChunkInfo& c : chunks) max_lanes = std::max(max_lanes, lanes * (c.elem_end - c.elem_begin));
+  for (const bool chip : {true, false})
+    for (const int threads : {32, 64, 128}) {
+      // few threads where they hold the chunk's elements in one pass: a barrier of one or two
+      // warps is cheaper and more chunks share an SM.  A single solve has SMs to spare and
+      // wants a warp for the elements and others for the nodes.
+      if (threads < 128 && max_lanes > (batch ? threads : threads / 2)) continue;
+      // the same work sums as the fused kernel's: its CTA size, or no thread of either with
+      // more than one element (further warps only add zeros)
+      if (energy_threads && threads != energy_threads && max_lanes > std::min(threads, energy_threads))
+        continue;
+      const void* fn = npe == 4 ? resident_kernel_tet4(refcompat, batch, threads, chip)
+                                : resident_kernel_tet10(refcompat, batch, threads, chip);
+      if (!fn) continue;
+      size_t smem = 0;
+      bool fits = true;
+      for (size_t i = 0; i < chunks.size(); i++) {
+        const ChunkInfo& c = chunks[i];
+        const int ne = c.elem_end - c.elem_begin, ns = rchunks[i].n_slots;
+        smem = std::max(smem, resident_smem(npe, c.n_local, ne, ns, chip));
+        fits = fits && npe * ne <= 65535 && ns <= 65535;  // 16-bit positions
+      }
+      if (!fits || (long long)smem + 2048 > smem_max) continue;
+      // one limit for every solver (a smaller one set later would refuse this one's launch)
+      if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 2048)))
+        return e;
+      int per_sm = 0;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem))) return e;
+      if ((long long)per_sm * sms < need_ctas) continue;
+      out->kernel = fn;
+      out->threads = threads;
+      out->on_chip = chip;
+      out->smem = smem;
+      out->ctas = per_sm * sms;
+      return cudaSuccess;
+    }
+  return cudaSuccess;
+}
+
+}  // namespace ci
