@@ -402,17 +402,16 @@ __global__ void __launch_bounds__(128, 1)
 // ---------------------------------------------------------------------------
 // Persistent form of the A B^T kernel: one CTA per SM walks the output tiles (grouped
 // raster: GM consecutive 128-row tiles share every BN-column tile, so the operand
-// panels in flight stay in L2).  Six warps with fixed roles:
+// panels in flight stay in L2).  Warps with fixed roles:
 //   warp 0  TMA producer: 128 x 64 and BN x 64 tiles into a TSTAGES-deep ring;
 //   warp 1  MMA issuer: tcgen05.mma into one of two TMEM accumulators (2 x BN columns),
 //           tcgen05.commit releases ring stages and, after a tile's last K step,
 //           hands the accumulator to the epilogue;
-//   warps 2-5  epilogue: TMEM lane quarter (warp % 4), tcgen05.ld, alpha / beta / bias /
-//           tanh, stores; then the accumulator goes back to the MMA issuer.
+//   warps 2..   epilogue (EPW warps): TMEM lane quarter (warp % 4), tcgen05.ld, alpha / beta / bias /
+//           tanh, stores (epi_store); then the accumulator goes back to the MMA issuer.
 // The epilogue of tile i overlaps the MMAs of tile i + 1.  Every wait is bounded; a role
 // that times out raises a shared abort flag so the others stop waiting, and the kernel
 // reports the error through *err.
-constexpr int PERS_THREADS = 192;
 constexpr int GROUP_M = 16;
 
 __device__ __forceinline__ bool mbar_wait_abort(uint32_t bar, uint32_t phase, volatile int* abort) {
@@ -431,6 +430,121 @@ __device__ __forceinline__ bool mbar_wait_abort(uint32_t bar, uint32_t phase, vo
   return false;
 }
 
+// Epilogue of 32 x 32 accumulators by one warp, turned through shared memory (buf, 32 rows
+// of EPI_LD floats): r holds lane's row, the stores go out row by row, 128 contiguous bytes
+// at a time (16-byte stores where C's rows allow it).  A lane storing its own row touches 32
+// sectors per instruction.  40,960 x 6,591 x 64, bound by its 1.08 GB of output (159 us at
+// the measured HBM rate): 1,356 -> 400 us, and with 6,592 columns 405 -> 231.  (Windows that
+// start on a sector or a line of each row, the rest carried in the buffer, measured 422 and
+// 452 us: the stores' own instructions then cost more than the parts of lines.)
+constexpr int EPI_LD = 36;
+
+__device__ __forceinline__ void epi_store(float* buf, const uint32_t (&r)[32], int row0, int M,
+                                          int col0, int N, float* C, int ldc, __nv_bfloat16* Cb,
+                                          float alpha, float beta, const float* __restrict__ bias,
+                                          int act, int lane) {
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    *reinterpret_cast<uint4*>(buf + lane * EPI_LD + 4 * j) =
+        make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+  __syncwarp();
+  const bool vec = col0 + 32 <= N && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(Cb) & 7) == 0;
+  if (vec) {
+    const int col = col0 + 4 * (lane & 7);
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias) b4 = make_float4(bias[col], bias[col + 1], bias[col + 2], bias[col + 3]);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int k = 4 * i + (lane >> 3), row = row0 + k;
+      const float4 t = *reinterpret_cast<const float4*>(buf + k * EPI_LD + 4 * (lane & 7));
+      if (row < M) {
+        const size_t at = (size_t)row * ldc + col;
+        float v[4] = {alpha * t.x, alpha * t.y, alpha * t.z, alpha * t.w};
+        if (beta != 0.f) {
+          const float4 c = *reinterpret_cast<const float4*>(C + at);
+          v[0] += beta * c.x;
+          v[1] += beta * c.y;
+          v[2] += beta * c.z;
+          v[3] += beta * c.w;
+        }
+        if (bias) {
+          v[0] += b4.x;
+          v[1] += b4.y;
+          v[2] += b4.z;
+          v[3] += b4.w;
+        }
+        if (act == 1)
+#pragma unroll
+          for (int j = 0; j < 4; j++) v[j] = tanhf(v[j]);
+        *reinterpret_cast<float4*>(C + at) = make_float4(v[0], v[1], v[2], v[3]);
+        if (Cb) {
+          __nv_bfloat162 lo, hi;
+          lo.x = __float2bfloat16(v[0]);
+          lo.y = __float2bfloat16(v[1]);
+          hi.x = __float2bfloat16(v[2]);
+          hi.y = __float2bfloat16(v[3]);
+          *reinterpret_cast<uint2*>(Cb + at) =
+              make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        }
+      }
+    }
+  } else {
+    const int col = col0 + lane;
+    const bool in = col < N;
+    const float bc = bias && in ? bias[col] : 0.f;
+    if (row0 + 32 <= M && beta == 0.f && act == 0 && !Cb) {  // whole block, C only
+      float* c = C + (size_t)row0 * ldc + col;
+#pragma unroll
+      for (int k0 = 0; k0 < 32; k0 += 16) {
+        float t[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) t[k] = buf[(k0 + k) * EPI_LD + lane];
+        if (in) {
+#pragma unroll
+          for (int k = 0; k < 16; k++) {
+            float v = alpha * t[k];
+            if (bias) v += bc;
+            *c = v;
+            c += ldc;
+          }
+        }
+      }
+    } else {
+#pragma unroll 8
+      for (int k = 0; k < 32; k++) {
+        const float t = buf[k * EPI_LD + lane];
+        const int row = row0 + k;
+        if (in && row < M) {
+          const size_t at = (size_t)row * ldc + col;
+          float v = alpha * t;
+          if (beta != 0.f) v += beta * C[at];
+          if (bias) v += bc;
+          if (act == 1) v = tanhf(v);
+          C[at] = v;
+          if (Cb) Cb[at] = __float2bfloat16(v);
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// 32 accumulator columns of this warp's TMEM lane quarter
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+      "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
+      "%30, %31}, [%32];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& mt, int& nt) {
   const int per_group = GROUP_M * tiles_n;
   const int g = t / per_group;
@@ -441,8 +555,8 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   nt = r / gm;
 }
 
-template <int BN>
-__global__ void __launch_bounds__(PERS_THREADS, 1)
+template <int BN, int STAGES, int EPW>
+__global__ void __launch_bounds__(64 + 32 * EPW, 1)
     k_gemm_tma_pers(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     float* C, int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha,
                     float beta, const float* __restrict__ bias, int act, int* err) {
@@ -453,8 +567,9 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + TSTAGES * A_BYTES;
-  __shared__ __align__(8) uint64_t full[TSTAGES], empty[TSTAGES], tfull[2], tempty[2];
+  uint8_t* sB = smem + STAGES * A_BYTES;
+  __shared__ __align__(16) float epi_buf[EPW][32 * EPI_LD];
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2];
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -470,13 +585,15 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   if (tid == 0) {
-    for (int s = 0; s < TSTAGES; s++) {
+    for (int s = 0; s < STAGES; s++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[s])) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[s])) : "memory");
     }
     for (int b = 0; b < 2; b++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tfull[b])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(smem_u32(&tempty[b])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&tempty[b])),
+                   "r"(EPW)
+                   : "memory");
     }
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -495,9 +612,9 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
         int mt, nt;
         tile_coords(t, tiles_m, tiles_n, mt, nt);
         for (int kt = 0; kt < ktiles; kt++, it++) {
-          const int s = (int)(it % TSTAGES);
-          if (it >= TSTAGES &&
-              !mbar_wait_abort(smem_u32(&empty[s]), (uint32_t)((it / TSTAGES) - 1) & 1u, abort)) {
+          const int s = (int)(it % STAGES);
+          if (it >= STAGES &&
+              !mbar_wait_abort(smem_u32(&empty[s]), (uint32_t)((it / STAGES) - 1) & 1u, abort)) {
             ok = false;
             break;
           }
@@ -525,8 +642,8 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t acc_tmem = tmem + (uint32_t)(b * BN);
         for (int kt = 0; kt < ktiles; kt++, it++) {
-          const int s = (int)(it % TSTAGES);
-          if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / TSTAGES) & 1u, abort)) {
+          const int s = (int)(it % STAGES);
+          if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) {
             ok = false;
             break;
           }
@@ -557,6 +674,9 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
     }
   } else {
     const int q = warp & 3;  // TMEM lanes 32 q .. 32 q + 31 (a warp's accessible quarter)
+    // its columns: all, or half of them where two warps share a quarter
+    constexpr int COLS = BN * 4 / EPW;
+    const int c_begin = (warp - 2) / 4 * COLS, c_end = c_begin + COLS;
     int j = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, j++) {
       const int b = j & 1;
@@ -567,48 +687,13 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       int mt, nt;
       tile_coords(t, tiles_m, tiles_n, mt, nt);
-      const int row = mt * BM + q * 32 + lane;
       const int n0 = nt * BN;
 #pragma unroll 1
-      for (int c = 0; c < BN; c += 16) {
-        uint32_t r[16];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-            "%11, %12, %13, %14, %15}, [%16];\n"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (row < M) {
-          float v[16];
-#pragma unroll
-          for (int jj = 0; jj < 16; jj++) {
-            const int col = n0 + c + jj;
-            v[jj] = alpha * __uint_as_float(r[jj]);
-            if (col < N) {
-              if (beta != 0.f) v[jj] += beta * C[(size_t)row * ldc + col];
-              if (bias) v[jj] += bias[col];
-              if (act == 1) v[jj] = tanhf(v[jj]);
-            }
-          }
-          float* crow = C + (size_t)row * ldc + n0 + c;
-          if (n0 + c + 16 <= N && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
-#pragma unroll
-            for (int k4 = 0; k4 < 4; k4++)
-              reinterpret_cast<float4*>(crow)[k4] =
-                  make_float4(v[4 * k4], v[4 * k4 + 1], v[4 * k4 + 2], v[4 * k4 + 3]);
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 16; jj++)
-              if (n0 + c + jj < N) crow[jj] = v[jj];
-          }
-          if (Cb)
-#pragma unroll
-            for (int jj = 0; jj < 16; jj++)
-              if (n0 + c + jj < N) Cb[(size_t)row * ldc + n0 + c + jj] = __float2bfloat16(v[jj]);
-        }
+      for (int c = c_begin; c < c_end && n0 + c < N; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c), r);
+        epi_store(epi_buf[warp - 2], r, mt * BM + q * 32, M, n0 + c, N, C, ldc, Cb, alpha, beta,
+                  bias, act, lane);
       }
       // this warp's quarter of the accumulator is read: hand it back to the MMA issuer
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -622,8 +707,8 @@ __global__ void __launch_bounds__(PERS_THREADS, 1)
   if (!ok) {
     // let the TMA loads still in flight land before the shared memory goes away
     if (warp == 0 && lane == 0)
-      for (long long it = issued > TSTAGES ? issued - TSTAGES : 0; it < issued; it++)
-        mbar_wait(smem_u32(&full[it % TSTAGES]), (uint32_t)(it / TSTAGES) & 1u);
+      for (long long it = issued > STAGES ? issued - STAGES : 0; it < issued; it++)
+        mbar_wait(smem_u32(&full[it % STAGES]), (uint32_t)(it / STAGES) & 1u);
     if (tid == 0) atomicExch(err, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -697,9 +782,9 @@ bool make_tile_map(CUtensorMap* map, const void* base, int rows, int K, int ld, 
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
+template <int BN, int STAGES = TSTAGES>
 constexpr int tma_smem_bytes() {
-  return TSTAGES * (BM * TBK * 2 + BN * TBK * 2) + 1024;
+  return STAGES * (BM * TBK * 2 + BN * TBK * 2) + 1024;
 }
 
 template <int BN>
@@ -730,24 +815,40 @@ int num_sms() {
   return n[dev] > 0 ? n[dev] : 1;
 }
 
-template <int BN>
-cudaError_t launch_tma_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t st, float* C,
-                            int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha,
-                            float beta, const float* bias, int act, int* err) {
+// The output of a tile takes as long to write as its products to compute at K of about 650
+// (128 x 256 FP32 at an SM's share of HBM against its tensor cores); up to 512 the kernel is
+// a stream of stores, and eight epilogue warps (with a ring of three stages to make room for
+// their buffers) keep more of them going than four.
+constexpr int kShortK = 512;
+
+template <int BN, int STAGES, int EPW>
+cudaError_t launch_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t st, float* C,
+                        int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha, float beta,
+                        const float* bias, int act, int* err) {
   static bool configured[64] = {};
+  constexpr int smem = tma_smem_bytes<BN, STAGES>();
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     const cudaError_t e = cudaFuncSetAttribute(
-        k_gemm_tma_pers<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem_bytes<BN>());
+        k_gemm_tma_pers<BN, STAGES, EPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = std::min(tiles, num_sms());
-  k_gemm_tma_pers<BN><<<grid, PERS_THREADS, tma_smem_bytes<BN>(), st>>>(
+  k_gemm_tma_pers<BN, STAGES, EPW><<<grid, 64 + 32 * EPW, smem, st>>>(
       ta, tb, C, ldc, Cb, M, N, K, alpha, beta, bias, act, err);
   return cudaGetLastError();
+}
+
+template <int BN>
+cudaError_t launch_tma_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t st, float* C,
+                            int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha,
+                            float beta, const float* bias, int act, int* err) {
+  return K <= kShortK ? launch_pers<BN, 3, 8>(ta, tb, st, C, ldc, Cb, M, N, K, alpha, beta, bias, act, err)
+                      : launch_pers<BN, TSTAGES, 4>(ta, tb, st, C, ldc, Cb, M, N, K, alpha, beta,
+                                                    bias, act, err);
 }
 
 // Tiny products (the plastic-strain network's 64-wide layers) on the CUDA cores: one

@@ -82,8 +82,8 @@ def gemm(A, B, transA=False, transB=False, out=None, out_bf16=None, beta=0.0):
     M = A.shape[1] if transA else A.shape[0]
     K = A.shape[0] if transA else A.shape[1]
     N = B.shape[0] if transB else B.shape[1]
-    if out is None:
-        out = torch.zeros((M, N), dtype=torch.float32, device=A.device)
+    if out is None:   # every entry is written; beta C reads zeros
+        out = (torch.zeros if beta else torch.empty)((M, N), dtype=torch.float32, device=A.device)
     err = torch.zeros(1, dtype=torch.int32, device=A.device)
     api.check(api.lib().ci_gemm_bf16(A.data_ptr(), A.shape[1], int(transA), B.data_ptr(), B.shape[1],
                                      int(transB), out.data_ptr(), out.shape[1],
