@@ -7,7 +7,19 @@
 // is written for the next layer.  This is the dense contraction of the surrogate (POD
 // projections and the MLP's forward/backward passes); the impact step itself has none.
 //
-// One CTA computes a 128 x BN tile (BN = 64 or 128).  Per K-tile of 64:
+// The kernels read both operands K-major (A B^T) by TMA (cp.async.bulk.tensor, 128-byte
+// swizzle): 128 x 64 and BN x 64 tiles through a shared-memory ring, one thread issuing the
+// loads, one the tcgen05.mma, mbarriers handing stages back and forth (full: TMA bytes
+// landed; empty: the MMAs reading a stage completed), accumulators in TMEM:
+//   k_gemm_tma_pers  one CTA per SM walking the output tiles, two TMEM accumulators so the
+//                    epilogue of one tile overlaps the MMAs of the next
+//   k_gemm_stream    a long A past a narrow B: equal unit ranges per SM, rows off 16-byte
+//                    boundaries in classes
+//   k_gemm_tma       split K (few output tiles, long K): one CTA per (tile, K range)
+// Operands that TMA cannot read (another transpose, rows off 16-byte boundaries) are copied
+// (k_pack_bf16) or, in k_gemm_stream's A, read in place.  What the copies do not cover (see
+// choose_operands) goes through k_gemm_bf16: one CTA computes a 128 x BN tile (BN = 64 or
+// 128).  Per K-tile of 64:
 //  1. all 128 threads stage A (128 x 64) and B (BN x 64) as K-major BF16 in shared
 //     memory, in the canonical no-swizzle layout of 8-row x 16-byte core matrices
 //     (core matrix (r/8, k/8) at r/8 * SBO + k/8 * LBO, LBO = 128 B, SBO = 1024 B);
@@ -16,17 +28,8 @@
 //     and commits to an mbarrier;
 //  3. every thread waits on the mbarrier (bounded spin: on timeout the kernel records
 //     an error flag, frees its TMEM and returns) before the stage is overwritten.
-// The epilogue reads the accumulator with tcgen05.ld (each warp its 32 TMEM lanes =
-// 32 rows), applies alpha, beta, bias, tanh and stores.
-//
-// C = A B^T with both operands K-major (transA = 0, transB = 1), M >= 128 and aligned
-// rows takes a pipelined kernel instead: TMA (cp.async.bulk.tensor, 128-byte swizzle)
-// streams 128 x 64 and BN x 64 tiles through a 4-stage shared-memory ring, one thread
-// issues the TMA loads, one thread the MMAs, and mbarriers hand stages back and forth
-// (full: TMA bytes landed; empty: the MMAs reading a stage completed).  Without split-K
-// that kernel is persistent (k_gemm_tma_pers: one CTA per SM walking the tiles, two
-// TMEM accumulators so the epilogue of one tile overlaps the MMAs of the next); with
-// split-K (few output tiles, long K) it runs one CTA per (tile, K range).
+// The epilogues read the accumulator with tcgen05.ld (each warp its 32 TMEM lanes =
+// 32 rows), apply alpha, beta, bias, tanh and store.
 #include <cuda.h>  // CUtensorMap and its enums; the encoder is fetched at run time
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -718,6 +721,366 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
                  : "memory");
 }
 
+// ---------------------------------------------------------------------------
+// C = A B^T for products that stream a long A past a narrow B (N <= 256: the POD's sketch,
+// projection and Gram products), bound by reading A once.
+//
+// Work split: the (tile, 64-deep K step) units of all tiles in one line, cut into one equal
+// range per SM, so no SM waits for a last wave; a tile cut by a range end goes to FP32 partial
+// sums that k_stream_reduce adds in K order (deterministic).  6,591 x 96 x 81,920, 1.1 GB (162 us
+// at the measured HBM rate): 249-253 us with 312 CTAs of a sixth of K each on 152 SMs, 196 so.
+//
+// Rows that TMA cannot address (lda not a multiple of 8, or A off a 16-byte boundary): rows
+// r = p i + c of one class c (p = 8 / gcd(lda, 8) classes) are a matrix whose row stride p lda
+// is a multiple of 8, from the 16-byte boundary at or before row c; its rows then start delta_c
+// elements into the tile.  B comes packed once per class, delta_c zeros in front, so the
+// products line up; the delta_c elements in front of A's rows (the end of another row) are
+// zeroed in shared memory before the first K step's MMAs, so that an infinity or a NaN there
+// stays with its own row.  81,920 x 96 x 6,591: 2,711-2,760 us with element-wise staging, 238 so (163 us at the measured HBM
+// rate).
+//
+// Accuracy: the tensor core's FP32 sums lose about 1.1e-9 of the result per product in a chain
+// (measured: 7.3e-6 after 6,591, 2.9e-5 after 28,000; here 4.7e-7 for either).  A chain here is kChain K steps (512
+// products); the epilogue warps add the chains' sums in registers, rounded to nearest, while
+// the next chain runs in the other accumulator.
+constexpr int kChain = 8;
+constexpr int kMaxClasses = 8;
+
+struct StreamMaps {
+  CUtensorMap a[kMaxClasses];  // [c] rows of class c
+  CUtensorMap b;               // [classes with a copy of B][N] rows
+};
+
+struct StreamArgs {
+  float* C;
+  __nv_bfloat16* Cb;
+  const float* bias;
+  float* partial;  // [2 gridDim.x][BN / 4][128] float4
+  int* err;
+  int ldc, M, N;
+  float alpha, beta;
+  int act;
+  int p, b_copies;         // classes; 1 or p copies of B
+  int delta[kMaxClasses];  // elements in front of the rows of a class
+  int tm, tn, kt;          // row tiles per class, column tiles, K steps
+};
+
+// Unit range of CTA b of g: [units b / g, units (b + 1) / g)
+__host__ __device__ __forceinline__ long long stream_begin(long long units, int b, int g) {
+  return units * b / g;
+}
+
+__device__ __forceinline__ void stream_tile(const StreamArgs& P, int t, int& c, int& mt, int& nt) {
+  c = t / (P.tm * P.tn);
+  const int r = t - c * P.tm * P.tn;
+  mt = r / P.tn;
+  nt = r - mt * P.tn;
+}
+
+template <int BN, int STAGES, int EPW>
+__global__ void __launch_bounds__(64 + 32 * EPW, 1)
+    k_gemm_stream(const __grid_constant__ StreamMaps maps, const __grid_constant__ StreamArgs P) {
+  constexpr int A_BYTES = BM * TBK * 2;
+  constexpr int B_BYTES = BN * TBK * 2;
+  constexpr uint32_t TCOLS = 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + STAGES * A_BYTES;
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2];
+  __shared__ __align__(16) float epi_buf[EPW][32 * EPI_LD];
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long long units = (long long)P.p * P.tm * P.tn * P.kt;
+  const long long u0 = stream_begin(units, blockIdx.x, gridDim.x);
+  const long long u1 = stream_begin(units, blockIdx.x + 1, gridDim.x);
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                     smem_u32(&tmem_base)),
+                 "r"(TCOLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[s])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[s])) : "memory");
+    }
+    for (int b = 0; b < 2; b++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tfull[b])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&tempty[b])),
+                   "r"(EPW)
+                   : "memory");
+    }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = tmem_base;
+  volatile int* abort = &abort_flag;
+  bool ok = true;
+  long long issued = 0;
+  if (warp == 0) {
+    if (lane == 0) {
+      long long it = 0;
+      for (long long u = u0; u < u1 && ok;) {
+        const int t = (int)(u / P.kt), k0 = (int)(u - (long long)t * P.kt);
+        const int k1 = (int)min((long long)P.kt, k0 + (u1 - u));
+        int c, mt, nt;
+        stream_tile(P, t, c, mt, nt);
+        const int brow = (P.b_copies > 1 ? c * P.N : 0) + nt * BN;
+        for (int k = k0; k < k1; k++, it++) {
+          const int s = (int)(it % STAGES);
+          if (it >= STAGES &&
+              !mbar_wait_abort(smem_u32(&empty[s]), (uint32_t)((it / STAGES) - 1) & 1u, abort)) {
+            ok = false;
+            break;
+          }
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
+                           smem_u32(&full[s])),
+                       "r"(A_BYTES + B_BYTES)
+                       : "memory");
+          tma_load_2d(smem_u32(sA + s * A_BYTES), &maps.a[c], k * TBK, mt * BM, smem_u32(&full[s]));
+          tma_load_2d(smem_u32(sB + s * B_BYTES), &maps.b, k * TBK, brow, smem_u32(&full[s]));
+          issued = it + 1;
+        }
+        u += k1 - k0;
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = instr_desc(BM, BN);
+    long long it = 0;
+    int j = 0;
+    for (long long u = u0; u < u1 && ok;) {
+      const int t = (int)(u / P.kt), k0 = (int)(u - (long long)t * P.kt);
+      const int k1 = (int)min((long long)P.kt, k0 + (u1 - u));
+      int c, mt, nt;
+      stream_tile(P, t, c, mt, nt);
+      const int delta = P.delta[c];
+      for (int kc = k0; kc < k1 && ok; kc += kChain, j++) {
+        const int b = j & 1;
+        if (j >= 2 && !mbar_wait_abort(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t acc_tmem = tmem + (uint32_t)(b * BN);
+        const int ke = min(k1, kc + kChain);
+        for (int k = kc; k < ke; k++, it++) {
+          const int s = (int)(it % STAGES);
+          // every lane waits, so that the masking below is ordered after the TMA write
+          if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) ok = false;
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          uint8_t* const a = sA + s * A_BYTES;
+          if (k == 0 && delta > 0) {
+            // elements 0 .. delta - 1 of every row: 16-byte chunk 0, at chunk (row % 8) of the
+            // swizzled row
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const int row = lane + 32 * i;
+              uint16_t* e = reinterpret_cast<uint16_t*>(a + row * 128 + ((row & 7) << 4));
+              for (int x = 0; x < delta; x++) e[x] = 0;
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+          }
+          if (lane == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+            for (int kk = 0; kk < TBK / 16; kk++) {
+              const uint64_t da = desc_sw128(smem_u32(a) + kk * 32);
+              const uint64_t db = desc_sw128(smem_u32(sB + s * B_BYTES) + kk * 32);
+              const uint32_t acc = (k > kc || kk > 0) ? 1u : 0u;
+              asm volatile(
+                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc_tmem),
+                  "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                  : "memory");
+            }
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                    smem_u32(&empty[s]))
+                : "memory");
+          }
+          __syncwarp();
+        }
+        if (ok && lane == 0)
+          asm volatile(
+              "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                  smem_u32(&tfull[b]))
+              : "memory");
+      }
+      if (!ok) break;
+      u += k1 - k0;
+    }
+  } else {
+    const int q = warp & 3;
+    constexpr int COLS = BN * 4 / EPW;  // this warp's columns
+    const int c_begin = (warp - 2) / 4 * COLS;
+    int j = 0;
+    for (long long u = u0; u < u1 && ok;) {
+      const int t = (int)(u / P.kt), k0 = (int)(u - (long long)t * P.kt);
+      const int k1 = (int)min((long long)P.kt, k0 + (u1 - u));
+      int c, mt, nt;
+      stream_tile(P, t, c, mt, nt);
+      float sum[COLS];
+      for (int kc = k0; kc < k1; kc += kChain, j++) {
+        const int b = j & 1;
+        if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+        for (int n = 0; n < COLS; n += 32) {
+          uint32_t r[32];
+          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            sum[n + i] = kc == k0 ? __uint_as_float(r[i]) : sum[n + i] + __uint_as_float(r[i]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&tempty[b]))
+                       : "memory");
+      }
+      if (!ok) break;
+      const int n0 = nt * BN + c_begin;
+      const int rows_c = (P.M - c + P.p - 1) / P.p;  // rows of the class
+      const bool whole = k0 == 0 && k1 == P.kt;
+      float4* part = reinterpret_cast<float4*>(P.partial) +
+                     ((size_t)(2 * blockIdx.x + (u == u0 ? 0 : 1)) * (BN / 4) + c_begin / 4) * 128;
+#pragma unroll
+      for (int n = 0; n < COLS; n += 32) {
+        if (n0 + n >= P.N) break;
+        if (whole) {
+          uint32_t r[32];
+#pragma unroll
+          for (int i = 0; i < 32; i++) r[i] = __float_as_uint(sum[n + i]);
+          epi_store(epi_buf[warp - 2], r, mt * BM + q * 32, rows_c, n0 + n, P.N,
+                    P.C + (size_t)c * P.ldc, P.p * P.ldc,
+                    P.Cb ? P.Cb + (size_t)c * P.ldc : nullptr, P.alpha, P.beta, P.bias, P.act, lane);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            part[(size_t)(n / 4 + i) * 128 + q * 32 + lane] = make_float4(
+                sum[n + 4 * i], sum[n + 4 * i + 1], sum[n + 4 * i + 2], sum[n + 4 * i + 3]);
+        }
+      }
+      u += k1 - k0;
+    }
+  }
+  ok = __syncthreads_and(ok) != 0;
+  if (!ok) {
+    // let the TMA loads still in flight land before the shared memory goes away
+    if (warp == 0 && lane == 0)
+      for (long long it = issued > STAGES ? issued - STAGES : 0; it < issued; it++)
+        mbar_wait(smem_u32(&full[it % STAGES]), (uint32_t)(it / STAGES) & 1u);
+    if (tid == 0) atomicExch(P.err, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS)
+                 : "memory");
+}
+
+// The tiles that range ends cut: their partial sums in K order (four contiguous runs of them by
+// four warps, then the runs in order), then the epilogue.  Block (tile, 4 columns, 32 rows).
+__global__ void __launch_bounds__(128) k_stream_reduce(const StreamArgs P, int BN, int g) {
+  __shared__ float4 run[4][32];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = blockIdx.z * 32 + lane;
+  const long long units = (long long)P.p * P.tm * P.tn * P.kt;
+  const long long ut = (long long)t * P.kt;
+  const int b0 = (int)(((ut + 1) * g - 1) / units), b1 = (int)(((ut + P.kt) * g - 1) / units);
+  if (b0 == b1) return;  // one CTA had the whole tile
+  const float4* part = reinterpret_cast<const float4*>(P.partial) + (size_t)blockIdx.y * 128 + row;
+  const int per = (b1 - b0 + 4) / 4, lo = b0 + w * per, hi = min(b1 + 1, lo + per);
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int b = lo; b < hi; b++) {
+    const int slot = 2 * b + (stream_begin(units, b, g) >= ut ? 0 : 1);
+    const float4 v = part[(size_t)slot * (BN / 4) * 128];
+    s.x += v.x;
+    s.y += v.y;
+    s.z += v.z;
+    s.w += v.w;
+  }
+  run[w][lane] = s;
+  __syncthreads();
+  int c, mt, nt;
+  stream_tile(P, t, c, mt, nt);
+  const int i = mt * BM + row, col = nt * BN + 4 * blockIdx.y;
+  if (w > 0 || i >= (P.M - c + P.p - 1) / P.p || col >= P.N) return;
+  for (int k = 1; k < 4; k++) {
+    const float4 v = run[k][lane];
+    s.x += v.x;
+    s.y += v.y;
+    s.z += v.z;
+    s.w += v.w;
+  }
+  const float acc[4] = {s.x, s.y, s.z, s.w};
+  const size_t at = ((size_t)i * P.p + c) * P.ldc + col;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (col + j >= P.N) break;
+    float v = P.alpha * acc[j];
+    if (P.beta != 0.f) v += P.beta * P.C[at + j];
+    if (P.bias) v += P.bias[col + j];
+    if (P.act == 1) v = tanhf(v);
+    P.C[at + j] = v;
+    if (P.Cb) P.Cb[at + j] = __float2bfloat16(v);
+  }
+}
+
+// Operand copies that TMA can address: out [copies][rows][ld] with ld a multiple of 8 (the
+// columns up to ld zero), copy c shifted by delta[c] zeros; the source [rows x K], or
+// [K x rows] when trans.  32 x 32 tiles through shared memory, so both sides are read and
+// written along their rows.
+struct PackArgs {
+  const __nv_bfloat16* in;
+  __nv_bfloat16* out;
+  int rows, K, ld_in, trans, ld;
+  int delta[kMaxClasses];
+};
+
+__global__ void __launch_bounds__(256) k_pack_bf16(const PackArgs P) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  const int d = P.delta[blockIdx.z];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const __nv_bfloat16 zero = __float2bfloat16(0.f);
+  __nv_bfloat16* out = P.out + (size_t)blockIdx.z * P.rows * P.ld;
+  const int r0 = blockIdx.y * 32;
+  for (int x0 = blockIdx.x * 128; x0 < min(P.ld, (int)(blockIdx.x + 1) * 128); x0 += 32) {
+    if (P.trans) {
+      for (int k = ty; k < 32; k += 8) {
+        const int x = x0 + k - d, r = r0 + tx;
+        tile[k][tx] = (x >= 0 && x < P.K && r < P.rows) ? P.in[(size_t)x * P.ld_in + r] : zero;
+      }
+      __syncthreads();
+      for (int k = ty; k < 32; k += 8)
+        if (r0 + k < P.rows && x0 + tx < P.ld) out[(size_t)(r0 + k) * P.ld + x0 + tx] = tile[tx][k];
+      __syncthreads();
+    } else {
+      for (int k = ty; k < 32; k += 8) {
+        const int x = x0 + tx - d, r = r0 + k;
+        if (r < P.rows && x0 + tx < P.ld)
+          out[(size_t)r * P.ld + x0 + tx] = (x >= 0 && x < P.K) ? P.in[(size_t)r * P.ld_in + x] : zero;
+      }
+    }
+  }
+}
+
 // C = alpha sum_z partial[z] (z in order) + beta C + bias, then tanh; BF16 copy.
 __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int ldc,
                                 __nv_bfloat16* Cb, int M, int N, float alpha, float beta,
@@ -770,7 +1133,7 @@ EncodeTiledFn tensor_map_encoder() {
 
 // 2-D map of a row-major BF16 matrix [rows x K] (leading dimension ld), boxes of
 // box_rows x 64 with the 128-byte swizzle; out-of-range elements read as zero.
-bool make_tile_map(CUtensorMap* map, const void* base, int rows, int K, int ld, int box_rows) {
+bool make_tile_map(CUtensorMap* map, const void* base, int rows, int K, long long ld, int box_rows) {
   const EncodeTiledFn enc = tensor_map_encoder();
   if (!enc) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
@@ -851,6 +1214,29 @@ cudaError_t launch_tma_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaSt
                                                     bias, act, err);
 }
 
+template <int BN, int STAGES, int EPW>
+cudaError_t launch_stream(const StreamMaps& maps, const StreamArgs& P, int grid, cudaStream_t st) {
+  static bool configured[64] = {};
+  constexpr int smem = tma_smem_bytes<BN, STAGES>();
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_gemm_stream<BN, STAGES, EPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  k_gemm_stream<BN, STAGES, EPW><<<grid, 64 + 32 * EPW, smem, st>>>(maps, P);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int tiles = P.p * P.tm * P.tn;
+  const int cols = std::min(BN, P.N);
+  k_stream_reduce<<<dim3(tiles, (cols + 3) / 4, BM / 32), 128, 0, st>>>(P, BN, grid);
+  return cudaGetLastError();
+}
+
+inline size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+
 // Tiny products (the plastic-strain network's 64-wide layers) on the CUDA cores: one
 // thread per output, the BF16 operands' products summed in FP32 in K order, then the
 // epilogue of the tensor-core kernels (alpha, beta, bias, tanh, BF16 copy).
@@ -874,6 +1260,144 @@ __global__ void __launch_bounds__(256) k_gemm_small(const __nv_bfloat16* A, int 
   if (act == 1) v = tanhf(v);
   C[(size_t)row * ldc + col] = v;
   if (Cb) Cb[(size_t)row * ldc + col] = __float2bfloat16(v);
+}
+
+// The stream's workspace, grown to `need` bytes (null: no memory); takes the lock.
+void* workspace(int dev, cudaStream_t st, size_t need, std::unique_lock<std::mutex>& lock) {
+  lock.lock();
+  if (!g_ws.count({dev, st})) {
+    size_t on_dev = 0;
+    for (const auto& kv : g_ws) on_dev += kv.first.first == dev;
+    if (on_dev >= kMaxWorkspaces)
+      for (auto it = g_ws.begin(); it != g_ws.end();) {
+        if (it->first.first == dev) {
+          if (it->second.p) cudaFree(it->second.p);
+          it = g_ws.erase(it);
+        } else {
+          ++it;
+        }
+      }
+  }
+  Workspace& w = g_ws[{dev, st}];
+  if (w.size < need) {
+    if (w.p) cudaFree(w.p);  // synchronises the device: no call still reads it
+    w.p = nullptr;
+    w.size = 0;
+    void* p = nullptr;
+    if (cudaMalloc(&p, need) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    w.p = static_cast<float*>(p);
+    w.size = need;
+  }
+  return w.p;
+}
+
+// How a product's operands reach the tensor-core kernels.
+struct Operands {
+  bool tma = false;     // A [M x K] and B [N x K] below can be addressed by TMA
+  bool stream = false;  // k_gemm_stream
+  const void* A = nullptr;
+  const void* B = nullptr;
+  long long lda = 0, ldb = 0;
+  int p = 1, b_copies = 1, b_cols = 0, max_delta = 0;
+  int delta[kMaxClasses] = {};
+  // copies to make: 0, 1 or 2 of them
+  PackArgs pack_a{}, pack_b{};
+  bool do_a = false, do_b = false;
+  size_t pack_bytes = 0;
+};
+
+// Copies are made for products that the CUDA cores do not take (more than 2^20 multiply-adds)
+// and whose copies stay below this; beyond it, and while the stream is captured into a graph
+// (whose replays would outlive the workspace), the staging kernel k_gemm_bf16 reads the
+// operands as they are.
+constexpr size_t kMaxPackBytes = (size_t)256 << 20;
+
+// Operands as they are where TMA can read them (A B^T, 16-byte rows).  Otherwise: a tall A
+// before a narrow B (the streaming products) stays in place, in row classes; any other
+// operand is copied to aligned rows, transposed if need be, which costs a pass over it
+// (81,920 x 96 x 96, A B: 97.2 us staged element by element, 22.7 with B copied; 96 x 96 x
+// 327,680, A^T B: 466 and 204 with both).
+int choose_operands(const void* A, int lda, int transA, const void* B, int ldb, int transB, int M,
+                    int N, int K, bool tma_shape, cudaStream_t st, Operands* op) {
+  const bool a_ok = !transA && lda >= K && lda % 8 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+  const bool b_ok = transB && ldb >= K && ldb % 8 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  op->A = A;
+  op->B = B;
+  op->lda = lda;
+  op->ldb = ldb;
+  op->b_cols = K;
+  if (!tensor_map_encoder()) return CI_OK;  // everything through the staging kernel
+  // A of 8 MB or more read once past a B of at most 256 rows, K long enough to cut
+  const bool streams = N <= 256 && (long long)M * K >= (1 << 22) && K >= 1024;
+  if (!tma_shape || streams) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      op->tma = tma_shape;
+      return CI_OK;
+    }
+  }
+  if (!tma_shape) {
+    if ((transA ? lda < M : lda < K) || (transB ? ldb < K : ldb < N)) return CI_OK;
+    const int kp8 = (K + 7) / 8 * 8;
+    if (!a_ok && !transA && streams && M >= 4096) {
+      const int g = lda % 8 == 0 ? 8 : lda % 4 == 0 ? 4 : lda % 2 == 0 ? 2 : 1;
+      op->p = kMaxClasses / g;
+      for (int c = 0; c < op->p; c++) {
+        op->delta[c] = (int)((reinterpret_cast<uintptr_t>(A) / 2 + (size_t)c * lda) & 7);
+        op->max_delta = std::max(op->max_delta, op->delta[c]);
+      }
+      op->b_copies = op->p;
+    } else if (!a_ok) {
+      op->do_a = true;
+      op->pack_a = {static_cast<const __nv_bfloat16*>(A), nullptr, M, K, lda, transA, kp8, {}};
+      op->pack_bytes += align256(sizeof(__nv_bfloat16) * (size_t)M * kp8);
+    }
+    if (!b_ok || op->max_delta > 0 || op->p > 1) {
+      op->do_b = true;
+      op->b_cols = op->max_delta ? (K + op->max_delta + 7) / 8 * 8 : K;
+      const int ld = (op->b_cols + 7) / 8 * 8;
+      op->pack_b = {static_cast<const __nv_bfloat16*>(B), nullptr, N, K, ldb, !transB, ld, {}};
+      for (int c = 0; c < op->p; c++) op->pack_b.delta[c] = op->delta[c];
+      op->pack_bytes += align256(sizeof(__nv_bfloat16) * (size_t)op->b_copies * N * ld);
+    }
+    if (op->pack_bytes > kMaxPackBytes) {
+      *op = Operands();
+      op->A = A;
+      op->B = B;
+      op->lda = lda;
+      op->ldb = ldb;
+      return CI_OK;
+    }
+  }
+  op->tma = true;
+  op->stream = streams;
+  return CI_OK;
+}
+
+// Enqueues the copies into `at` and points the operands to them.
+bool pack_operands(Operands* op, char* at, cudaStream_t st) {
+  auto run = [&](PackArgs& a, int copies) {
+    a.out = reinterpret_cast<__nv_bfloat16*>(at);
+    at += align256(sizeof(__nv_bfloat16) * (size_t)copies * a.rows * a.ld);
+    const dim3 grid((a.ld + 127) / 128, (a.rows + 31) / 32, copies);
+    k_pack_bf16<<<grid, 256, 0, st>>>(a);
+    return cudaGetLastError() == cudaSuccess;
+  };
+  if (op->do_a) {
+    if (!run(op->pack_a, 1)) return false;
+    op->A = op->pack_a.out;
+    op->lda = op->pack_a.ld;
+  }
+  if (op->do_b) {
+    if (!run(op->pack_b, op->b_copies)) return false;
+    op->B = op->pack_b.out;
+    op->ldb = op->pack_b.ld;
+  }
+  return true;
 }
 
 }  // namespace
@@ -904,53 +1428,87 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
                ? CI_OK
                : ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: small-product launch failed");
   }
-  bool tma = tma_shape;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess)
+    return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: no current device");
+  __nv_bfloat16* cb = static_cast<__nv_bfloat16*>(C_bf16);
+  std::unique_lock<std::mutex> ws_lock(g_ws_mu, std::defer_lock);  // held until enqueued
+  Operands op;
+  {
+    const int rc = choose_operands(A, lda, transA, B, ldb, transB, M, N, K, tma_shape, st, &op);
+    if (rc) return rc;
+  }
+  if (op.stream) {
+    const int bn = N <= 64 ? 64 : N <= 96 ? 96 : N <= 128 ? 128 : 256;
+    StreamArgs P{};
+    P.C = C;
+    P.Cb = cb;
+    P.bias = bias;
+    P.err = d_error;
+    P.ldc = ldc;
+    P.M = M;
+    P.N = N;
+    P.alpha = alpha;
+    P.beta = beta;
+    P.act = activation;
+    P.p = op.p;
+    P.b_copies = op.b_copies;
+    for (int c = 0; c < kMaxClasses; c++) P.delta[c] = op.delta[c];
+    P.tm = ((M + op.p - 1) / op.p + BM - 1) / BM;
+    P.tn = (N + bn - 1) / bn;
+    P.kt = (K + op.max_delta + TBK - 1) / TBK;
+    const long long units = (long long)P.p * P.tm * P.tn * P.kt;
+    const int grid = (int)std::min<long long>(num_sms(), units);
+    const size_t part = align256(sizeof(float) * 2 * (size_t)grid * BM * bn);
+    char* ws = static_cast<char*>(workspace(dev, st, part + op.pack_bytes, ws_lock));
+    if (!ws) return ci::set_last_error(CI_ERR_NOMEM, "ci_gemm_bf16: workspace");
+    P.partial = reinterpret_cast<float*>(ws);
+    if (!pack_operands(&op, ws + part, st))
+      return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: packing launch failed");
+    StreamMaps maps;
+    bool ok = make_tile_map(&maps.b, op.B, N * op.b_copies, op.b_cols, op.ldb, bn);
+    for (int c = 0; c < op.p && ok; c++) {
+      const uintptr_t row = reinterpret_cast<uintptr_t>(op.A) + 2 * (size_t)c * op.lda;
+      ok = make_tile_map(&maps.a[c], reinterpret_cast<const void*>(row & ~(uintptr_t)15),
+                         (M - c + op.p - 1) / op.p, K + op.delta[c], (long long)op.p * op.lda, BM);
+    }
+    if (!ok) return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: tensor map");
+    const cudaError_t e = bn == 64   ? launch_stream<64, 8, 4>(maps, P, grid, st)
+                          : bn == 96  ? launch_stream<96, 7, 4>(maps, P, grid, st)
+                          : bn == 128 ? launch_stream<128, 5, 8>(maps, P, grid, st)
+                                      : launch_stream<256, 3, 8>(maps, P, grid, st);
+    return e == cudaSuccess ? CI_OK : ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(e));
+  }
+  bool tma = op.tma;
   const int bn_tma = N <= 64 ? 64 : N <= 128 ? 128 : 256;
-  CUtensorMap ta, tb;
-  tma = tma && make_tile_map(&ta, A, M, K, lda, BM) && make_tile_map(&tb, B, N, K, ldb, bn_tma);
   const int bn = tma ? bn_tma : (N <= 64 ? 64 : 128);
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-  // split K when the output has too few tiles to fill the GPU and K is long
+  // Split K when the output has too few tiles to fill the GPU and K is long.  With more than
+  // half a tile per SM the split costs more than it gives (2,048 x 2,048 x 512, 128 tiles: 11.9
+  // us whole, 38.9 in two halves of K), but a longer chain of products loses accuracy, so only
+  // K up to 896 (1e-6 of the result) stays whole.
   int splits = 1;
-  if (tiles < 304 && K >= 8 * BK) splits = std::min((304 + tiles - 1) / tiles, (K + 4 * BK - 1) / (4 * BK));
+  const bool whole = tma && 2 * tiles > num_sms() && K <= 896;
+  if (!whole && tiles < 304 && K >= 8 * BK)
+    splits = std::min((304 + tiles - 1) / tiles, (K + 4 * BK - 1) / (4 * BK));
   splits = std::max(1, std::min(splits, 512));
   int k_chunk = (K + splits - 1) / splits;
   k_chunk = (k_chunk + BK - 1) / BK * BK;
   splits = (K + k_chunk - 1) / k_chunk;
   float* partial = nullptr;
-  std::unique_lock<std::mutex> ws_lock(g_ws_mu, std::defer_lock);  // held until enqueued
-  if (splits > 1) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess)
-      return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: no current device");
-    const size_t need = sizeof(float) * (size_t)splits * M * N;
-    ws_lock.lock();
-    if (!g_ws.count({dev, st})) {
-      size_t on_dev = 0;
-      for (const auto& kv : g_ws) on_dev += kv.first.first == dev;
-      if (on_dev >= kMaxWorkspaces)
-        for (auto it = g_ws.begin(); it != g_ws.end();) {
-          if (it->first.first == dev) {
-            if (it->second.p) cudaFree(it->second.p);
-            it = g_ws.erase(it);
-          } else {
-            ++it;
-          }
-        }
-    }
-    Workspace& w = g_ws[{dev, st}];
-    if (w.size < need) {
-      if (w.p) cudaFree(w.p);  // synchronises the device: no call still reads it
-      w.p = nullptr;
-      w.size = 0;
-      if (cudaMalloc(&w.p, need) != cudaSuccess)
-        return ci::set_last_error(CI_ERR_NOMEM, "ci_gemm_bf16: split-K workspace");
-      w.size = need;
-    }
-    partial = w.p;
+  const size_t part = splits > 1 ? align256(sizeof(float) * (size_t)splits * M * N) : 0;
+  if (part + op.pack_bytes) {
+    char* ws = static_cast<char*>(workspace(dev, st, part + op.pack_bytes, ws_lock));
+    if (!ws) return ci::set_last_error(CI_ERR_NOMEM, "ci_gemm_bf16: workspace");
+    if (splits > 1) partial = reinterpret_cast<float*>(ws);
+    if (!pack_operands(&op, ws + part, st))
+      return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: packing launch failed");
   }
+  CUtensorMap ta, tb;
+  if (tma && !(make_tile_map(&ta, op.A, M, K, op.lda, BM) &&
+               make_tile_map(&tb, op.B, N, K, op.ldb, bn_tma)))
+    return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: tensor map");
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, splits);
-  __nv_bfloat16* cb = static_cast<__nv_bfloat16*>(C_bf16);
   cudaError_t le = cudaSuccess;
   if (tma && splits == 1) {
     if (bn == 64)

@@ -257,17 +257,15 @@ int ci_batch_run_peaks(ci_batch* b, int every, int max_snaps, float* peak_disp, 
  * `stream`.  A, B: BF16 row-major with leading dimensions lda, ldb, transA / transB
  * select op() = transpose.  C: FP32 row-major (ldc); C_bf16 (may be NULL) receives a
  * BF16 copy.  All pointers are device pointers.  *d_error (device int) is set to 1 if
- * a tensor-core wait timed out (the result is then invalid).  When the output has few
- * 128-row tiles and K is long, K is split across CTAs: partial tiles go to a per-device
- * FP32 workspace (one per device and stream, grown by cudaMalloc on first need, at most
- * 32 streams' kept per device) and are summed in a fixed order, so results are
- * deterministic; calls on different streams may run concurrently.  Three paths, all with the same epilogue (alpha, beta C, bias, tanh,
- * BF16 copy): C = A B^T with both operands K-major (transA = 0, transB = 1), M >= 128,
- * N >= 16, K >= 64, 16-byte aligned A and B and leading dimensions that are multiples
- * of 8 runs on a TMA-fed pipelined tensor-core kernel; any other form with at most
- * 2^20 multiply-adds (M N K <= 1048576) runs on the CUDA cores, one thread per output
- * summing the BF16 products in FP32 in K order; the remaining forms run on a
- * tensor-core kernel that stages its operands itself. */
+ * a tensor-core wait timed out (the result is then invalid).  Products of at most 2^20
+ * multiply-adds (M N K <= 1048576) outside the form A B^T with 16-byte rows run on the CUDA
+ * cores, one thread per output summing the BF16 products in FP32 in K order; all others on
+ * the tensor cores.  A workspace per device and stream (grown by cudaMalloc on first need,
+ * at most 32 streams' kept per device) holds the FP32 partial sums of products whose K is
+ * cut across CTAs, added in a fixed order so that results are deterministic, and aligned
+ * copies (at most 256 MB per call) of operands that the tensor kernels cannot read in
+ * place; calls on different streams may run concurrently.  While `stream` is being captured
+ * no copies are made. */
 int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int transB, float* C,
                  int ldc, void* C_bf16, int M, int N, int K, float alpha, float beta,
                  const float* bias, int activation, int* d_error, void* stream);

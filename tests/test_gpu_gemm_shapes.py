@@ -73,3 +73,73 @@ def test_epilogue_forms(cilib, M, N, K, form):
     torch = pytest.importorskip("torch")
     c, ref = product(cilib, torch, M, N, K, lda_pad=(-K) % 8, ldb_pad=(-K) % 8, seed=M + N, **form)
     assert close(c, ref)
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 16, 1024), (4103, 96, 1031), (5000, 64, 2050),
+                                   (8200, 65, 1100), (4097, 131, 1999), (4099, 256, 1027),
+                                   (96, 96, 50001), (300, 30, 15000)])
+@pytest.mark.parametrize("form", [dict(), dict(lda_pad=1), dict(lda_pad=2, a_off=3), dict(a_off=8),
+                                  dict(lda_pad=4, ldc_pad=3, bias=True, copy=True),
+                                  dict(ldb_pad=3, b_off=5, beta=0.5, alpha=0.01, act=1)])
+def test_streaming_products(cilib, M, N, K, form):
+    """A long A past a narrow B: one unit range per SM, cut tiles, rows of every offset to a
+    16-byte boundary (row classes), B copied; NaN around the operands; repeats to the bit."""
+    torch = pytest.importorskip("torch")
+    c, ref = product(cilib, torch, M, N, K, seed=M + K, **form)
+    assert close(c, ref)
+    c2, _ = product(cilib, torch, M, N, K, seed=M + K, **form)
+    assert np.array_equal(c, c2)
+
+
+@pytest.mark.parametrize("lda_pad", [0, 1, 2, 4, 7])
+def test_an_infinite_row_end_stays_in_its_row(cilib, lda_pad):
+    """Row classes read the end of the row before; an infinity there reaches its own row only."""
+    torch = pytest.importorskip("torch")
+
+    def edit(a):
+        a[17, -1] = float("inf")
+        a[4000, -3:] = float("nan")
+
+    M, N, K = 4099, 40, 1025
+    c, ref = product(cilib, torch, M, N, K, lda_pad=lda_pad, a_edit=edit, seed=5)
+    bad = ~np.isfinite(c).all(axis=1)
+    assert sorted(np.flatnonzero(bad)) == [17, 4000]
+    assert close(c[~bad], ref[~bad])
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 70, 1000), (1000, 17, 130), (20000, 96, 96), (129, 300, 67),
+                                   (700, 9, 1500), (2000, 1000, 40), (5, 3000, 3000)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (1, 1), (0, 1)])
+@pytest.mark.parametrize("form", [dict(), dict(lda_pad=3, ldb_pad=1, a_off=1, b_off=2)])
+def test_copied_operands(cilib, M, N, K, ta, tb, form):
+    """Products whose operands TMA cannot read go through aligned copies, in every transpose
+    form, M, N and K below a tile among them."""
+    torch = pytest.importorskip("torch")
+    c, ref = product(cilib, torch, M, N, K, ta=ta, tb=tb, bias=True, seed=M + N, **form)
+    assert close(c, ref)
+
+
+def test_captured_product(cilib):
+    """While its stream is captured a product takes no workspace: replays read the operands."""
+    torch = pytest.importorskip("torch")
+    M, N, K = 300, 100, 131
+    a = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    b = torch.randn((N, K), device="cuda").to(torch.bfloat16)
+    c = torch.zeros((M, N), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def call():
+        st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert cilib.lib().ci_gemm_bf16(a.data_ptr(), K, 0, b.data_ptr(), K, 1, c.data_ptr(), N,
+                                        None, M, N, K, 1.0, 0.0, None, 0, err.data_ptr(), st) == 0
+
+    call()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call()
+    a.mul_(0.5)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = (a.double() @ b.double().t()).cpu().numpy()
+    assert close(c.double().cpu().numpy(), ref)
