@@ -103,9 +103,14 @@ struct Group {
   DBuf<ElemParams> inst_ep;
   DBuf<NodeParams> inst_np;
   DBuf<int> inst_nsteps, step_ctr;
-  // resident form of the step (ci_resident.cuh): kernel, entry lists, tagged slots, the
-  // order in which CTAs take chunks with its counter and the abort flag, the next tag
-  ResidentPick res;
+  // resident form of the step (ci_resident.cuh): the kernels, each with its instances' part
+  // of the order in which CTAs take chunks; entry lists, tagged slots, the order's counter
+  // and the abort flag, the next tag
+  struct Resident {
+    ResidentPick pick;
+    int begin, count;
+  };
+  std::vector<Resident> res;
   DBuf<uint32_t> node_ent, node_slots;
   DBuf<uint16_t> ent;
   DBuf<int> slots;
@@ -138,7 +143,7 @@ namespace {
 
 // The group runs resident (the tet10 kernel has four lanes per element; the autotuner also
 // tries one, which runs from a graph).
-bool resident(const Group& G) { return G.res.kernel && (G.npe == 4 || G.elem_lanes == 4); }
+bool resident(const Group& G) { return !G.res.empty() && (G.npe == 4 || G.elem_lanes == 4); }
 
 ElemParams make_ep(const ci_material& m, double dt) {
   ElemParams p{};
@@ -430,49 +435,72 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   CB_CUDA(G.step_ctr.alloc(1));
   CB_CUDA(G.peak.alloc(G.insts.size()));
   CB_CUDA(npe == 4 ? configure<4>((int)G.smem) : configure<10>((int)G.smem));
-  // the resident form, where one instance's chunks fit the GPU together
-  G.res = ResidentPick();
-  std::vector<ResidentChunk> rchunks;
+  // the resident form, where every instance's chunks fit the GPU together: a launch for the
+  // instances of each CTA size (resident_threads)
+  G.res.clear();
   if (may_reside) {
+    std::vector<ResidentChunk> rchunks;
+    std::vector<int> threads(n_inst);
     int at = 0;
-    for (size_t j = 0; j < n_inst; j++)
+    for (size_t j = 0; j < n_inst; j++) {
       for (const ResidentChunk& c : tab[src[j]].chunks) {
         rchunks.push_back({at, c.n_slots});
         at += c.n_slots;
       }
-    CB_CUDA(pick_resident(npe, false, true, chunks, rchunks, 0, most_chunks, b->device, &G.res));
-  }
-  if (G.res.kernel) {
-    ResidentTables all;
-    long long so = 0;
-    for (size_t j = 0; j < n_inst; j++) {
-      const ResidentTables& t = tab[src[j]];
-      all.node_ent.insert(all.node_ent.end(), t.node_ent.begin(), t.node_ent.end());
-      all.node_slots.insert(all.node_slots.end(), t.node_slots.begin(), t.node_slots.end());
-      all.ent.insert(all.ent.end(), t.ent.begin(), t.ent.end());
-      for (int sl : t.slots) all.slots.push_back(sl + (int)so);
-      so += plans[j]->slot_row[plans[j]->N];
+      threads[j] = resident_threads(npe, true, plans[j]->max_chunk_elems);
     }
     // instances with the most work first, so that the last to end are short ones
     std::vector<int> by(n_inst), order;
     for (size_t j = 0; j < n_inst; j++) by[j] = (int)j;
     chunk0.push_back(G.C);
     std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
+      if (threads[x] != threads[y]) return threads[x] > threads[y];
       return (long long)nsteps[x] * plans[x]->E > (long long)nsteps[y] * plans[y]->E;
     });
-    for (int j : by)
-      for (int c = chunk0[j]; c < chunk0[j + 1]; c++) order.push_back(c);
-    CB_CUDA(G.node_ent.upload(all.node_ent, st));
-    CB_CUDA(G.node_slots.upload(all.node_slots, st));
-    CB_CUDA(G.ent.upload(all.ent, st));
-    CB_CUDA(G.slots.upload(all.slots, st));
-    CB_CUDA(G.rchunks.upload(rchunks, st));
-    CB_CUDA(G.order.upload(order, st));
-    CB_CUDA(G.claim.alloc(2));
-    CB_CUDA(G.halo.alloc(2 * (size_t)G.S));
-    CB_CUDA(cudaMemsetAsync(G.halo.p, 0, sizeof(float4) * 2 * (size_t)G.S, st));
-    G.tag = 1;
-    CB_CUDA(cudaStreamSynchronize(st));
+    bool all_fit = true;
+    for (size_t i = 0; i < n_inst && all_fit;) {
+      const int p = threads[by[i]], begin = (int)order.size();
+      std::vector<ChunkInfo> ci;
+      std::vector<ResidentChunk> rc;
+      int most = 0;
+      for (; i < n_inst && threads[by[i]] == p; i++) {
+        const int c0 = chunk0[by[i]], c1 = chunk0[by[i] + 1];
+        most = std::max(most, c1 - c0);
+        for (int c = c0; c < c1; c++) {
+          order.push_back(c);
+          ci.push_back(chunks[c]);
+          rc.push_back(rchunks[c]);
+        }
+      }
+      Group::Resident r{ResidentPick(), begin, (int)order.size() - begin};
+      CB_CUDA(pick_resident(npe, false, true, ci, rc, 0, most, b->device, &r.pick));
+      all_fit = r.pick.kernel != nullptr;
+      G.res.push_back(r);
+    }
+    if (!all_fit) G.res.clear();
+    if (all_fit) {
+      ResidentTables all;
+      long long so = 0;
+      for (size_t j = 0; j < n_inst; j++) {
+        const ResidentTables& t = tab[src[j]];
+        all.node_ent.insert(all.node_ent.end(), t.node_ent.begin(), t.node_ent.end());
+        all.node_slots.insert(all.node_slots.end(), t.node_slots.begin(), t.node_slots.end());
+        all.ent.insert(all.ent.end(), t.ent.begin(), t.ent.end());
+        for (int sl : t.slots) all.slots.push_back(sl + (int)so);
+        so += plans[j]->slot_row[plans[j]->N];
+      }
+      CB_CUDA(G.node_ent.upload(all.node_ent, st));
+      CB_CUDA(G.node_slots.upload(all.node_slots, st));
+      CB_CUDA(G.ent.upload(all.ent, st));
+      CB_CUDA(G.slots.upload(all.slots, st));
+      CB_CUDA(G.rchunks.upload(rchunks, st));
+      CB_CUDA(G.order.upload(order, st));
+      CB_CUDA(G.claim.alloc(2));
+      CB_CUDA(G.halo.alloc(2 * (size_t)G.S));
+      CB_CUDA(cudaMemsetAsync(G.halo.p, 0, sizeof(float4) * 2 * (size_t)G.S, st));
+      G.tag = 1;
+      CB_CUDA(cudaStreamSynchronize(st));
+    }
   }
   CB_CUDA(cudaStreamSynchronize(st));
   return CI_OK;
@@ -499,7 +527,6 @@ int enqueue_resident(Group& G, int total, const Snapshots& sn) {
       CB_CUDA(cudaMemsetAsync(G.halo.p, 0, sizeof(float4) * 2 * (size_t)G.S, st));
       G.tag = 1;
     }
-    CB_CUDA(cudaMemsetAsync(G.claim.p, 0, 2 * sizeof(int), st));
     const FusedArgs F = group_args(G, 0);
     ResidentArgs A{};
     A.P = F.P;
@@ -532,8 +559,6 @@ int enqueue_resident(Group& G, int total, const Snapshots& sn) {
     A.inst_ep = G.inst_ep.p;
     A.inst_np = G.inst_np.p;
     A.inst_nsteps = G.inst_nsteps.p;
-    A.order = G.order.p;
-    A.n_chunks = G.C;
     A.step0 = step0;
     A.every = std::max(1, sn.every);
     A.snap_end = sn.n_snaps == 0               ? 0
@@ -543,9 +568,14 @@ int enqueue_resident(Group& G, int total, const Snapshots& sn) {
     A.snap = sn.snap;
     A.peak = sn.peak;
     G.tag += (unsigned)k;
-    void* args[] = {&A};
-    CB_CUDA(cudaLaunchCooperativeKernel(G.res.kernel, dim3(std::min(G.res.ctas, G.C)),
-                                        dim3(G.res.threads), args, G.res.smem, st));
+    for (const Group::Resident& r : G.res) {
+      CB_CUDA(cudaMemsetAsync(G.claim.p, 0, 2 * sizeof(int), st));
+      A.order = G.order.p + r.begin;
+      A.n_chunks = r.count;
+      void* args[] = {&A};
+      CB_CUDA(cudaLaunchCooperativeKernel(r.pick.kernel, dim3(std::min(r.pick.ctas, r.count)),
+                                          dim3(r.pick.threads), args, r.pick.smem, st));
+    }
   }
   return CI_OK;
 }

@@ -137,17 +137,31 @@ __device__ __forceinline__ bool res_receive(const ResidentArgs& A, const float4*
   return true;
 }
 
+struct ResidentParams {
+  ElemParams ep;
+  NodeParams np;
+};
+
 template <int NPE, int MODE, int P, bool CHIP, bool BATCH>
 __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* sm, int ci,
-                                          float (*red)[2][P / 32]) {
+                                          float (*red)[2][P / 32], ResidentParams* par) {
   constexpr int NQ = Rule<NPE>::NQ;
   constexpr int LN = NPE == 10 ? 4 : 1;  // lanes per element
   constexpr int EPW = P / LN;            // elements per window
   constexpr int EU = NPE == 4 ? 8 : 4;   // a node's entries and slots loaded at once
   const int tid = threadIdx.x;
   const ChunkInfo ch = A.P.chunks[ci];
-  const ElemParams ep = BATCH ? A.inst_ep[ch.inst] : A.ep;
-  const NodeParams np = BATCH ? A.inst_np[ch.inst] : A.np;
+  // an instance's parameters are read where they are used (a copy per thread would take some
+  // thirty registers), a single solve's come as constants
+  if (BATCH) {
+    if (tid == 0) {
+      par->ep = A.inst_ep[ch.inst];
+      par->np = A.inst_np[ch.inst];
+    }
+    res_sync<P>();
+  }
+  const ElemParams& ep = BATCH ? par->ep : A.ep;
+  const NodeParams& np = BATCH ? par->np : A.np;
   int n = A.nsteps;
   if (BATCH) n = max(0, min(n, A.inst_nsteps[ch.inst] - A.step0));
   const bool snaps = BATCH && A.snap_end > 0;
@@ -372,6 +386,8 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
       const bool act = i < ne;
       const int ii = act ? i : 0;
       if (NPE == 10) {
+        // a warp past the last element skips the window (its lanes have no part in the sums)
+        if (CHIP && w + (tid & ~31) / LN >= ne) break;
         int ln[10];
 #pragma unroll
         for (int a = 0; a < 10; a++)
@@ -573,28 +589,36 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   return true;
 }
 
-// Registers: at most 128 (four CTAs of 128 threads per SM), 80 for batches of one- and
-// two-warp chunks, which want as many chunks on an SM as they can get.
+// Resident CTAs per SM: at most 128 registers for four CTAs of 128 threads; batches of small
+// chunks up to the register count at which they spill little (tet4: 64 threads at 64
+// registers 1.77 us per instance and step of 28-element chunks, at 96 2.65).
+constexpr int resident_min_ctas(int npe, int p, bool batch) {
+  if (p == 128) return 4;
+  if (!batch || npe == 10) return 10;
+  return p == 64 ? 16 : 20;
+}
+
 template <int NPE, int MODE, int P, bool CHIP, bool BATCH>
-__global__ void __launch_bounds__(P, P == 128 ? 4 : P == 64 ? 10 : 20)
+__global__ void __launch_bounds__(P, resident_min_ctas(NPE, P, BATCH))
     k_resident(const __grid_constant__ ResidentArgs A) {
   extern __shared__ __align__(16) unsigned char res_sm[];
   __shared__ float red[2][2][P / 32];
   if constexpr (!BATCH) {
-    res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, blockIdx.x, red);
+    res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, blockIdx.x, red, nullptr);
   } else {
     // batches: chunks taken in order, an instance's chunks next to each other.  A CTA waits
     // only for chunks of its own instance; those before it in the order are running or
     // done, and the earliest instance with a chunk still to be taken gets every CTA that
     // comes free until all its chunks (no more than there are CTAs) are running.
     __shared__ int taken;
+    __shared__ ResidentParams par;
     for (;;) {
       if (threadIdx.x == 0) taken = atomicAdd(A.claim, 1);
       res_sync<P>();
       const int c = taken;
       res_sync<P>();
       if (c >= A.n_chunks) return;
-      if (!res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, A.order[c], red)) return;
+      if (!res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, A.order[c], red, &par)) return;
       res_sync<P>();
     }
   }

@@ -75,10 +75,18 @@ __host__ __device__ constexpr size_t resident_smem(int npe, int nl, int ne, int 
                  : 121 * (size_t)nl + 12 * (size_t)ns + 64;
 }
 
-// Picks the kernel for chunks of the given sizes ((local nodes, elements) pairs);
-// `energy_threads`: the fused kernel's CTA size whose work sums have to come out the same
-// (0: the sums are not read).  No kernel if the chunks do not fit or `need_ctas` of them
-// cannot be on the GPU together.
+// Threads of the kernel for chunks of at most `elements` elements.  A single solve has SMs to
+// spare and wants a warp for the elements beside one for the nodes; a batch wants as many
+// chunks on an SM as it can get.  us per instance and step, 16 equal cubes: tet4 of 16 elements
+// per chunk 0.86 with 32 threads, 1.19 with 64; 28 and 41 elements 1.73 and 2.02 with 64, 1.92
+// and 2.10 with 32; tet10 of 16 and 18 elements 2.2 and 4.4 with 64 threads, 5.5 and 5.7 with
+// 128; 28 and 41 elements 6.4 and 6.8 with 128, 9.6 and 11.6 with 64 (a launch per step of all
+// 16: tet4 2.81, 4.73, 5.30, tet10 3.24, 5.52, 6.84, 8.34).
+int resident_threads(int npe, bool batch, int elements);
+
+// Picks the kernel for `chunks`; `energy_threads`: the fused kernel's CTA size whose work sums
+// have to come out the same (0: the sums are not read).  No kernel if the chunks do not fit or
+// `need_ctas` of them cannot be on the GPU together.
 cudaError_t pick_resident(int npe, bool refcompat, bool batch, const std::vector<ChunkInfo>& chunks,
                           const std::vector<ResidentChunk>& rchunks, int energy_threads,
                           int need_ctas, int device, ResidentPick* out);

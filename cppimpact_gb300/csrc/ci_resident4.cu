@@ -27,6 +27,12 @@ namespace ci {
 
 const void* resident_kernel_tet10(bool refcompat, bool batch, int threads, bool chip);
 
+int resident_threads(int npe, bool batch, int elements) {
+  if (npe == 10) return batch && elements <= 24 ? 64 : 128;
+  if (!batch) return elements <= 32 ? 64 : 128;
+  return elements <= 24 ? 32 : elements <= 64 ? 64 : 128;
+}
+
 cudaError_t pick_resident(int npe, bool refcompat, bool batch, const std::vector<ChunkInfo>& chunks,
                           const std::vector<ResidentChunk>& rchunks, int energy_threads,
                           int need_ctas, int device, ResidentPick* out) {
@@ -38,44 +44,40 @@ cudaError_t pick_resident(int npe, bool refcompat, bool batch, const std::vector
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) return e;
   if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device))) return e;
   if (!coop) return cudaSuccess;
-  const int lanes = npe == 10 ? 4 : 1;
-  int max_lanes = 0;  // threads that an element per thread (a point per thread) fills
-  for (const ChunkInfo& c : chunks) max_lanes = std::max(max_lanes, lanes * (c.elem_end - c.elem_begin));
-  for (const bool chip : {true, false})
-    for (const int threads : {32, 64, 128}) {
-      // few threads where they hold the chunk's elements in one pass: a barrier of one or two
-      // warps is cheaper and more chunks share an SM.  A single solve has SMs to spare and
-      // wants a warp for the elements and others for the nodes.
-      if (threads < 128 && max_lanes > (batch ? threads : threads / 2)) continue;
-      // the same work sums as the fused kernel's: its CTA size, or no thread of either with
-      // more than one element (further warps only add zeros)
-      if (energy_threads && threads != energy_threads && max_lanes > std::min(threads, energy_threads))
-        continue;
-      const void* fn = npe == 4 ? resident_kernel_tet4(refcompat, batch, threads, chip)
-                                : resident_kernel_tet10(refcompat, batch, threads, chip);
-      if (!fn) continue;
-      size_t smem = 0;
-      bool fits = true;
-      for (size_t i = 0; i < chunks.size(); i++) {
-        const ChunkInfo& c = chunks[i];
-        const int ne = c.elem_end - c.elem_begin, ns = rchunks[i].n_slots;
-        smem = std::max(smem, resident_smem(npe, c.n_local, ne, ns, chip));
-        fits = fits && npe * ne <= 65535 && ns <= 65535;  // 16-bit positions
-      }
-      if (!fits || (long long)smem + 2048 > smem_max) continue;
-      // one limit for every solver (a smaller one set later would refuse this one's launch)
-      if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 2048)))
-        return e;
-      int per_sm = 0;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem))) return e;
-      if ((long long)per_sm * sms < need_ctas) continue;
-      out->kernel = fn;
-      out->threads = threads;
-      out->on_chip = chip;
-      out->smem = smem;
-      out->ctas = per_sm * sms;
-      return cudaSuccess;
+  int most = 0;
+  for (const ChunkInfo& c : chunks) most = std::max(most, c.elem_end - c.elem_begin);
+  const int threads = resident_threads(npe, batch, most);
+  // the same work sums as the fused kernel's: its CTA size, or no thread of either with more
+  // than one element or point (further warps only add zeros)
+  if (energy_threads && threads != energy_threads &&
+      (npe == 10 ? 4 : 1) * most > std::min(threads, energy_threads))
+    return cudaSuccess;
+  for (const bool chip : {true, false}) {
+    const void* fn = npe == 4 ? resident_kernel_tet4(refcompat, batch, threads, chip)
+                              : resident_kernel_tet10(refcompat, batch, threads, chip);
+    if (!fn) continue;
+    size_t smem = 0;
+    bool fits = true;
+    for (size_t i = 0; i < chunks.size(); i++) {
+      const ChunkInfo& c = chunks[i];
+      const int ne = c.elem_end - c.elem_begin, ns = rchunks[i].n_slots;
+      smem = std::max(smem, resident_smem(npe, c.n_local, ne, ns, chip));
+      fits = fits && npe * ne <= 65535 && ns <= 65535;  // 16-bit positions
     }
+    if (!fits || (long long)smem + 2048 > smem_max) continue;
+    // one limit for every solver (a smaller one set later would refuse this one's launch)
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 2048)))
+      return e;
+    int per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem))) return e;
+    if ((long long)per_sm * sms < need_ctas) continue;
+    out->kernel = fn;
+    out->threads = threads;
+    out->on_chip = chip;
+    out->smem = smem;
+    out->ctas = per_sm * sms;
+    return cudaSuccess;
+  }
   return cudaSuccess;
 }
 
