@@ -41,6 +41,7 @@
 #include <string>
 
 #include "../../include/cppimpact_gb300.h"
+#include "ci_pdl.h"
 
 namespace ci {
 int set_last_error(int code, const char* msg);
@@ -283,6 +284,8 @@ __global__ void __launch_bounds__(128, 1)
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  ci::pdl_next();
+  ci::pdl_wait();
   const uint32_t tmem = tmem_base;
   bool ok = true;
   int issued = 0;
@@ -604,6 +607,8 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  ci::pdl_next();
+  ci::pdl_wait();
   const uint32_t tmem = tmem_base;
   volatile int* abort = &abort_flag;
   bool ok = true;
@@ -821,6 +826,8 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  ci::pdl_next();
+  ci::pdl_wait();
   const uint32_t tmem = tmem_base;
   volatile int* abort = &abort_flag;
   bool ok = true;
@@ -995,15 +1002,21 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
 }
 
 // The tiles that range ends cut: their partial sums in K order (four contiguous runs of them by
-// four warps, then the runs in order), then the epilogue.  Block (tile, 4 columns, 32 rows).
+// four warps, then the runs in order), then the epilogue.  Block (range end, 4 columns, 32
+// rows); the first end inside a tile stands for the tile.
 __global__ void __launch_bounds__(128) k_stream_reduce(const StreamArgs P, int BN, int g) {
   __shared__ float4 run[4][32];
-  const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  ci::pdl_next();
+  ci::pdl_wait();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int row = blockIdx.z * 32 + lane;
   const long long units = (long long)P.p * P.tm * P.tn * P.kt;
+  const int b0 = blockIdx.x;  // ranges b0 and b0 + 1 meet at u
+  const long long u = stream_begin(units, b0 + 1, g);
+  const int t = (int)(u / P.kt);
   const long long ut = (long long)t * P.kt;
-  const int b0 = (int)(((ut + 1) * g - 1) / units), b1 = (int)(((ut + P.kt) * g - 1) / units);
-  if (b0 == b1) return;  // one CTA had the whole tile
+  if (u == ut || stream_begin(units, b0, g) > ut) return;
+  const int b1 = (int)(((ut + P.kt) * g - 1) / units);
   const float4* part = reinterpret_cast<const float4*>(P.partial) + (size_t)blockIdx.y * 128 + row;
   const int per = (b1 - b0 + 4) / 4, lo = b0 + w * per, hi = min(b1 + 1, lo + per);
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1055,6 +1068,8 @@ struct PackArgs {
 };
 
 __global__ void __launch_bounds__(256) k_pack_bf16(const PackArgs P) {
+  ci::pdl_next();
+  ci::pdl_wait();
   __shared__ __nv_bfloat16 tile[32][34];
   const int d = P.delta[blockIdx.z];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -1085,6 +1100,8 @@ __global__ void __launch_bounds__(256) k_pack_bf16(const PackArgs P) {
 __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int ldc,
                                 __nv_bfloat16* Cb, int M, int N, float alpha, float beta,
                                 const float* bias, int act) {
+  ci::pdl_next();
+  ci::pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= (long long)M * N) return;
   const int row = (int)(i / N), col = (int)(i % N);
@@ -1164,9 +1181,8 @@ cudaError_t launch_tma(const CUtensorMap& ta, const CUtensorMap& tb, dim3 grid, 
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  k_gemm_tma<BN><<<grid, 128, tma_smem_bytes<BN>(), st>>>(ta, tb, C, ldc, Cb, M, N, K, alpha, beta,
-                                                         bias, act, err, k_chunk, partial);
-  return cudaGetLastError();
+  return ci::launch_pdl(k_gemm_tma<BN>, grid, 128, tma_smem_bytes<BN>(), st, ta, tb, C, ldc, Cb, M, N,
+                        K, alpha, beta, bias, act, err, k_chunk, partial);
 }
 
 int num_sms() {
@@ -1200,9 +1216,8 @@ cudaError_t launch_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaStream
   }
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = std::min(tiles, num_sms());
-  k_gemm_tma_pers<BN, STAGES, EPW><<<grid, 64 + 32 * EPW, smem, st>>>(
-      ta, tb, C, ldc, Cb, M, N, K, alpha, beta, bias, act, err);
-  return cudaGetLastError();
+  return ci::launch_pdl(k_gemm_tma_pers<BN, STAGES, EPW>, grid, 64 + 32 * EPW, smem, st, ta, tb, C,
+                        ldc, Cb, M, N, K, alpha, beta, bias, act, err);
 }
 
 template <int BN>
@@ -1226,13 +1241,12 @@ cudaError_t launch_stream(const StreamMaps& maps, const StreamArgs& P, int grid,
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  k_gemm_stream<BN, STAGES, EPW><<<grid, 64 + 32 * EPW, smem, st>>>(maps, P);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = ci::launch_pdl(k_gemm_stream<BN, STAGES, EPW>, grid, 64 + 32 * EPW, smem, st,
+                                       maps, P);
   if (e != cudaSuccess) return e;
-  const int tiles = P.p * P.tm * P.tn;
+  if (grid == 1) return cudaSuccess;
   const int cols = std::min(BN, P.N);
-  k_stream_reduce<<<dim3(tiles, (cols + 3) / 4, BM / 32), 128, 0, st>>>(P, BN, grid);
-  return cudaGetLastError();
+  return ci::launch_pdl(k_stream_reduce, dim3(grid - 1, (cols + 3) / 4, BM / 32), 128, 0, st, P, BN, grid);
 }
 
 inline size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
@@ -1245,6 +1259,8 @@ __global__ void __launch_bounds__(256) k_gemm_small(const __nv_bfloat16* A, int 
                                                     float* C, int ldc, __nv_bfloat16* Cb, int M,
                                                     int N, int K, float alpha, float beta,
                                                     const float* bias, int act) {
+  ci::pdl_next();
+  ci::pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= (long long)M * N) return;
   const int row = (int)(i / N), col = (int)(i % N);
@@ -1384,8 +1400,7 @@ bool pack_operands(Operands* op, char* at, cudaStream_t st) {
     a.out = reinterpret_cast<__nv_bfloat16*>(at);
     at += align256(sizeof(__nv_bfloat16) * (size_t)copies * a.rows * a.ld);
     const dim3 grid((a.ld + 127) / 128, (a.rows + 31) / 32, copies);
-    k_pack_bf16<<<grid, 256, 0, st>>>(a);
-    return cudaGetLastError() == cudaSuccess;
+    return ci::launch_pdl(k_pack_bf16, grid, 256, 0, st, a) == cudaSuccess;
   };
   if (op->do_a) {
     if (!run(op->pack_a, 1)) return false;
@@ -1420,11 +1435,11 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   // CUDA cores, where a 128-row tile pipeline would cost more than the product
   if (!tma_shape && (long long)M * N * K <= (1LL << 20)) {
     const long long outs = (long long)M * N;
-    k_gemm_small<<<(unsigned)((outs + 255) / 256), 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(A), lda, transA, static_cast<const __nv_bfloat16*>(B),
-        ldb, transB, C, ldc, static_cast<__nv_bfloat16*>(C_bf16), M, N, K, alpha, beta, bias,
-        activation);
-    return cudaGetLastError() == cudaSuccess
+    return ci::launch_pdl(k_gemm_small, (unsigned)((outs + 255) / 256), 256, 0, st,
+                          static_cast<const __nv_bfloat16*>(A), lda, transA,
+                          static_cast<const __nv_bfloat16*>(B), ldb, transB, C, ldc,
+                          static_cast<__nv_bfloat16*>(C_bf16), M, N, K, alpha, beta, bias,
+                          activation) == cudaSuccess
                ? CI_OK
                : ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: small-product launch failed");
   }
@@ -1481,7 +1496,7 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   }
   bool tma = op.tma;
   const int bn_tma = N <= 64 ? 64 : N <= 128 ? 128 : 256;
-  const int bn = tma ? bn_tma : (N <= 64 ? 64 : 128);
+  int bn = tma ? bn_tma : (N <= 64 ? 64 : 128);
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
   // Split K when the output has too few tiles to fill the GPU and K is long.  With more than
   // half a tile per SM the split costs more than it gives (2,048 x 2,048 x 512, 128 tiles: 11.9
@@ -1495,6 +1510,11 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   int k_chunk = (K + splits - 1) / splits;
   k_chunk = (k_chunk + BK - 1) / BK * BK;
   splits = (K + k_chunk - 1) / k_chunk;
+  // Narrower tiles while they leave the GPU half empty: 256 x 256 x 256, two tiles of 256
+  // columns, 13.5 us, eight of 64 7.3 (cold, under a profiler).  The sums of an output do not
+  // depend on its tile.
+  if (tma)
+    while (bn > 64 && 2LL * ((M + BM - 1) / BM) * ((N + bn - 1) / bn) * splits <= num_sms()) bn /= 2;
   float* partial = nullptr;
   const size_t part = splits > 1 ? align256(sizeof(float) * (size_t)splits * M * N) : 0;
   if (part + op.pack_bytes) {
@@ -1506,7 +1526,7 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   }
   CUtensorMap ta, tb;
   if (tma && !(make_tile_map(&ta, op.A, M, K, op.lda, BM) &&
-               make_tile_map(&tb, op.B, N, K, op.ldb, bn_tma)))
+               make_tile_map(&tb, op.B, N, K, op.ldb, bn)))
     return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: tensor map");
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, splits);
   cudaError_t le = cudaSuccess;
@@ -1540,8 +1560,8 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   }
   if (splits > 1) {
     const long long mn = (long long)M * N;
-    k_splitk_reduce<<<(unsigned)((mn + 255) / 256), 256, 0, st>>>(partial, splits, C, ldc, cb, M, N,
-                                                                  alpha, beta, bias, activation);
+    ci::launch_pdl(k_splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, st, partial, splits, C, ldc,
+                   cb, M, N, alpha, beta, bias, activation);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(e));

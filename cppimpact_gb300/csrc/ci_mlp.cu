@@ -4,7 +4,12 @@
 // The products of layers 2 and 3 are arranged as A B^T with both operands K-major (the
 // form of the TMA-pipelined tcgen05 kernel): BF16 copies of W2 and W3 are kept
 // transposed, and the weight gradients read transposed activations and output
-// gradients.
+// gradients.  A training batch is bound by its chain of small kernels, so what lies between
+// the products is fused into one kernel per product: layer 1 from the rows of X with its
+// transposed copy, the loss gradient with its transpose and bias gradient, the tanh
+// derivative with the same, Adam with the BF16 copies in both orders (23 launches a batch
+// before, 14 now, each set up while the one before runs, ci_pdl.h; 4 -> 256 -> 256 -> 5120, batches
+// of 256: 238 us a batch before, 97 now).
 //
 // Parameters, in the order ci_mlp_get_params / set_params use:
 //   W1 [n_in x H], b1 [H], W2 [H x H], b2 [H], W3 [H x n_out], b3 [n_out]
@@ -20,6 +25,7 @@
 #include <vector>
 
 #include "../../include/cppimpact_gb300.h"
+#include "ci_pdl.h"
 
 namespace ci {
 int set_last_error(int code, const char* msg);
@@ -43,27 +49,24 @@ using bf16 = __nv_bfloat16;
   } while (0)
 
 __global__ void k_to_bf16(const float* in, bf16* out, long long n) {
+  ci::pdl_next();
+  ci::pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) out[i] = __float2bfloat16(in[i]);
 }
 
-// dY = scale (Y - T) (scale = 2 / (rows * cols)) for row r = blockIdx.y, whose targets
-// are row idx[r] of T (row r when idx is null); with LOSS, per-block partial sums of
-// (Y - T)^2
-template <bool LOSS>
-__global__ void k_mse_grad(const float* Y, const float* T, const int* idx, int cols, float* dY,
-                           bf16* dYb, float scale, double* part) {
+// Per-block partial sums of (Y - T)^2 for row r = blockIdx.y, whose targets are row idx[r] of T
+// (row r when idx is null)
+__global__ void k_mse_loss(const float* Y, const float* T, const int* idx, int cols, double* part) {
+  ci::pdl_next();
+  ci::pdl_wait();
   __shared__ double red[256];
   const int r = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0.0;
   if (c < cols) {
-    const size_t i = (size_t)r * cols + c;
-    const float d = Y[i] - T[(size_t)(idx ? idx[r] : r) * cols + c];
-    dY[i] = scale * d;
-    dYb[i] = __float2bfloat16(scale * d);
+    const float d = Y[(size_t)r * cols + c] - T[(size_t)(idx ? idx[r] : r) * cols + c];
     s = (double)d * d;
   }
-  if (!LOSS) return;
   red[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
@@ -73,60 +76,128 @@ __global__ void k_mse_grad(const float* Y, const float* T, const int* idx, int c
   if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
 }
 
-// dZ = dH (1 - H^2)
-__global__ void k_tanh_back(const float* dH, const float* H, float* dZ, bf16* dZb, long long n) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n) {
-    const float v = dH[i] * (1.f - H[i] * H[i]);
-    dZ[i] = v;
-    dZb[i] = __float2bfloat16(v);
-  }
-}
-
-// column sums of a [rows x cols] matrix: 32 columns per CTA, 8 row groups (rows
-// r = g, g + 8, ... in order), then the 8 partial sums in group order
-__global__ void __launch_bounds__(256) k_colsum(const float* A, int rows, int cols, float* out) {
-  __shared__ float part[8][33];
-  const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + tx;
+// The passes over a [rows x cols] gradient between two products, CB columns and all rows per
+// CTA of 8 CB threads (thread: column tx, row group g): the value of entry (r, c) from `value`,
+// its BF16 copy in row order (vb, may be null) and transposed (vT, may be null), and the column
+// sums (group g of 8 sums rows r = g, g + 8, ... in order, then the 8 partial sums in group
+// order).  Products and sums are rounded one by one.  What bounds it is latency: 32 rows of a
+// thread are in flight at once (256 x 5,120, cold under a profiler: 8 behind branches about 25 us,
+// 14.4 so), and narrow gradients take 8 columns per CTA.
+template <int CB, class Value>
+__device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* vT, float* colsum,
+                                            Value value) {
+  ci::pdl_next();
+  ci::pdl_wait();
+  constexpr int U = 32, TR = 8 * U;  // rows per turn
+  __shared__ bf16 tile[CB][TR + 2];
+  __shared__ float part[8][CB];
+  const int tx = threadIdx.x % CB, g = threadIdx.x / CB;
+  const int c0 = blockIdx.x * CB, c = c0 + tx;
   float s = 0.f;
-  if (c < cols)
-    for (int r = g; r < rows; r += 8) s += A[(size_t)r * cols + c];
+  for (int r0 = 0; r0 < rows; r0 += TR) {
+    // (indices past the end load the last entry, so that no branch holds a load back)
+    float v[U];
+#pragma unroll
+    for (int i = 0; i < U; i++) v[i] = value(min(r0 + g + 8 * i, rows - 1), min(c, cols - 1));
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      const int r = r0 + g + 8 * i;
+      if (r < rows && c < cols) {
+        s = __fadd_rn(s, v[i]);
+        const bf16 h = __float2bfloat16(v[i]);
+        if (vb) vb[(size_t)r * cols + c] = h;
+        tile[tx][g + 8 * i] = h;
+      }
+    }
+    if (vT) {
+      __syncthreads();
+      for (int i = threadIdx.x; i < CB * TR; i += 8 * CB) {
+        const int k = i / TR, r = i % TR;
+        if (c0 + k < cols && r0 + r < rows) vT[(size_t)(c0 + k) * rows + r0 + r] = tile[k][r];
+      }
+      __syncthreads();
+    }
+  }
   part[g][tx] = s;
   __syncthreads();
   if (g == 0 && c < cols) {
     float t = part[0][tx];
     for (int k = 1; k < 8; k++) t += part[k][tx];
-    out[c] = t;
+    colsum[c] = t;
   }
 }
 
-// Layer 1 when n_in is small (the surrogate's 4 impact parameters): Z = tanh(X W1 + b1)
-// with the BF16 operands of the GEMM path, FP32 products summed in input order; writes
-// the FP32 activation and its BF16 copy.
-__global__ void k_layer1_fwd(const bf16* X, const bf16* W1, const float* b1, int rows, int n_in,
-                             int H, float* Z, bf16* Hb) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)rows * H) return;
-  const int r = (int)(i / H), h = (int)(i % H);
-  float acc = 0.f;
-  for (int k = 0; k < n_in; k++)
-    acc = fmaf(__bfloat162float(X[(size_t)r * n_in + k]), __bfloat162float(W1[(size_t)k * H + h]), acc);
-  const float z = tanhf(acc + b1[h]);
-  Z[i] = z;
-  Hb[i] = __float2bfloat16(z);
+// dY = scale (Y - T) (scale = 2 / (rows * cols)) for row r, whose targets are row idx[r] of T
+// (row r when idx is null): BF16 in both orders, and gb = its column sums
+template <int CB>
+__global__ void __launch_bounds__(8 * CB) k_mse_grad(const float* __restrict__ Y,
+                                                     const float* __restrict__ T,
+                                                     const int* __restrict__ idx, int rows, int cols,
+                                                     float scale, bf16* dYb, bf16* dYbT, float* gb) {
+  column_pass<CB>(rows, cols, dYb, dYbT, gb, [&](int r, int c) {
+    return __fmul_rn(scale, Y[(size_t)r * cols + c] - T[(size_t)(idx ? idx[r] : r) * cols + c]);
+  });
 }
 
-// gW1 = X^T dZ1 [n_in x H] for small n_in: one warp per entry; lane j sums rows j, j+32,
-// ... in order, then the 32 lane sums in a fixed butterfly order
-__global__ void k_layer1_wgrad(const bf16* X, const bf16* dZb, int rows, int n_in, int H, float* gW) {
+// dZ = dH (1 - H^2): BF16 in row order and transposed (either may be null), and gb
+template <int CB>
+__global__ void __launch_bounds__(8 * CB) k_tanh_back(const float* __restrict__ dH,
+                                                      const float* __restrict__ H, int rows,
+                                                      int cols, bf16* dZb, bf16* dZbT, float* gb) {
+  column_pass<CB>(rows, cols, dZb, dZbT, gb, [&](int r, int c) {
+    const size_t i = (size_t)r * cols + c;
+    const float h = H[i];
+    return __fmul_rn(dH[i], __fmaf_rn(-h, h, 1.f));
+  });
+}
+
+// Layer 1 when n_in is small (the surrogate's 4 impact parameters): Z = tanh(X W1 + b1)
+// with the BF16 operands of the GEMM path, FP32 products summed in input order, from row
+// idx[r] of X (row r when idx is null); the FP32 activation and its BF16 copies in row order
+// and (HbT, may be null) transposed.  32 x 32 entries per CTA.
+__global__ void __launch_bounds__(256) k_layer1_fwd(const float* X, const int* idx, const bf16* W1,
+                                                    const float* b1, int rows, int n_in, int H,
+                                                    float* Z, bf16* Hb, bf16* HbT) {
+  ci::pdl_next();
+  ci::pdl_wait();
+  __shared__ bf16 tile[32][34];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int h0 = blockIdx.x * 32, r0 = blockIdx.y * 32, h = h0 + tx;
+  for (int j = ty; j < 32; j += 8) {
+    const int r = r0 + j;
+    if (r < rows && h < H) {
+      const float* x = X + (size_t)(idx ? idx[r] : r) * n_in;
+      float acc = 0.f;
+      for (int k = 0; k < n_in; k++)
+        acc = fmaf(__bfloat162float(__float2bfloat16(x[k])), __bfloat162float(W1[(size_t)k * H + h]), acc);
+      const float z = tanhf(acc + b1[h]);
+      Z[(size_t)r * H + h] = z;
+      const bf16 zb = __float2bfloat16(z);
+      Hb[(size_t)r * H + h] = zb;
+      tile[j][tx] = zb;
+    }
+  }
+  if (!HbT) return;
+  __syncthreads();
+  for (int j = ty; j < 32; j += 8)
+    if (h0 + j < H && r0 + tx < rows) HbT[(size_t)(h0 + j) * rows + r0 + tx] = tile[tx][j];
+}
+
+// gW1 = X^T dZ1 [n_in x H] for small n_in from the transposed dZ1 [H x rows]: one warp per
+// entry; lane j sums rows j, j+32, ... in order, then the 32 lane sums in a fixed butterfly order
+__global__ void k_layer1_wgrad(const float* X, const int* idx, const bf16* dZbT, int rows, int n_in,
+                               int H, float* gW) {
+  ci::pdl_next();
+  ci::pdl_wait();
   const int w = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= n_in * H) return;
   const int k = w / H, h = w % H;
   float acc = 0.f;
+#pragma unroll 4
   for (int r = lane; r < rows; r += 32)
-    acc = fmaf(__bfloat162float(X[(size_t)r * n_in + k]), __bfloat162float(dZb[(size_t)r * H + h]), acc);
+    acc = fmaf(__bfloat162float(__float2bfloat16(X[(size_t)(idx ? idx[r] : r) * n_in + k])),
+               __bfloat162float(dZbT[(size_t)h * rows + r]), acc);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) gW[w] = acc;
@@ -136,6 +207,8 @@ __global__ void k_layer1_wgrad(const bf16* X, const bf16* dZb, int rows, int n_i
 // tiles through shared memory
 __global__ void __launch_bounds__(256) k_transpose_bf16(const bf16* in, int rows, int cols,
                                                         int ld_in, bf16* out, int ld_out) {
+  ci::pdl_next();
+  ci::pdl_wait();
   __shared__ bf16 tile[32][34];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -152,28 +225,94 @@ __global__ void __launch_bounds__(256) k_transpose_bf16(const bf16* in, int rows
 
 inline cudaError_t transpose_bf16(const bf16* in, int rows, int cols, bf16* out, cudaStream_t st) {
   const dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-  k_transpose_bf16<<<grid, 256, 0, st>>>(in, rows, cols, cols, out, rows);
-  return cudaGetLastError();
+  return ci::launch_pdl(k_transpose_bf16, grid, 256, 0, st, in, rows, cols, cols, out, rows);
 }
 
-// Adam (Kingma & Ba 2015) on FP32 master weights; refreshes the BF16 copy
-__global__ void k_adam(float* p, const float* g, float* m, float* v, bf16* pb, long long n, float lr,
-                       float b1, float b2, float eps, float c1, float c2) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float mh = mi / c1, vh = vi / c2;
-  const float pi = p[i] - lr * mh / (sqrtf(vh) + eps);
-  p[i] = pi;
-  if (pb) pb[i] = __float2bfloat16(pi);
+// Adam (Kingma & Ba 2015) on FP32 master weights, rounded one operation at a time; refreshes
+// the BF16 copy, which it returns
+struct AdamArgs {
+  float *p, *m, *v;
+  const float* g;
+  bf16* pb;
+  float lr, b1, b2, eps, c1, c2;
+};
+
+// N entries at once, entry i[k] used where on[k] (its loads are made in any case)
+template <int N>
+__device__ __forceinline__ void adam_step(const AdamArgs& A, const long long (&i)[N],
+                                          const bool (&on)[N], bf16 (&h)[N]) {
+  float g[N], m[N], v[N], p[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    g[k] = A.g[i[k]];
+    m[k] = A.m[i[k]];
+    v[k] = A.v[i[k]];
+    p[k] = A.p[i[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    m[k] = __fmaf_rn(1.f - A.b1, g[k], __fmul_rn(A.b1, m[k]));
+    v[k] = __fmaf_rn(__fmul_rn(1.f - A.b2, g[k]), g[k], __fmul_rn(A.b2, v[k]));
+    const float mh = m[k] / A.c1, vh = v[k] / A.c2;
+    p[k] = p[k] - __fmul_rn(A.lr, mh) / (sqrtf(vh) + A.eps);
+    h[k] = __float2bfloat16(p[k]);
+    if (on[k]) {
+      A.m[i[k]] = m[k];
+      A.v[i[k]] = v[k];
+      A.p[i[k]] = p[k];
+      A.pb[i[k]] = h[k];
+    }
+  }
+}
+
+// All parameters: W2 [H x H] and W3 [H x n_out] in 32 x 32 tiles, whose BF16 copies also go
+// transposed to wT (W2^T then W3^T), then the rest (W1 b1, b2, b3) by entries
+__global__ void __launch_bounds__(256) k_adam(const AdamArgs A, int n_in, int H, int n_out, bf16* wT) {
+  ci::pdl_next();
+  ci::pdl_wait();
+  __shared__ bf16 tile[32][34];
+  const int tr = (H + 31) / 32, t2 = tr * tr, tc3 = (n_out + 31) / 32, t3 = tr * tc3;
+  const long long o2 = (long long)n_in * H + H, o3 = o2 + (long long)H * H + H;
+  const int b = blockIdx.x;
+  if (b < t2 + t3) {
+    const bool third = b >= t2;
+    const int t = third ? b - t2 : b, ncol = third ? n_out : H, tc = third ? tc3 : tr;
+    const int r0 = t / tc * 32, c0 = t % tc * 32;
+    const long long off = third ? o3 : o2;
+    bf16* out = wT + (third ? (size_t)H * H : 0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    long long i[4];
+    bool on[4];
+    bf16 h[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int r = r0 + ty + 8 * k, c = c0 + tx;
+      on[k] = r < H && c < ncol;
+      i[k] = off + (long long)min(r, H - 1) * ncol + min(c, ncol - 1);
+    }
+    adam_step<4>(A, i, on, h);
+#pragma unroll
+    for (int k = 0; k < 4; k++) tile[ty + 8 * k][tx] = h[k];
+    __syncthreads();
+    for (int j = ty; j < 32; j += 8)
+      if (c0 + j < ncol && r0 + tx < H) out[(size_t)(c0 + j) * H + r0 + tx] = tile[tx][j];
+    return;
+  }
+  // the entries before W2, then b2, then b3
+  const long long e = (long long)(b - t2 - t3) * 256 + threadIdx.x;
+  if (e >= o2 + H + n_out) return;
+  const long long i[1] = {e < o2       ? e
+                          : e < o2 + H ? e + (long long)H * H
+                                       : e + (long long)H * H + (long long)H * n_out};
+  const bool on[1] = {true};
+  bf16 h[1];
+  adam_step<1>(A, i, on, h);
 }
 
 // rows of X picked by idx -> Xb (BF16)
 __global__ void k_gather_rows(const float* X, const int* idx, int rows, int nx, bf16* Xb) {
+  ci::pdl_next();
+  ci::pdl_wait();
   const int r = blockIdx.x;
   if (r >= rows) return;
   const int s = idx[r];
@@ -210,9 +349,9 @@ struct ci_mlp {
   DBuf<int> err;
   long long step = 0;
   int cap = 0;                // rows the activation buffers hold
-  DBuf<float> Z1, Z2, Y, dY, dH2, dZ2, dH1, dZ1;
+  DBuf<float> Z1, Z2, Y, dH2, dH1;
   DBuf<bf16> Xb, H1b, H2b, dYb, dZ2b, dZ1b;
-  DBuf<bf16> H1bT, H2bT, dYbT, dZ2bT;  // transposes [cols x rows] for the weight gradients
+  DBuf<bf16> H1bT, H2bT, dYbT, dZ2bT, dZ1bT;  // transposes [cols x rows] for the weight gradients
   DBuf<double> part;
   DBuf<int> idx;
 };
@@ -225,11 +364,8 @@ int ensure_cap(ci_mlp* M, int rows) {
   CM_CUDA(M->Z1.alloc(r * M->H));
   CM_CUDA(M->Z2.alloc(r * M->H));
   CM_CUDA(M->Y.alloc(r * M->n_out));
-  CM_CUDA(M->dY.alloc(r * M->n_out));
   CM_CUDA(M->dH2.alloc(r * M->H));
-  CM_CUDA(M->dZ2.alloc(r * M->H));
   CM_CUDA(M->dH1.alloc(r * M->H));
-  CM_CUDA(M->dZ1.alloc(r * M->H));
   CM_CUDA(M->Xb.alloc(r * M->n_in));
   CM_CUDA(M->H1b.alloc(r * M->H));
   CM_CUDA(M->H2b.alloc(r * M->H));
@@ -240,6 +376,7 @@ int ensure_cap(ci_mlp* M, int rows) {
   CM_CUDA(M->H2bT.alloc(r * M->H));
   CM_CUDA(M->dYbT.alloc(r * M->n_out));
   CM_CUDA(M->dZ2bT.alloc(r * M->H));
+  CM_CUDA(M->dZ1bT.alloc(r * M->H));
   CM_CUDA(M->part.alloc(r * nb(M->n_out)));
   CM_CUDA(M->idx.alloc(r));
   M->cap = rows;
@@ -259,8 +396,9 @@ int refresh_wT(ci_mlp* M, cudaStream_t st) {
   return CI_OK;
 }
 
-// forward of `rows` rows already in Xb; writes Y (and the hidden activations)
-int forward(ci_mlp* M, int rows, cudaStream_t st) {
+// forward of `rows` rows of X (idx[r], or r when idx is null); writes Y and the hidden
+// activations, with keep also what the weight gradients read of them
+int forward(ci_mlp* M, const float* X, const int* idx, int rows, bool keep, cudaStream_t st) {
   const bf16* W1 = M->pb.p + M->off[0];
   const bf16* W2T = M->wT.p;
   const bf16* W3T = M->wT.p + (size_t)M->H * M->H;
@@ -268,32 +406,32 @@ int forward(ci_mlp* M, int rows, cudaStream_t st) {
   const float* b2 = M->p.p + M->off[3];
   const float* b3 = M->p.p + M->off[5];
   if (M->n_in < 16) {
-    k_layer1_fwd<<<nb((long long)rows * M->H), 256, 0, st>>>(M->Xb.p, W1, b1, rows, M->n_in, M->H,
-                                                             M->Z1.p, M->H1b.p);
-    CM_CUDA(cudaGetLastError());
+    CM_CUDA(ci::launch_pdl(k_layer1_fwd, dim3((M->H + 31) / 32, (rows + 31) / 32), 256, 0, st, 
+        X, idx, W1, b1, rows, M->n_in, M->H, M->Z1.p, M->H1b.p, keep ? M->H1bT.p : nullptr));
   } else {
+    if (idx)
+      CM_CUDA(ci::launch_pdl(k_gather_rows, rows, 32, 0, st, X, idx, rows, M->n_in, M->Xb.p));
+    else
+      CM_CUDA(ci::launch_pdl(k_to_bf16, nb((long long)rows * M->n_in), 256, 0, st, X, M->Xb.p,
+                             (long long)rows * M->n_in));
     CM_OK(gemm(M, M->Xb.p, M->n_in, 0, W1, M->H, 0, M->Z1.p, M->H, M->H1b.p, rows, M->H, M->n_in,
                0.f, b1, 1, st));
+    if (keep) CM_CUDA(transpose_bf16(M->H1b.p, rows, M->H, M->H1bT.p, st));
   }
   CM_OK(gemm(M, M->H1b.p, M->H, 0, W2T, M->H, 1, M->Z2.p, M->H, M->H2b.p, rows, M->H, M->H, 0.f, b2,
              1, st));
+  if (keep) CM_CUDA(transpose_bf16(M->H2b.p, rows, M->H, M->H2bT.p, st));
   CM_OK(gemm(M, M->H2b.p, M->H, 0, W3T, M->H, 1, M->Y.p, M->n_out, nullptr, rows, M->n_out, M->H,
              0.f, b3, 0, st));
   return CI_OK;
 }
 
-// loss and gradients into M->g for `rows` rows in Xb, whose targets are rows idx[r] of T
-// (rows r when idx is null); *loss (may be NULL) gets the mean squared error (host,
+// loss and gradients into M->g after forward(keep) of the same rows, whose targets are rows
+// idx[r] of T (rows r when idx is null); *loss (may be NULL) gets the mean squared error (host,
 // synchronises)
-int backward(ci_mlp* M, int rows, cudaStream_t st, double* loss, const float* T, const int* idx) {
-  const long long ny = (long long)rows * M->n_out, nh = (long long)rows * M->H;
-  const dim3 mse_grid(nb(M->n_out), rows);
-  if (loss)
-    k_mse_grad<true><<<mse_grid, 256, 0, st>>>(M->Y.p, T, idx, M->n_out, M->dY.p, M->dYb.p,
-                                               2.0f / (float)ny, M->part.p);
-  else
-    k_mse_grad<false><<<mse_grid, 256, 0, st>>>(M->Y.p, T, idx, M->n_out, M->dY.p, M->dYb.p,
-                                                2.0f / (float)ny, M->part.p);
+int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows, cudaStream_t st,
+             double* loss) {
+  const long long ny = (long long)rows * M->n_out;
   float* gW1 = M->g.p + M->off[0];
   float* gb1 = M->g.p + M->off[1];
   float* gW2 = M->g.p + M->off[2];
@@ -302,36 +440,39 @@ int backward(ci_mlp* M, int rows, cudaStream_t st, double* loss, const float* T,
   float* gb3 = M->g.p + M->off[5];
   const bf16* W2 = M->pb.p + M->off[2];
   const bf16* W3 = M->pb.p + M->off[4];
+  if (loss) {
+    CM_CUDA(ci::launch_pdl(k_mse_loss, dim3(nb(M->n_out), rows), 256, 0, st, M->Y.p, T, idx, M->n_out, M->part.p));
+  }
   // layer 3: gW3 = H2^T dY as (H2^T) (dY^T)^T
-  CM_CUDA(transpose_bf16(M->H2b.p, rows, M->H, M->H2bT.p, st));
-  CM_CUDA(transpose_bf16(M->dYb.p, rows, M->n_out, M->dYbT.p, st));
+  const float scale = 2.0f / (float)ny;
+  const bool wide = M->n_out > 2048;
+  CM_CUDA(ci::launch_pdl(wide ? k_mse_grad<32> : k_mse_grad<8>,
+                         wide ? (M->n_out + 31) / 32 : (M->n_out + 7) / 8, wide ? 256 : 64, 0, st,
+                         M->Y.p, T, idx, rows, M->n_out, scale, M->dYb.p, M->dYbT.p, gb3));
   CM_OK(gemm(M, M->H2bT.p, rows, 0, M->dYbT.p, rows, 1, gW3, M->n_out, nullptr, M->H, M->n_out,
              rows, 0.f, nullptr, 0, st));
-  k_colsum<<<(M->n_out + 31) / 32, 256, 0, st>>>(M->dY.p, rows, M->n_out, gb3);
   CM_OK(gemm(M, M->dYb.p, M->n_out, 0, W3, M->n_out, 1, M->dH2.p, M->H, nullptr, rows, M->H,
              M->n_out, 0.f, nullptr, 0, st));
-  // Z2 holds tanh(Z2) = H2 (the GEMM wrote the activated values)
-  k_tanh_back<<<nb(nh), 256, 0, st>>>(M->dH2.p, M->Z2.p, M->dZ2.p, M->dZ2b.p, nh);
-  // layer 2: gW2 = H1^T dZ2 as (H1^T) (dZ2^T)^T
-  CM_CUDA(transpose_bf16(M->H1b.p, rows, M->H, M->H1bT.p, st));
-  CM_CUDA(transpose_bf16(M->dZ2b.p, rows, M->H, M->dZ2bT.p, st));
+  // layer 2: gW2 = H1^T dZ2 as (H1^T) (dZ2^T)^T; Z2 holds tanh(Z2) = H2 (the GEMM wrote the
+  // activated values)
+  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, (M->H + 7) / 8, 64, 0, st, M->dH2.p, M->Z2.p, rows, M->H, M->dZ2b.p,
+                                               M->dZ2bT.p, gb2));
   CM_OK(gemm(M, M->H1bT.p, rows, 0, M->dZ2bT.p, rows, 1, gW2, M->H, nullptr, M->H, M->H, rows, 0.f,
              nullptr, 0, st));
-  k_colsum<<<(M->H + 31) / 32, 256, 0, st>>>(M->dZ2.p, rows, M->H, gb2);
   CM_OK(gemm(M, M->dZ2b.p, M->H, 0, W2, M->H, 1, M->dH1.p, M->H, nullptr, rows, M->H, M->H, 0.f,
              nullptr, 0, st));
-  k_tanh_back<<<nb(nh), 256, 0, st>>>(M->dH1.p, M->Z1.p, M->dZ1.p, M->dZ1b.p, nh);
   // layer 1
-  if (M->n_in < 16) {
-    k_layer1_wgrad<<<nb(32LL * M->n_in * M->H), 256, 0, st>>>(M->Xb.p, M->dZ1b.p, rows, M->n_in,
-                                                               M->H, gW1);
-    CM_CUDA(cudaGetLastError());
+  const bool small = M->n_in < 16;
+  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, (M->H + 7) / 8, 64, 0, st, M->dH1.p, M->Z1.p, rows, M->H,
+                                               small ? nullptr : M->dZ1b.p,
+                                               small ? M->dZ1bT.p : nullptr, gb1));
+  if (small) {
+    CM_CUDA(ci::launch_pdl(k_layer1_wgrad, nb(32LL * M->n_in * M->H), 256, 0, st, X, idx, M->dZ1bT.p, rows, M->n_in,
+                                                               M->H, gW1));
   } else {
     CM_OK(gemm(M, M->Xb.p, M->n_in, 1, M->dZ1b.p, M->H, 0, gW1, M->H, nullptr, M->n_in, M->H, rows,
                0.f, nullptr, 0, st));
   }
-  k_colsum<<<(M->H + 31) / 32, 256, 0, st>>>(M->dZ1.p, rows, M->H, gb1);
-  CM_CUDA(cudaGetLastError());
   if (loss) {
     std::vector<double> part((size_t)rows * nb(M->n_out));
     CM_CUDA(cudaMemcpyAsync(part.data(), M->part.p, sizeof(double) * part.size(),
@@ -426,9 +567,7 @@ int ci_mlp_predict(ci_mlp* M, const float* d_X, int n, float* d_Y, void* stream)
   for (int r0 = 0; r0 < n; r0 += 4096) {
     const int rows = std::min(4096, n - r0);
     CM_OK(ensure_cap(M, rows));
-    k_to_bf16<<<nb((long long)rows * M->n_in), 256, 0, st>>>(d_X + (size_t)r0 * M->n_in, M->Xb.p,
-                                                             (long long)rows * M->n_in);
-    CM_OK(forward(M, rows, st));
+    CM_OK(forward(M, d_X + (size_t)r0 * M->n_in, nullptr, rows, false, st));
     CM_CUDA(cudaMemcpyAsync(d_Y + (size_t)r0 * M->n_out, M->Y.p, sizeof(float) * rows * M->n_out,
                             cudaMemcpyDeviceToDevice, st));
   }
@@ -439,12 +578,8 @@ int ci_mlp_gradients(ci_mlp* M, const float* d_X, const float* d_T, int n, float
                      double* loss) {
   if (!M || !d_X || !d_T || n <= 0) return ci::set_last_error(CI_ERR_INVALID, "bad argument");
   CM_OK(ensure_cap(M, n));
-  std::vector<int> idx(n);
-  for (int i = 0; i < n; i++) idx[i] = i;
-  CM_CUDA(cudaMemcpy(M->idx.p, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  k_gather_rows<<<n, 32>>>(d_X, M->idx.p, n, M->n_in, M->Xb.p);
-  CM_OK(forward(M, n, 0));
-  CM_OK(backward(M, n, 0, loss, d_T, nullptr));
+  CM_OK(forward(M, d_X, nullptr, n, true, 0));
+  CM_OK(backward(M, d_X, d_T, nullptr, n, 0, loss));
   if (h_grad) CM_CUDA(cudaMemcpy(h_grad, M->g.p, sizeof(float) * M->np, cudaMemcpyDeviceToHost));
   return check_err(M, 0);
 }
@@ -466,19 +601,20 @@ int ci_mlp_train(ci_mlp* M, const float* d_X, const float* d_T, int n, int batch
     double ep_loss = 0.0;
     int nbatches = 0;
     for (int b0 = 0; b0 + batch <= n; b0 += batch) {
-      k_gather_rows<<<batch, 32, 0, st>>>(d_X, M->idx.p + b0, batch, M->n_in, M->Xb.p);
-      CM_OK(forward(M, batch, st));
+      const int* idx = M->idx.p + b0;
+      CM_OK(forward(M, d_X, idx, batch, true, st));
       const bool last = b0 + 2 * batch > n;
       double l = 0.0;
-      CM_OK(backward(M, batch, st, (h_loss && last) ? &l : nullptr, d_T, M->idx.p + b0));
+      CM_OK(backward(M, d_X, d_T, idx, batch, st, (h_loss && last) ? &l : nullptr));
       ep_loss += l;
       nbatches += last ? 1 : 0;
       M->step++;
       const float c1 = 1.f - std::pow(b1, (float)M->step), c2 = 1.f - std::pow(b2, (float)M->step);
-      k_adam<<<nb(M->np), 256, 0, st>>>(M->p.p, M->g.p, M->m.p, M->v.p, M->pb.p, M->np, lr, b1, b2,
-                                        eps, c1, c2);
-      CM_CUDA(cudaGetLastError());
-      CM_OK(refresh_wT(M, st));
+      const AdamArgs A{M->p.p, M->m.p, M->v.p, M->g.p, M->pb.p, lr, b1, b2, eps, c1, c2};
+      const int tr = (M->H + 31) / 32;
+      const long long rest = (long long)M->n_in * M->H + 2LL * M->H + M->n_out;
+      CM_CUDA(ci::launch_pdl(k_adam, (unsigned)(tr * tr + tr * ((M->n_out + 31) / 32)) + nb(rest), 256, 0, st, 
+          A, M->n_in, M->H, M->n_out, M->wT.p));
     }
     if (h_loss) h_loss[ep] = nbatches ? ep_loss / nbatches : 0.0;
   }
