@@ -82,8 +82,10 @@ struct Group {
   int npe = 0, nq = 0;
   int N = 0, E = 0, C = 0, n_bnd = 0;
   long long S = 0, Lt = 0;
-  int max_local = 0;
+  int max_local = 0, max_chunk_elems = 0;
   size_t smem = 0;
+  bool repeats = false;  // Plan::repeats of any instance
+  StepForm step;  // of the tet4 step kernel
   int block_threads = 128, elem_lanes = 4, chunk_nodes = 896, chunk_elements = 0;
   float tuned_ms_per_step = 0.f;  // autotuner's trial time of the chosen shape (0: not tuned)
   std::vector<int> insts;  // global instance ids
@@ -93,6 +95,8 @@ struct Group {
   DBuf<ChunkInfo> chunks;
   DBuf<uint16_t> conn;
   DBuf<uint8_t> color;
+  DBuf<uint4> conn8;  // tet10
+  DBuf<uint2> conn2;
   DBuf<int> lgid, lslot, lsrow, slot_row, bnd, node_inst;
   DBuf<float> lx0, slot0, slot1, mass, d0f, acc, epbar, peak;
   DBuf<double> ua, va, ub, vb, v0, d0, work;
@@ -177,6 +181,8 @@ FusedArgs group_args(const Group& G, int i_in_graph) {
   F.P.chunks = G.chunks.p;
   F.P.conn_local = G.conn.p;
   F.P.color = G.color.p;
+  F.P.conn8 = G.conn8.p;
+  F.P.conn2 = G.conn2.p;
   F.P.local_gid = G.lgid.p;
   F.P.local_slot = G.lslot.p;
   F.P.local_srow = reinterpret_cast<const int2*>(G.lsrow.p);
@@ -215,50 +221,56 @@ FusedArgs group_args(const Group& G, int i_in_graph) {
   return F;
 }
 
-template <int NPE, int BS>
-cudaError_t launch_batch_bs(Group& G, const FusedArgs& F) {
-  const ElemParams ep{};
-  const NodeParams np{};
-  if (NPE == 10 && G.elem_lanes == 4)
-    k_step_qp10<EM_J2, BS, true><<<G.C, BS, G.smem, G.stream>>>(F, ep, np);
-  else if (NPE == 10)
-    k_step_t10<EM_J2, BS, true><<<G.C, BS, G.smem, G.stream>>>(F, ep, np);
-  else
-    k_step<NPE, EM_J2, BS, true><<<G.C, BS, G.smem, G.stream>>>(F, ep, np);
+template <int BS>
+StepKernel batch_kernel10(int elem_lanes) {
+  return elem_lanes == 4 ? k_step_qp10<EM_J2, BS, true> : k_step_t10<EM_J2, BS, true>;
+}
+
+// The form of the group's tet4 step kernel at its present shape; before a capture of it.
+cudaError_t prepare_step(Group& G) {
+  if (G.npe != 4) return cudaSuccess;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e) return e;
+  G.step = step_form(G.C, device, G.block_threads, G.max_local, G.max_chunk_elems);
+  return configure_step_kernel<EM_J2, true>(G.block_threads, G.step, device);
+}
+
+cudaError_t launch_batch(Group& G, const FusedArgs& F) {
+  const int bs = G.block_threads;
+  if (G.npe == 4) {
+    step_kernel<EM_J2, true>(bs, G.step)<<<G.C, bs * G.step.W, G.step.smem, G.stream>>>(
+        F, ElemParams{}, NodeParams{});
+    return cudaGetLastError();
+  }
+  const int lanes = G.repeats ? 1 : G.elem_lanes;
+  const StepKernel k = bs == 64    ? batch_kernel10<64>(lanes)
+                       : bs == 256 ? batch_kernel10<256>(lanes)
+                                   : batch_kernel10<128>(lanes);
+  k<<<G.C, bs, G.smem, G.stream>>>(F, ElemParams{}, NodeParams{});
   return cudaGetLastError();
 }
 
-template <int NPE>
-cudaError_t launch_batch(Group& G, const FusedArgs& F) {
-  if (G.block_threads == 64) return launch_batch_bs<NPE, 64>(G, F);
-  if (G.block_threads == 256) return launch_batch_bs<NPE, 256>(G, F);
-  return launch_batch_bs<NPE, 128>(G, F);
-}
-
-template <int NPE, int BS>
-cudaError_t configure_bs(int bytes) {
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_step<NPE, EM_J2, BS, true>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  if (NPE == 10) {
-    if ((e = cudaFuncSetAttribute(k_step_qp10<EM_J2, BS, true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    if ((e = cudaFuncSetAttribute(k_step_t10<EM_J2, BS, true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-  }
-  return cudaFuncSetAttribute(k_elem<NPE, EM_MASS_HRZ, 256>,
+template <int BS>
+cudaError_t configure10(int bytes) {
+  cudaError_t e = cudaFuncSetAttribute(k_step_qp10<EM_J2, BS, true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e) return e;
+  return cudaFuncSetAttribute(k_step_t10<EM_J2, BS, true>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 template <int NPE>
 cudaError_t configure(int bytes) {
   cudaError_t e;
-  if ((e = configure_bs<NPE, 64>(bytes))) return e;
-  if ((e = configure_bs<NPE, 128>(bytes))) return e;
-  if ((e = configure_bs<NPE, 256>(bytes))) return e;
+  if (NPE == 10) {
+    if ((e = configure10<64>(bytes))) return e;
+    if ((e = configure10<128>(bytes))) return e;
+    if ((e = configure10<256>(bytes))) return e;
+  }
+  if ((e = cudaFuncSetAttribute(k_elem<NPE, EM_MASS_HRZ, 256>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
   return cudaFuncSetAttribute(k_elem<NPE, EM_MASS_ROWSUM, 256>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
@@ -313,7 +325,8 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   // sizes and offsets
   G.N = G.E = G.C = 0;
   G.S = G.Lt = 0;
-  G.max_local = 0;
+  G.max_local = G.max_chunk_elems = 0;
+  G.repeats = false;
   for (size_t j = 0; j < plans.size(); j++) {
     Inst& T = b->inst[G.insts[j]];
     const Plan& P = *plans[j];
@@ -327,6 +340,8 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
     G.S += P.slot_row[P.N];
     G.Lt += (long long)P.local_gid.size();
     G.max_local = std::max(G.max_local, P.max_local);
+    G.repeats |= P.repeats;
+    G.max_chunk_elems = std::max(G.max_chunk_elems, P.max_chunk_elems);
   }
   const int npe = G.npe;
   std::vector<ChunkInfo> chunks;
@@ -404,6 +419,13 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   CB_CUDA(G.chunks.upload(chunks, st));
   CB_CUDA(G.conn.upload(conn, st));
   CB_CUDA(G.color.upload(color, st));
+  if (npe == 10) {
+    CB_CUDA(G.conn8.alloc(G.E));
+    CB_CUDA(G.conn2.alloc(G.E));
+    k_pack_conn10<<<(G.E + 255) / 256, 256, 0, st>>>(G.conn.p, G.color.p, (int)G.E, G.conn8.p,
+                                                   G.conn2.p);
+    CB_CUDA(cudaGetLastError());
+  }
   CB_CUDA(G.lgid.upload(lgid, st));
   CB_CUDA(G.lslot.upload(lslot, st));
   CB_CUDA(G.lsrow.upload(lsrow, st));
@@ -584,12 +606,13 @@ int capture_graph(Group& G) {
   if (G.graph) cudaGraphExecDestroy(G.graph);
   G.graph = nullptr;
   if (resident(G)) return CI_OK;  // runs without one
+  CB_CUDA(prepare_step(G));
   cudaGraph_t g = nullptr;
   CB_CUDA(cudaStreamBeginCapture(G.stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   for (int i = 0; i < kGraphSteps && err == cudaSuccess; i++) {
     const FusedArgs F = group_args(G, i);
-    err = G.npe == 4 ? launch_batch<4>(G, F) : launch_batch<10>(G, F);
+    err = launch_batch(G, F);
   }
   if (err == cudaSuccess) {
     k_tick<<<1, 1, 0, G.stream>>>(G.step_ctr.p, kGraphSteps);
@@ -1041,7 +1064,7 @@ int run_intervals(ci_batch* b, int every, const Snapshots& sn, float* device_ms,
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < every && err == cudaSuccess; i++) {
       const FusedArgs F = group_args(G, i);
-      err = G.npe == 4 ? launch_batch<4>(G, F) : launch_batch<10>(G, F);
+      err = launch_batch(G, F);
     }
     if (err == cudaSuccess) {
       k_tick<<<1, 1, 0, G.stream>>>(G.step_ctr.p, every);

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kThreads) k_energy_partials(const double* __re
     ci::DevState S{};
     S.status = status;
     float f[NPE][3];
-    ci::element_force<NPE, ci::EM_REFCOMPAT>(p, S, e, E, xe, ue, f, wint, wp, vol);
+    ci::element_force<NPE, ci::EM_REFCOMPAT>(p, S, e, xe, ue, f, wint, wp, vol);
   }
   const float t0 = ci::block_sum<kThreads>(wint, red);
   const float t1 = ci::block_sum<kThreads>(vol, red);

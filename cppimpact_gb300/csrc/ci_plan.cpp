@@ -211,6 +211,8 @@ bool build_plan(int N, int E, int npe, const double* xloc, const int* conn, int 
         lo_m |= used_lo[P.node_new[en[a]]];
         hi_m |= used_hi[P.node_new[en[a]]];
       }
+      for (int a = 1; a < npe; a++)
+        for (int b = 0; b < a; b++) P.repeats |= en[a] == en[b];
       int k;
       if (~lo_m) {
         k = __builtin_ctzll(~lo_m);

@@ -41,6 +41,7 @@ struct Plan {
   int n_chunks = 0;
   int max_local = 0, max_colors = 0, max_chunk_elems = 0;
   long long n_ghosts = 0, n_boundary = 0;
+  bool repeats = false;  // an element names a node twice: not for the four-lane step kernels
   std::vector<ChunkInfo> chunks;
   std::vector<int> elem_orig;        // plan element -> original element
   std::vector<uint16_t> conn_local;  // [npe][E] local node ids, SoA by corner

@@ -452,7 +452,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
               du[a][c] = pr[c].y;
             }
           }
-          element_force<NPE, MODE>(ep, S, CHIP ? i : ch.elem_begin + i, E, x, du, f, wint, wp, vol);
+          element_force<NPE, MODE>(ep, S, CHIP ? i : ch.elem_begin + i, x, du, f, wint, wp, vol);
           if (CHIP)
 #pragma unroll
             for (int a = 0; a < NPE; a++) fbuf[a * ne + i] = make_float4(f[a][0], f[a][1], f[a][2], 0.f);

@@ -90,11 +90,14 @@ struct ci_solver {
   bool started = false;
   long long steps_done = 0;
   size_t smem_bytes = 0;
+  ci::StepForm step;  // of the tet4 step kernel
 
   // device plan
   DBuf<ci::ChunkInfo> d_chunks;
   DBuf<uint16_t> d_conn;
   DBuf<uint8_t> d_color;
+  DBuf<uint4> d_conn8;  // tet10
+  DBuf<uint2> d_conn2;
   DBuf<int> d_lgid, d_lslot, d_slot_row, d_lsrow;
   DBuf<float> d_lx0;  // [3][Lt]
   // state (A buffer = d_u/d_v always holds the state between calls; B is the fused
@@ -156,6 +159,8 @@ struct ci_solver {
     P.chunks = d_chunks.p;
     P.conn_local = d_conn.p;
     P.color = d_color.p;
+    P.conn8 = d_conn8.p;
+    P.conn2 = d_conn2.p;
     P.local_gid = d_lgid.p;
     P.local_slot = d_lslot.p;
     P.local_srow = reinterpret_cast<const int2*>(d_lsrow.p);
@@ -266,26 +271,19 @@ cudaError_t launch_elem(ci_solver* s, const ci::DevState& D, const ci::ElemParam
   return cudaGetLastError();
 }
 
-template <int NPE, int BS>
-cudaError_t configure_step(int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(ci::k_step<NPE, ci::EM_J2, BS>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e) return e;
-  if (NPE == 10) {
-    if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_J2, BS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_REFCOMPAT, BS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    if ((e = cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_J2, BS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    if ((e = cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_REFCOMPAT, BS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-  }
-  return cudaFuncSetAttribute(ci::k_step<NPE, ci::EM_REFCOMPAT, BS>,
+template <int BS>
+cudaError_t configure_step10(int bytes) {
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_J2, BS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
+  if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_REFCOMPAT, BS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
+  if ((e = cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_J2, BS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
+  return cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_REFCOMPAT, BS>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
@@ -303,34 +301,24 @@ cudaError_t configure_npe(int bytes) {
   if ((e = cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_MASS_ROWSUM, kBS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
     return e;
-  if ((e = configure_step<NPE, 64>(bytes))) return e;
-  if ((e = configure_step<NPE, 128>(bytes))) return e;
-  if ((e = configure_step<NPE, 256>(bytes))) return e;
+  if (NPE == 10) {
+    if ((e = configure_step10<64>(bytes))) return e;
+    if ((e = configure_step10<128>(bytes))) return e;
+    if ((e = configure_step10<256>(bytes))) return e;
+  }
   return cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_MASS_HRZ, kBS>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-template <int NPE, int BS>
-cudaError_t launch_fused_bs(ci_solver* s, const ci::FusedArgs& F, const ci::ElemParams& ep,
-                            const ci::NodeParams& np) {
-  if (NPE == 10 && s->opt.elem_lanes == 4) {
-    if (s->opt.mode != CI_MODE_REFCOMPAT)
-      ci::k_step_qp10<ci::EM_J2, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-    else
-      ci::k_step_qp10<ci::EM_REFCOMPAT, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-    return cudaGetLastError();
-  }
-  if (NPE == 10) {
-    if (s->opt.mode != CI_MODE_REFCOMPAT)
-      ci::k_step_t10<ci::EM_J2, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-    else
-      ci::k_step_t10<ci::EM_REFCOMPAT, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-    return cudaGetLastError();
-  }
-  if (s->opt.mode != CI_MODE_REFCOMPAT)
-    ci::k_step<NPE, ci::EM_J2, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-  else
-    ci::k_step<NPE, ci::EM_REFCOMPAT, BS><<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
+template <int BS>
+cudaError_t launch_fused10(ci_solver* s, const ci::FusedArgs& F, const ci::ElemParams& ep,
+                           const ci::NodeParams& np) {
+  const bool j2 = s->opt.mode != CI_MODE_REFCOMPAT;
+  const ci::StepKernel k =
+      s->opt.elem_lanes == 4 && !s->plan.repeats
+          ? (j2 ? ci::k_step_qp10<ci::EM_J2, BS> : ci::k_step_qp10<ci::EM_REFCOMPAT, BS>)
+          : (j2 ? ci::k_step_t10<ci::EM_J2, BS> : ci::k_step_t10<ci::EM_REFCOMPAT, BS>);
+  k<<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
   return cudaGetLastError();
 }
 
@@ -339,13 +327,15 @@ cudaError_t launch_fused(ci_solver* s, const ci::FusedArgs& F) {
   const ci::NodeParams np = s->node_params();
   const int bs = s->opt.block_threads;
   if (s->npe == 4) {
-    if (bs == 64) return launch_fused_bs<4, 64>(s, F, ep, np);
-    if (bs == 128) return launch_fused_bs<4, 128>(s, F, ep, np);
-    return launch_fused_bs<4, 256>(s, F, ep, np);
+    const ci::StepKernel k = s->opt.mode != CI_MODE_REFCOMPAT
+                                 ? ci::step_kernel<ci::EM_J2, false>(bs, s->step)
+                                 : ci::step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step);
+    k<<<s->C, bs * s->step.W, s->step.smem, s->stream>>>(F, ep, np);
+    return cudaGetLastError();
   }
-  if (bs == 64) return launch_fused_bs<10, 64>(s, F, ep, np);
-  if (bs == 128) return launch_fused_bs<10, 128>(s, F, ep, np);
-  return launch_fused_bs<10, 256>(s, F, ep, np);
+  if (bs == 64) return launch_fused10<64>(s, F, ep, np);
+  if (bs == 128) return launch_fused10<128>(s, F, ep, np);
+  return launch_fused10<256>(s, F, ep, np);
 }
 
 cudaError_t launch_finalize(ci_solver* s, const ci::FusedArgs& F) {
@@ -689,6 +679,17 @@ int setup_resident(ci_solver* s) {
   CI_CUDA(cudaMemsetAsync(s->d_res_halo.p, 0, sizeof(float4) * 2 * (size_t)s->S, s->stream));
   CI_CUDA(cudaMemsetAsync(s->d_res_abort.p, 0, sizeof(int), s->stream));
   CI_CUDA(cudaStreamSynchronize(s->stream));
+  return CI_OK;
+}
+
+// Form of the tet4 step kernel.
+int setup_step(ci_solver* s) {
+  const ci::Plan& P = s->plan;
+  s->step = ci::step_form(s->C, s->device, s->opt.block_threads, P.max_local, P.max_chunk_elems);
+  const int bs = s->opt.block_threads;
+  CI_CUDA(s->opt.mode != CI_MODE_REFCOMPAT
+              ? (ci::configure_step_kernel<ci::EM_J2, false>(bs, s->step, s->device))
+              : (ci::configure_step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step, s->device)));
   return CI_OK;
 }
 
@@ -1097,6 +1098,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   s->vel0.assign(3, 0.0);
 
   CI_CUDA(s->npe == 4 ? configure_npe<4>((int)s->smem_bytes) : configure_npe<10>((int)s->smem_bytes));
+  if (s->plan.repeats && s->opt.step_kernel != 1) s->opt.step_kernel = 3;  // not the task kernel
   if (s->opt.step_kernel == 0) {
     // automatic: the task kernel when the chunks of a four-lane tet10 mesh need more than
     // 0.8 of a round of the fused kernel's resident CTAs -- meshes whose chunks are cut by
@@ -1126,6 +1128,13 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   if ((rc = upload(s->d_chunks, P.chunks, s->stream))) return rc;
   if ((rc = upload(s->d_conn, P.conn_local, s->stream))) return rc;
   if ((rc = upload(s->d_color, P.color, s->stream))) return rc;
+  if (s->npe == 10) {
+    CI_CUDA(s->d_conn8.alloc(s->E));
+    CI_CUDA(s->d_conn2.alloc(s->E));
+    ci::k_pack_conn10<<<(s->E + 255) / 256, 256, 0, s->stream>>>(s->d_conn.p, s->d_color.p, s->E,
+                                                               s->d_conn8.p, s->d_conn2.p);
+    CI_CUDA(cudaGetLastError());
+  }
   if ((rc = upload(s->d_lgid, P.local_gid, s->stream))) return rc;
   if ((rc = upload(s->d_lslot, P.local_slot, s->stream))) return rc;
   if ((rc = upload(s->d_lsrow, P.local_srow, s->stream))) return rc;
@@ -1142,6 +1151,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   }
   if (s->opt.step_kernel == 2 && (rc = setup_flow(s.get()))) return rc;
   if (s->opt.step_kernel == 3 && (rc = setup_resident(s.get()))) return rc;
+  if (s->npe == 4 && (rc = setup_step(s.get()))) return rc;
   CI_CUDA(s->d_mass.alloc(N));
   CI_CUDA(s->d_d0.alloc(N));
   CI_CUDA(s->d_d0f.alloc(N));
