@@ -1477,7 +1477,8 @@ __global__ void __launch_bounds__(BS, 768 / BS) k_step_qp10(FusedArgs A, ElemPar
 // A call of n steps is one launch whose CTAs claim tasks from a counter, in the order
 //   N(0, .);  then for j = 0 .. n-1:  E(j, .), N(j+1, .),
 // each block in one task order of the chunks (reverse Cuthill-McKee on the graph of
-// chunks sharing a node, so that a task's dependencies lie about one block back).
+// chunks sharing a node, so that a task's dependencies lie about one block back), or with
+// the two kinds in turns (flow_decode).
 // N(j, c): chunk c completes S^j of the nodes it owns -- from S^{j-1} and the halo of step
 //   j-1 exactly as the fused kernel's staging does (N(0) reads the state as it is, N(n)
 //   also stores the accelerations) -- and writes each node's record (u and dt v rounded to
@@ -1519,6 +1520,7 @@ struct FlowArgs {
   int* abort_flag;
   int C;
   int nsteps;
+  int lag;  // of the node tasks behind the element tasks, in tasks; 0: block by block
   unsigned long long wait_ns;  // a wait gives up after this long without progress
   int stall_chunk;             // test hook: this chunk never publishes (-1: none)
 };
@@ -1586,28 +1588,39 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Task t: j (the step whose state it completes or uses), position r of its chunk in the
-// task order, element or node task.  Order: N(0, .) for every chunk, then per step j the
-// element tasks E(j, .) and the node tasks N(j + 1, .), each block in the task order of
-// the chunks.
-__device__ __forceinline__ void flow_decode(int t, int C, int& j, int& r, bool& elem) {
+// task order, element or node task.  Order: N(0, .) for every chunk; then, block by block
+// (lag 0), per step j the element tasks E(j, .) and the node tasks N(j + 1, .), each block in
+// the task order of the chunks, or the element tasks of all steps and the node tasks of all
+// steps in turns, the latter lag tasks behind.
+__device__ __forceinline__ void flow_decode(const FlowArgs& F, int t, int& j, int& r, bool& elem) {
+  const int C = F.C;
   if (t < C) {
     j = 0;
     r = t;
     elem = false;
-  } else {
-    const int q = (t - C) % (2 * C);
-    j = (t - C) / (2 * C);
-    elem = q < C;
-    r = elem ? q : q - C;
-    if (!elem) j++;
+    return;
   }
+  int k = t - C;  // then the number of the task among those of its kind
+  if (F.lag == 0) {
+    elem = k % (2 * C) < C;
+    k = k / (2 * C) * C + k % C;
+  } else if (k < F.lag) {
+    elem = true;
+  } else {
+    k -= F.lag;
+    const int both = F.C * F.nsteps - F.lag;
+    elem = k < 2 * both && (k & 1) == 0;
+    k = k < 2 * both ? (elem ? F.lag + k / 2 : k / 2) : k - both;
+  }
+  j = k / C + (elem ? 0 : 1);
+  r = k % C;
 }
 
 // One warp: copy task t's descriptor into buf (one commit group).
 __device__ __forceinline__ void flow_fetch(const FlowArgs& F, int t, int* buf) {
   int j, r;
   bool elem;
-  flow_decode(t, F.C, j, r, elem);
+  flow_decode(F, t, j, r, elem);
   const int* src = F.desc + ((size_t)(elem ? 0 : F.C) + r) * F.desc_stride;
   for (int k = threadIdx.x & 31; 4 * k < F.desc_stride; k += 32) cp_async16(buf + 4 * k, src + 4 * k);
   cp_async_commit();
@@ -1782,7 +1795,7 @@ __global__ void __launch_bounds__(BS, 768 / BS) k_flow_qp10(FlowArgs F, ElemPara
       if (t < ntasks) {
         int j, r;
         bool elem;
-        flow_decode(t, F.C, j, r, elem);
+        flow_decode(F, t, j, r, elem);
         if (threadIdx.x == 0) tn = atomicAdd(F.task_ctr, 1);
         ok = elem ? flow_wait(F, F.node_done, dcur + kFlowDescHead, dcur[kFlowDescCount], j)
                   : (j == 0 || flow_wait(F, F.elem_done, dcur + kFlowDescHead,
@@ -1801,7 +1814,7 @@ __global__ void __launch_bounds__(BS, 768 / BS) k_flow_qp10(FlowArgs F, ElemPara
     if (t >= F.C + 2 * F.C * F.nsteps || !sh_ok) break;
     int j, r;
     bool elem;
-    flow_decode(t, F.C, j, r, elem);
+    flow_decode(F, t, j, r, elem);
     // the descriptor is read here only: after the task's last barrier warp 0 overwrites
     // it with the next task's
     ChunkInfo ch;
@@ -1817,7 +1830,7 @@ __global__ void __launch_bounds__(BS, 768 / BS) k_flow_qp10(FlowArgs F, ElemPara
       // read again: not kept in registers through the element loop
       memcpy(&ch, dcur, sizeof(ChunkInfo));
       c = dcur[kFlowDescChunk];
-      flow_decode(sh_cur, F.C, j, r, elem);
+      flow_decode(F, sh_cur, j, r, elem);
       node_epilogue<BS>(F.A[j & 1], ch, make_tile(sm + 2 * F.desc_stride, ch.n_local), threadIdx.x);
       if (ep.accum_energy) add_chunk_work<BS>(F.A[0], c, wint, wp, red);
       __syncthreads();

@@ -131,7 +131,7 @@ struct ci_solver {
   // and the abort flag ([2C + 2] ints), and the CTAs it keeps resident
   DBuf<float4> d_rec;  // task kernel records: [2][N] float4 then [2][N] float2
   DBuf<int> d_flow_desc, d_flow_ctr;
-  int flow_ctas = 0, flow_stride = 0;
+  int flow_ctas = 0, flow_stride = 0, flow_lag = 0;
   unsigned long long flow_wait_ns = ci::kFlowWaitNs;
   int flow_stall_chunk = -1;  // test hook, for the next task-kernel launch only
   size_t flow_smem = 0;
@@ -600,6 +600,21 @@ int setup_flow(ci_solver* s) {
   CI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, s->flow_smem));
   CI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
   s->flow_ctas = std::max(1, std::min(per_sm * sms, C));
+  // Element and node tasks in turns, the node tasks C / 2 behind, where no task then depends on
+  // one that is claimed less than half of the CTAs' claims before it: the SMs hold both kinds
+  // at any time, the ones bound by issue and the others by memory (604,800-element shell, C
+  // 2,067, dependencies up to 323 ahead in the order: 96.6 -> 93.3 us per step).  Else block by
+  // block: half of the shell, 1,023 and 113, 56.9 in turns and 55.6 so, a cube of 384,000
+  // elements 78.0 and 70.4.
+  std::vector<int> pos(C);
+  for (int r = 0; r < C; r++) pos[order[r]] = r;
+  int ahead = 0;
+  for (int c = 0; c < C; c++) {
+    for (int k = own_row[c]; k < own_row[c + 1]; k++) ahead = std::max(ahead, pos[own_idx[k]] - pos[c]);
+    for (int k = touch_row[c]; k < touch_row[c + 1]; k++)
+      ahead = std::max(ahead, pos[touch_idx[k]] - pos[c]);
+  }
+  s->flow_lag = 2 * (C / 2 - ahead) >= s->flow_ctas ? C / 2 : 0;
   return CI_OK;
 }
 
@@ -623,6 +638,7 @@ cudaError_t enqueue_flow(ci_solver* s, int n) {
     }
     F.desc = s->d_flow_desc.p;
     F.desc_stride = s->flow_stride;
+    F.lag = s->flow_lag;
     F.node_done = s->d_flow_ctr.p;
     F.elem_done = s->d_flow_ctr.p + C;
     F.task_ctr = s->d_flow_ctr.p + 2 * C;
