@@ -62,6 +62,25 @@ struct DBuf {
   }
 };
 
+// The status word, in page-locked host memory that kernels set bits of: the host reads it
+// after a synchronisation without a copy (a call of one step, 6,000 tet4: 30 -> 18 us).
+struct StatusWord {
+  unsigned int* host = nullptr;
+  unsigned int* p = nullptr;  // its address on the device
+  ~StatusWord() {
+    if (host) cudaFreeHost(host);
+  }
+  cudaError_t alloc() {
+    cudaError_t e = cudaHostAlloc(&host, sizeof(unsigned int), cudaHostAllocMapped);
+    if (!e) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&p), host, 0);
+    if (!e) clear();
+    return e;
+  }
+  // while no kernel runs
+  unsigned int read() const { return *static_cast<volatile unsigned int*>(host); }
+  void clear() { *static_cast<volatile unsigned int*>(host) = 0; }
+};
+
 }  // namespace
 
 namespace ci {
@@ -115,7 +134,7 @@ struct ci_solver {
   DBuf<float2> d_sig_b;
   DBuf<float> d_epbar;
   DBuf<double> d_work;     // [C][4]
-  DBuf<unsigned int> d_status;
+  StatusWord d_status;
   // one-shot scratch (never aliases the running state)
   DBuf<double> d_u2, d_v2, d_f;
   DBuf<float4> d_sig_a2;
@@ -400,9 +419,8 @@ cudaError_t enqueue_step(ci_solver* s, bool store_acc) {
 }
 
 int check_status(ci_solver* s) {
-  unsigned int st = 0;
-  CI_CUDA(cudaMemcpyAsync(&st, s->d_status.p, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
   CI_CUDA(cudaStreamSynchronize(s->stream));
+  const unsigned int st = s->d_status.read();
   if (st & ci::ST_DEGENERATE) return fail(CI_ERR_DEGENERATE, "an element has det J <= 0");
   if (st & ci::ST_NONFINITE) return fail(CI_ERR_NONFINITE, "non-finite nodal state");
   if (st & ci::ST_FLOW_TIMEOUT) {
@@ -468,8 +486,8 @@ int reset_history(ci_solver* s) {
   CI_CUDA(cudaMemsetAsync(s->d_contact.p, 0, N, s->stream));
   CI_CUDA(cudaMemsetAsync(s->d_acc.p, 0, sizeof(float) * 3 * N, s->stream));
   CI_CUDA(cudaMemsetAsync(s->d_work.p, 0, sizeof(double) * 4 * s->C, s->stream));
-  CI_CUDA(cudaMemsetAsync(s->d_status.p, 0, sizeof(unsigned int), s->stream));
   CI_CUDA(cudaStreamSynchronize(s->stream));
+  s->d_status.clear();
   s->started = false;
   s->steps_done = 0;
   return CI_OK;
@@ -1177,7 +1195,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   CI_CUDA(s->d_sig_b.alloc(E * s->nq));
   CI_CUDA(s->d_epbar.alloc(E * s->nq));
   CI_CUDA(s->d_work.alloc(4 * (size_t)s->C));
-  CI_CUDA(s->d_status.alloc(1));
+  CI_CUDA(s->d_status.alloc());
   CI_CUDA(s->d_epart.alloc(3 * ((N + 255) / 256)));
   if ((rc = upload_reference(s.get()))) return rc;
   if ((rc = reset_state(s.get()))) return rc;
@@ -1259,6 +1277,20 @@ int ci_steps_done(const ci_solver* s, long long* nsteps) {
   return CI_OK;
 }
 
+// The device's address of a caller's array of n doubles that lies whole in page-locked host
+// memory, else null.
+static double* mapped_address(const double* p, size_t n) {
+  if (!p || reinterpret_cast<size_t>(p) % sizeof(double)) return nullptr;
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, p) || cudaPointerGetAttributes(&b, p + n - 1)) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  double* d = static_cast<double*>(a.devicePointer);
+  return static_cast<double*>(b.devicePointer) == d + n - 1 ? d : nullptr;
+}
+
 int ci_get_state(ci_solver* s, double* x, double* v, double* mass, float* sigma, float* epbar,
                  unsigned char* contact) {
   if (!s) return fail(CI_ERR_INVALID, "null solver");
@@ -1269,14 +1301,19 @@ int ci_get_state(ci_solver* s, double* x, double* v, double* mass, float* sigma,
     // permuted to the caller's order on the GPU, then one copy per array
     int rc = ensure_exchange(s);
     if (rc) return rc;
+    // a small state goes straight into page-locked arrays (1,331 nodes 22.2 -> 17.7 us, 4,096
+    // 23.6 -> 19.8, 9,261 26.3 -> 24.4; 50,653 would take 60.0 instead of 42.8)
+    const bool direct = N <= 8192;
+    double* const xm = direct ? mapped_address(x, 3 * (size_t)N) : nullptr;
+    double* const vm = direct ? mapped_address(v, 3 * (size_t)N) : nullptr;
     k_state_to_caller<<<(N + 255) / 256, 256, 0, s->stream>>>(
-        s->d_u.p, s->d_v.p, s->d_Xc.p, s->d_node_new.p, N, x ? s->d_xc.p : nullptr,
-        v ? s->d_vc.p : nullptr);
+        s->d_u.p, s->d_v.p, s->d_Xc.p, s->d_node_new.p, N, xm ? xm : x ? s->d_xc.p : nullptr,
+        vm ? vm : v ? s->d_vc.p : nullptr);
     CI_CUDA(cudaGetLastError());
-    if (x)
+    if (x && !xm)
       CI_CUDA(cudaMemcpyAsync(x, s->d_xc.p, sizeof(double) * 3 * (size_t)N, cudaMemcpyDeviceToHost,
                               s->stream));
-    if (v)
+    if (v && !vm)
       CI_CUDA(cudaMemcpyAsync(v, s->d_vc.p, sizeof(double) * 3 * (size_t)N, cudaMemcpyDeviceToHost,
                               s->stream));
   }
@@ -1557,9 +1594,8 @@ int ci_get_energy(ci_solver* s, ci_energy* e) {
 int ci_get_status(ci_solver* s, unsigned int* status) {
   if (!s || !status) return fail(CI_ERR_INVALID, "null argument");
   CI_CUDA(cudaSetDevice(s->device));
-  CI_CUDA(cudaMemcpyAsync(status, s->d_status.p, sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                          s->stream));
   CI_CUDA(cudaStreamSynchronize(s->stream));
+  *status = s->d_status.read();
   return CI_OK;
 }
 
