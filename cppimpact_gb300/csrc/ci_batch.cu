@@ -239,16 +239,14 @@ cudaError_t prepare_step(Group& G) {
 cudaError_t launch_batch(Group& G, const FusedArgs& F) {
   const int bs = G.block_threads;
   if (G.npe == 4) {
-    step_kernel<EM_J2, true>(bs, G.step)<<<G.C, bs * G.step.W, G.step.smem, G.stream>>>(
-        F, ElemParams{}, NodeParams{});
-    return cudaGetLastError();
+    return launch_pdl(step_kernel<EM_J2, true>(bs, G.step), G.C, bs * G.step.W, G.step.smem,
+                      G.stream, F, ElemParams{}, NodeParams{});
   }
   const int lanes = G.repeats ? 1 : G.elem_lanes;
   const StepKernel k = bs == 64    ? batch_kernel10<64>(lanes)
                        : bs == 256 ? batch_kernel10<256>(lanes)
                                    : batch_kernel10<128>(lanes);
-  k<<<G.C, bs, G.smem, G.stream>>>(F, ElemParams{}, NodeParams{});
-  return cudaGetLastError();
+  return launch_pdl(k, G.C, bs, G.smem, G.stream, F, ElemParams{}, NodeParams{});
 }
 
 template <int BS>

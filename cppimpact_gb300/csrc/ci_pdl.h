@@ -1,10 +1,10 @@
 // ci_pdl.h -- programmatic dependent launch for chains of small kernels.
 //
 // A kernel launched with launch_pdl may start while the one before it on the stream still
-// runs; it calls pdl_wait() before its first access to global memory, which returns when
-// everything before it has completed, and pdl_next() as early as it can, which lets the
-// kernel after it start.  Launch and setup then overlap the tail of the kernel before (a training
-// batch of 14 launches, 123 -> 97 us).  Kernels that do not take part
+// runs; before its first access to global memory that another kernel writes it calls pdl_wait(),
+// which returns when everything before it has completed, and it may call pdl_next(), which lets
+// the kernel after it start before its end.  Launch and setup then overlap the tail of the
+// kernel before (a training batch of 14 launches, 123 -> 97 us).  Kernels that do not take part
 // order themselves as ever.
 #pragma once
 #include <cuda_runtime.h>

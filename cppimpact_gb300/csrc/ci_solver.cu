@@ -337,8 +337,7 @@ cudaError_t launch_fused10(ci_solver* s, const ci::FusedArgs& F, const ci::ElemP
       s->opt.elem_lanes == 4 && !s->plan.repeats
           ? (j2 ? ci::k_step_qp10<ci::EM_J2, BS> : ci::k_step_qp10<ci::EM_REFCOMPAT, BS>)
           : (j2 ? ci::k_step_t10<ci::EM_J2, BS> : ci::k_step_t10<ci::EM_REFCOMPAT, BS>);
-  k<<<s->C, BS, s->smem_bytes, s->stream>>>(F, ep, np);
-  return cudaGetLastError();
+  return ci::launch_pdl(k, s->C, BS, s->smem_bytes, s->stream, F, ep, np);
 }
 
 cudaError_t launch_fused(ci_solver* s, const ci::FusedArgs& F) {
@@ -349,8 +348,7 @@ cudaError_t launch_fused(ci_solver* s, const ci::FusedArgs& F) {
     const ci::StepKernel k = s->opt.mode != CI_MODE_REFCOMPAT
                                  ? ci::step_kernel<ci::EM_J2, false>(bs, s->step)
                                  : ci::step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step);
-    k<<<s->C, bs * s->step.W, s->step.smem, s->stream>>>(F, ep, np);
-    return cudaGetLastError();
+    return ci::launch_pdl(k, s->C, bs * s->step.W, s->step.smem, s->stream, F, ep, np);
   }
   if (bs == 64) return launch_fused10<64>(s, F, ep, np);
   if (bs == 128) return launch_fused10<128>(s, F, ep, np);
