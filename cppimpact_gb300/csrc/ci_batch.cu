@@ -85,7 +85,8 @@ struct Group {
   int max_local = 0, max_chunk_elems = 0;
   size_t smem = 0;
   bool repeats = false;  // Plan::repeats of any instance
-  StepForm step;  // of the tet4 step kernel
+  StepForm step;      // of the tet4 step kernel
+  StepForm10 step10;  // of the four-lane tet10 step kernel
   int block_threads = 128, elem_lanes = 4, chunk_nodes = 896, chunk_elements = 0;
   float tuned_ms_per_step = 0.f;  // autotuner's trial time of the chosen shape (0: not tuned)
   std::vector<int> insts;  // global instance ids
@@ -221,51 +222,43 @@ FusedArgs group_args(const Group& G, int i_in_graph) {
   return F;
 }
 
-template <int BS>
-StepKernel batch_kernel10(int elem_lanes) {
-  return elem_lanes == 4 ? k_step_qp10<EM_J2, BS, true> : k_step_t10<EM_J2, BS, true>;
+// One-lane groups and those with a repeated node have the kernel of one thread per element.
+bool one_lane(const Group& G) { return G.repeats || G.elem_lanes != 4; }
+
+StepKernel kernel10(const Group& G) {
+  const int bs = G.block_threads;
+  if (!one_lane(G)) return step_kernel10<EM_J2, true>(bs, G.step10);
+  return bs == 64    ? k_step_t10<EM_J2, 64, true>
+         : bs == 256 ? k_step_t10<EM_J2, 256, true>
+                     : k_step_t10<EM_J2, 128, true>;
 }
 
-// The form of the group's tet4 step kernel at its present shape; before a capture of it.
+// The form of the group's step kernel at its present shape; before a capture of it.
 cudaError_t prepare_step(Group& G) {
-  if (G.npe != 4) return cudaSuccess;
   int device = 0;
   const cudaError_t e = cudaGetDevice(&device);
   if (e) return e;
-  G.step = step_form(G.C, device, G.block_threads, G.max_local, G.max_chunk_elems);
-  return configure_step_kernel<EM_J2, true>(G.block_threads, G.step, device);
+  const int bs = G.block_threads;
+  if (G.npe == 4) {
+    G.step = step_form(G.C, device, bs, G.max_local, G.max_chunk_elems);
+    return configure_step_kernel(step_kernel<EM_J2, true>(bs, G.step), device);
+  }
+  G.step10 = step_form10(G.C, device, bs, G.max_local, G.max_chunk_elems);
+  return configure_step_kernel(kernel10(G), device);
 }
 
 cudaError_t launch_batch(Group& G, const FusedArgs& F) {
   const int bs = G.block_threads;
-  if (G.npe == 4) {
+  if (G.npe == 4)
     return launch_pdl(step_kernel<EM_J2, true>(bs, G.step), G.C, bs * G.step.W, G.step.smem,
                       G.stream, F, ElemParams{}, NodeParams{});
-  }
-  const int lanes = G.repeats ? 1 : G.elem_lanes;
-  const StepKernel k = bs == 64    ? batch_kernel10<64>(lanes)
-                       : bs == 256 ? batch_kernel10<256>(lanes)
-                                   : batch_kernel10<128>(lanes);
-  return launch_pdl(k, G.C, bs, G.smem, G.stream, F, ElemParams{}, NodeParams{});
-}
-
-template <int BS>
-cudaError_t configure10(int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_step_qp10<EM_J2, BS, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e) return e;
-  return cudaFuncSetAttribute(k_step_t10<EM_J2, BS, true>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return launch_pdl(kernel10(G), G.C, one_lane(G) ? bs : G.step10.threads,
+                    one_lane(G) ? G.smem : G.step10.smem, G.stream, F, ElemParams{}, NodeParams{});
 }
 
 template <int NPE>
 cudaError_t configure(int bytes) {
   cudaError_t e;
-  if (NPE == 10) {
-    if ((e = configure10<64>(bytes))) return e;
-    if ((e = configure10<128>(bytes))) return e;
-    if ((e = configure10<256>(bytes))) return e;
-  }
   if ((e = cudaFuncSetAttribute(k_elem<NPE, EM_MASS_HRZ, 256>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
     return e;

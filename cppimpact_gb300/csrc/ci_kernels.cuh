@@ -1106,9 +1106,7 @@ inline StepForm step_form(int C, int device, int bs, int max_local, int max_elem
 }
 
 // Its shared-memory limit is the device's, whatever a solver needs: several solvers share it.
-template <int MODE, bool BATCH>
-inline cudaError_t configure_step_kernel(int bs, const StepForm& f, int device) {
-  const StepKernel k = step_kernel<MODE, BATCH>(bs, f);
+inline cudaError_t configure_step_kernel(StepKernel k, int device) {
   int smem_max = 0;
   cudaError_t e =
       cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -1268,11 +1266,11 @@ __device__ __forceinline__ void tet10_rs_slot(const Tet10QP& t, const float (&Pm
 // records, the stress update from the stored stress (s4, s2: xx yy zz xy, yz xz) and
 // plastic strain ep0, which an active lane passes updated to put(), the work terms, and in
 // keep the element force on the nodes this lane owns (q, q + 4 and, for q < 2, q + 8).
-template <int MODE, class Put>
+template <int MODE, class Work, class Put>
 __device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& t, int q,
                                            const Tile& T, const int (&ln)[10], bool act, float4 s4,
-                                           float2 s2, float ep0, unsigned* status, float& wint,
-                                           float& wp, float (&keep)[3][3], Put put) {
+                                           float2 s2, float ep0, unsigned* status, Work work,
+                                           float (&keep)[3][3], Put put) {
   constexpr float W = 1.0f / 24.0f;
   float2 JG[9];
 #pragma unroll
@@ -1323,8 +1321,10 @@ __device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& 
     float wq = 0.f;
 #pragma unroll
     for (int k = 0; k < 6; k++) wq = fmaf(s0[k] + s[k], de[k], wq);
-    wint = fmaf(0.5f * wd, wq, wint);
-    if (MODE == EM_J2) wp = fmaf(wd * (ep.sy0 + ep.H * epn), epn - ep0, wp);
+    if (MODE == EM_J2)
+      work(0.5f * wd, wq, wd * (ep.sy0 + ep.H * epn), epn - ep0);
+    else
+      work(0.5f * wd, wq, 0.f, 0.f);
   }
   const float Sg[9] = {s[0], s[3], s[5], s[3], s[1], s[4], s[5], s[4], s[2]};
   float Pm[9];
@@ -1382,10 +1382,12 @@ __device__ __forceinline__ void add_nodes(const Tile& T, int n0, int n1, int n2,
   if (third) T.acc[n2] = sum(t2, f[2]);
 }
 
-template <int MODE, int BS, bool CG, bool PF>
+// The element loop of BS threads.  fold (null: a thread sums the work of its points itself)
+// gets the work factors of every point of the chunk.
+template <int MODE, int BS, bool CG, bool PF, bool FOLD = false>
 __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const ElemParams& ep,
                                                   const ChunkInfo& ch, const Tile& T, int tid,
-                                                  float& wint, float& wp) {
+                                                  float& wint, float& wp, float4* fold = nullptr) {
   const DevPlan& P = A.P;
   const int q = tid & 3;
   const Tet10QP t = tet10_qp(q);
@@ -1425,7 +1427,15 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
     int ln[10];
     conn10_unpack(n8, n2, ln);
     float keep[3][3];
-    qp10_point<MODE>(ep, t, q, T, ln, act, s4, s2, ep0, A.status, wint, wp, keep,
+    auto work = [&](float h, float wd, float hp, float wdp) {
+      if (FOLD) {
+        fold[4 * (w - ch.elem_begin) + tid] = make_float4(h, wd, hp, wdp);
+      } else {
+        wint = fmaf(h, wd, wint);
+        if (MODE == EM_J2) wp = fmaf(hp, wdp, wp);
+      }
+    };
+    qp10_point<MODE>(ep, t, q, T, ln, act, s4, s2, ep0, A.status, work, keep,
                      [&](float4 a4, float2 a2, float epn) {
                        A.sig_a[qi] = a4;
                        A.sig_b[qi] = a2;
@@ -1448,35 +1458,79 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
   }
 }
 
-// The fused kernels' element phase: the loop, then the chunk's partial nodal forces to
-// the halo and its work to chunk c's sums.
-template <int MODE, int BS, bool PF>
-__device__ __forceinline__ void step_qp10_elements(const FusedArgs& A, const ElemParams& ep,
-                                                   const ChunkInfo& ch, const Tile& T, int tid,
-                                                   int c, float* red) {
-  float wint, wp;
-  qp10_element_loop<MODE, BS, false, PF>(A, ep, ch, T, tid, wint, wp);
-  __syncthreads();
-  node_epilogue<BS>(A, ch, T, tid);
-  if (ep.accum_energy) add_chunk_work<BS>(A, c, wint, wp, red);
-}
-
-// 6 CTAs of 128 threads per SM (80 registers) fit the 896-node chunk's shared tile
-template <int MODE, int BS, bool BATCH = false>
-__global__ void __launch_bounds__(BS, 768 / BS) k_step_qp10(FusedArgs A, ElemParams ep_arg, NodeParams np_arg) {
+// Fused step of tet10, four lanes per element, TH threads.  768 threads of 80 registers on an SM
+// fit the 896-node chunk's shared tile.  What bounds a mesh of one round of CTAs is latency, so
+// where the CTAs leave room on the SMs they are wider than the BS threads asked for
+// (step_form10): 604 chunks of 143 elements, four on an SM, 18.5 us per step with 128 threads,
+// 16.7 with 192.  Nodal sums go by colour and do not depend on TH; the work sums keep the
+// order of BS threads (fold, after the tile).
+template <int MODE, int BS, int TH, bool BATCH = false>
+__global__ void __launch_bounds__(TH, 768 / TH) k_step_qp10(FusedArgs A, ElemParams ep_arg, NodeParams np_arg) {
   extern __shared__ float sm[];
   const DevPlan& P = A.P;
+  const int tid = threadIdx.x;
   const ChunkInfo ch = P.chunks[blockIdx.x];
   pdl_wait();
   const ChunkStep cs = chunk_step<BATCH>(A, ch, ep_arg, np_arg);
   if (cs.mode == 2) return;
   const Tile T = make_tile(sm, ch.n_local);
-  __shared__ float red[BS / 32];
+  __shared__ float red[TH / 32];
 
-  stage_nodes<BS>(A, cs.ep, cs.np, ch, cs.state_final, T, threadIdx.x);
+  stage_nodes<TH>(A, cs.ep, cs.np, ch, cs.state_final, T, tid);
   if (cs.mode == 1) return;
   __syncthreads();
-  step_qp10_elements<MODE, BS, true>(A, cs.ep, ch, T, threadIdx.x, blockIdx.x, red);
+  float4* fold = reinterpret_cast<float4*>(T.acc + ch.n_local);
+  float wint, wp;
+  qp10_element_loop<MODE, TH, false, true, (TH > BS)>(A, cs.ep, ch, T, tid, wint, wp, fold);
+  __syncthreads();
+  node_epilogue<TH>(A, ch, T, tid);
+  if (!cs.ep.accum_energy) return;
+  if (TH > BS && tid < BS) {
+    const int n = 4 * (ch.elem_end - ch.elem_begin);
+    for (int i = tid; i < n; i += BS) {
+      const float4 h = fold[i];
+      wint = fmaf(h.x, h.y, wint);
+      if (MODE == EM_J2) wp = fmaf(h.z, h.w, wp);
+    }
+  }
+  add_chunk_work<BS>(A, blockIdx.x, wint, wp, red);
+}
+
+// Threads and shared memory of k_step_qp10 for C chunks of at most max_local nodes and max_elems
+// elements: the widest CTAs of which all fit on the GPU together.  us per step, 86,400 elements
+// in 604 chunks: 18.3 with 128 threads, 16.7 with 192 (four on an SM), 23.5 with 256 (three: a
+// second round); 48,000 and 63,888 in as many 13.6 and 17.1, 13.5 and 17.0 with 192.
+struct StepForm10 {
+  int threads = 0;
+  size_t smem = 0;
+};
+
+inline StepForm10 step_form10(int C, int device, int bs, int max_local, int max_elems) {
+  int sms = 0, smem_sm = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+  const size_t tile = 40 * ((size_t)max_local + 2), smem = tile + 4 * sizeof(float4) * max_elems;
+  StepForm10 f;
+  f.threads = bs;
+  f.smem = tile;
+  if (bs != 128) return f;
+  const int need = (C + sms - 1) / sms;
+  for (const int th : {192, 256, 384})
+    if (th * need <= 768 && need * (smem + 2048) <= (size_t)smem_sm && th < 4 * max_elems + 64) {
+      f.threads = th;
+      f.smem = smem;
+    }
+  return f;
+}
+
+template <int MODE, bool BATCH>
+inline StepKernel step_kernel10(int bs, const StepForm10& f) {
+  if (bs == 64) return k_step_qp10<MODE, 64, 64, BATCH>;
+  if (bs == 256) return k_step_qp10<MODE, 256, 256, BATCH>;
+  return f.threads == 384   ? k_step_qp10<MODE, 128, 384, BATCH>
+         : f.threads == 256 ? k_step_qp10<MODE, 128, 256, BATCH>
+         : f.threads == 192 ? k_step_qp10<MODE, 128, 192, BATCH>
+                            : k_step_qp10<MODE, 128, 128, BATCH>;
 }
 
 // ---------------------------------------------------------------------------

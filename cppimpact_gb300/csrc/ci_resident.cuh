@@ -402,7 +402,11 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
           ep0 = S.epbar[qi];
         }
         float keep[3][3];
-        qp10_point<MODE>(ep, t10, q, T, ln, act, s4, s2, ep0, A.status, wint, wp, keep,
+        auto work = [&](float h, float wd, float hp, float wdp) {
+          wint = fmaf(h, wd, wint);
+          if (MODE == EM_J2) wp = fmaf(hp, wdp, wp);
+        };
+        qp10_point<MODE>(ep, t10, q, T, ln, act, s4, s2, ep0, A.status, work, keep,
                          [&](float4 a4, float2 a2, float epn) {
                            S.sig_a[qi] = a4;
                            S.sig_b[qi] = a2;

@@ -109,7 +109,8 @@ struct ci_solver {
   bool started = false;
   long long steps_done = 0;
   size_t smem_bytes = 0;
-  ci::StepForm step;  // of the tet4 step kernel
+  ci::StepForm step;      // of the tet4 step kernel
+  ci::StepForm10 step10;  // of the four-lane tet10 step kernel
 
   // device plan
   DBuf<ci::ChunkInfo> d_chunks;
@@ -299,11 +300,7 @@ cudaError_t configure_step10(int bytes) {
   if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_REFCOMPAT, BS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
     return e;
-  if ((e = cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_J2, BS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  return cudaFuncSetAttribute(ci::k_step_qp10<ci::EM_REFCOMPAT, BS>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return cudaSuccess;
 }
 
 // Raise the dynamic shared-memory limit of the element kernels once per solver (not
@@ -333,10 +330,11 @@ template <int BS>
 cudaError_t launch_fused10(ci_solver* s, const ci::FusedArgs& F, const ci::ElemParams& ep,
                            const ci::NodeParams& np) {
   const bool j2 = s->opt.mode != CI_MODE_REFCOMPAT;
-  const ci::StepKernel k =
-      s->opt.elem_lanes == 4 && !s->plan.repeats
-          ? (j2 ? ci::k_step_qp10<ci::EM_J2, BS> : ci::k_step_qp10<ci::EM_REFCOMPAT, BS>)
-          : (j2 ? ci::k_step_t10<ci::EM_J2, BS> : ci::k_step_t10<ci::EM_REFCOMPAT, BS>);
+  if (s->opt.elem_lanes == 4 && !s->plan.repeats)
+    return ci::launch_pdl(j2 ? ci::step_kernel10<ci::EM_J2, false>(BS, s->step10)
+                             : ci::step_kernel10<ci::EM_REFCOMPAT, false>(BS, s->step10),
+                          s->C, s->step10.threads, s->step10.smem, s->stream, F, ep, np);
+  const ci::StepKernel k = j2 ? ci::k_step_t10<ci::EM_J2, BS> : ci::k_step_t10<ci::EM_REFCOMPAT, BS>;
   return ci::launch_pdl(k, s->C, BS, s->smem_bytes, s->stream, F, ep, np);
 }
 
@@ -714,14 +712,22 @@ int setup_resident(ci_solver* s) {
   return CI_OK;
 }
 
-// Form of the tet4 step kernel.
+// Form of the step kernel.
 int setup_step(ci_solver* s) {
   const ci::Plan& P = s->plan;
-  s->step = ci::step_form(s->C, s->device, s->opt.block_threads, P.max_local, P.max_chunk_elems);
   const int bs = s->opt.block_threads;
-  CI_CUDA(s->opt.mode != CI_MODE_REFCOMPAT
-              ? (ci::configure_step_kernel<ci::EM_J2, false>(bs, s->step, s->device))
-              : (ci::configure_step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step, s->device)));
+  const bool j2 = s->opt.mode != CI_MODE_REFCOMPAT;
+  if (s->npe == 4) {
+    s->step = ci::step_form(s->C, s->device, bs, P.max_local, P.max_chunk_elems);
+    CI_CUDA(ci::configure_step_kernel(j2 ? ci::step_kernel<ci::EM_J2, false>(bs, s->step)
+                                         : ci::step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step),
+                                      s->device));
+  } else {
+    s->step10 = ci::step_form10(s->C, s->device, bs, P.max_local, P.max_chunk_elems);
+    CI_CUDA(ci::configure_step_kernel(j2 ? ci::step_kernel10<ci::EM_J2, false>(bs, s->step10)
+                                         : ci::step_kernel10<ci::EM_REFCOMPAT, false>(bs, s->step10),
+                                      s->device));
+  }
   return CI_OK;
 }
 
@@ -1141,7 +1147,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
     if (s->npe == 10 && s->opt.elem_lanes == 4 && s->opt.block_threads == 128) {
       int per_sm = 0, sms = 0;
       CI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, ci::k_step_qp10<ci::EM_J2, 128>, 128, s->smem_bytes));
+          &per_sm, ci::k_step_qp10<ci::EM_J2, 128, 128>, 128, s->smem_bytes));
       CI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
       if (5LL * s->C > 4LL * per_sm * sms) s->opt.step_kernel = 2;
     }
@@ -1183,7 +1189,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   }
   if (s->opt.step_kernel == 2 && (rc = setup_flow(s.get()))) return rc;
   if (s->opt.step_kernel == 3 && (rc = setup_resident(s.get()))) return rc;
-  if (s->npe == 4 && (rc = setup_step(s.get()))) return rc;
+  if ((rc = setup_step(s.get()))) return rc;
   CI_CUDA(s->d_mass.alloc(N));
   CI_CUDA(s->d_d0.alloc(N));
   CI_CUDA(s->d_d0f.alloc(N));

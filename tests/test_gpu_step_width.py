@@ -1,5 +1,5 @@
-"""The tet4 step kernel's widths (windows of block_threads elements at a time): on one plan the
-state does not depend on them."""
+"""The step kernels' widths (CTAs wider than block_threads): on one plan the state does not
+depend on them."""
 import numpy as np
 import pytest
 
@@ -38,6 +38,23 @@ def test_state_and_work(cilib, n, elements, nodes, mode):
            for bs in (64, 128, 256)]
     a, ea = out[0]
     assert (a["contact"] & 2).any()
+    for b, eb in out[1:]:
+        for k in ("x", "v", "sigma", "epbar", "contact"):
+            assert np.array_equal(a[k], b[k]), k
+        for k in ("internal", "plastic"):
+            assert eb[k] == pytest.approx(ea[k], rel=1e-5), k
+
+
+@pytest.mark.parametrize("n,elements,nodes,mode", [(12, 300, 896, "j2"), (17, 97, 512, "refcompat"),
+                                                   (20, 250, 896, "j2"), (22, 150, 896, "j2"),
+                                                   (20, 0, 896, "refcompat")])
+def test_state_and_work_tet10(cilib, n, elements, nodes, mode):
+    """The four-lane kernel with 384, 256 and 192 threads for the 128 asked for (35 to 608
+    chunks) against 64 and 256: states equal bit for bit, work sums as above."""
+    m = mg.cube(n, 2)
+    out = [solve(cilib, m, mode, chunk_elements=elements, chunk_nodes=nodes, block_threads=bs)
+           for bs in (64, 128, 256)]
+    a, ea = out[0]
     for b, eb in out[1:]:
         for k in ("x", "v", "sigma", "epbar", "contact"):
             assert np.array_equal(a[k], b[k]), k
