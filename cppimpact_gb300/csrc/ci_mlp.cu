@@ -9,7 +9,7 @@
 // transposed copy, the loss gradient with its transpose and bias gradient, the tanh
 // derivative with the same, Adam with the BF16 copies in both orders (23 launches a batch
 // before, 14 now, each set up while the one before runs, ci_pdl.h; 4 -> 256 -> 256 -> 5120, batches
-// of 256: 238 us a batch before, 97 now).
+// of 256: 238 us a batch before, 95 now).
 //
 // Parameters, in the order ci_mlp_get_params / set_params use:
 //   W1 [n_in x H], b1 [H], W2 [H x H], b2 [H], W3 [H x n_out], b3 [n_out]
@@ -55,25 +55,36 @@ __global__ void k_to_bf16(const float* in, bf16* out, long long n) {
   if (i < n) out[i] = __float2bfloat16(in[i]);
 }
 
-// Per-block partial sums of (Y - T)^2 for row r = blockIdx.y, whose targets are row idx[r] of T
-// (row r when idx is null)
-__global__ void k_mse_loss(const float* Y, const float* T, const int* idx, int cols, double* part) {
+// Partial sums of (Y - T)^2 over 256 columns of row r, whose targets are row idx[r] of T (row r
+// when idx is null): part[r][block of columns], the 256 squares added as a tree of halves.  A warp
+// per partial sum with 16 values in flight a lane (256 x 5,120, cold under a profiler: 27.3 us
+// with a CTA and eight barriers per partial sum, 13.3 so; FP64 bounds it).
+__global__ void __launch_bounds__(256) k_mse_loss(const float* Y, const float* T, const int* idx,
+                                                  int rows, int cols, double* part) {
   ci::pdl_next();
   ci::pdl_wait();
-  __shared__ double red[256];
-  const int r = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
-  double s = 0.0;
-  if (c < cols) {
-    const float d = Y[(size_t)r * cols + c] - T[(size_t)(idx ? idx[r] : r) * cols + c];
-    s = (double)d * d;
+  const int lane = threadIdx.x & 31, blocks = (cols + 255) / 256;
+  const long long w = blockIdx.x * 8LL + (threadIdx.x >> 5);
+  if (w >= (long long)rows * blocks) return;
+  const int r = (int)(w / blocks), c0 = (int)(w % blocks) * 256 + lane;
+  const float* y = Y + (size_t)r * cols;
+  const float* t = T + (size_t)(idx ? idx[r] : r) * cols;
+  float d[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const int c = min(c0 + 32 * j, cols - 1);
+    d[j] = y[c] - t[c];
   }
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+  double s[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) s[j] = c0 + 32 * j < cols ? (double)d[j] * d[j] : 0.0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < o; j++) s[j] += s[j + o];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s[0] += __shfl_down_sync(0xffffffffu, s[0], o);
+  if (lane == 0) part[w] = s[0];
 }
 
 // The passes over a [rows x cols] gradient between two products, CB columns and all rows per
@@ -441,7 +452,8 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
   const bf16* W2 = M->pb.p + M->off[2];
   const bf16* W3 = M->pb.p + M->off[4];
   if (loss) {
-    CM_CUDA(ci::launch_pdl(k_mse_loss, dim3(nb(M->n_out), rows), 256, 0, st, M->Y.p, T, idx, M->n_out, M->part.p));
+    CM_CUDA(ci::launch_pdl(k_mse_loss, (unsigned)(((long long)rows * nb(M->n_out) + 7) / 8), 256, 0, st, M->Y.p, T,
+                           idx, rows, M->n_out, M->part.p));
   }
   // layer 3: gW3 = H2^T dY as (H2^T) (dY^T)^T
   const float scale = 2.0f / (float)ny;
