@@ -1346,7 +1346,7 @@ constexpr size_t kMaxPackBytes = (size_t)256 << 20;
 // (81,920 x 96 x 96, A B: 97.2 us staged element by element, 22.7 with B copied; 96 x 96 x
 // 327,680, A^T B: 466 and 204 with both).
 int choose_operands(const void* A, int lda, int transA, const void* B, int ldb, int transB, int M,
-                    int N, int K, bool tma_shape, cudaStream_t st, Operands* op) {
+                    int N, int K, bool tma_shape, bool plain, cudaStream_t st, Operands* op) {
   const bool a_ok = !transA && lda >= K && lda % 8 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
   const bool b_ok = transB && ldb >= K && ldb % 8 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
   op->A = A;
@@ -1355,6 +1355,10 @@ int choose_operands(const void* A, int lda, int transA, const void* B, int ldb, 
   op->ldb = ldb;
   op->b_cols = K;
   if (!tensor_map_encoder()) return CI_OK;  // everything through the staging kernel
+  if (plain) {  // no workspace for copies or ranges
+    op->tma = tma_shape;
+    return CI_OK;
+  }
   // A of 8 MB or more read once past a B of at most 256 rows, K long enough to cut
   const bool streams = N <= 256 && (long long)M * K >= (1 << 22) && K >= 1024;
   if (!tma_shape || streams) {
@@ -1424,12 +1428,10 @@ bool pack_operands(Operands* op, char* at, cudaStream_t st) {
   return true;
 }
 
-}  // namespace
-
-extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int transB,
-                            float* C, int ldc, void* C_bf16, int M, int N, int K, float alpha,
-                            float beta, const float* bias, int activation, int* d_error,
-                            void* stream) {
+// plain: without the streaming kernel and without copies (after an allocation for them failed)
+int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int transB, float* C,
+              int ldc, void* C_bf16, int M, int N, int K, float alpha, float beta,
+              const float* bias, int activation, int* d_error, void* stream, bool plain) {
   if (!A || !B || !C || !d_error || M <= 0 || N <= 0 || K <= 0)
     return ci::set_last_error(CI_ERR_INVALID, "ci_gemm_bf16: null pointer or empty shape");
   if (activation != 0 && activation != 1)
@@ -1459,7 +1461,7 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   std::unique_lock<std::mutex> ws_lock(g_ws_mu, std::defer_lock);  // held until enqueued
   Operands op;
   {
-    const int rc = choose_operands(A, lda, transA, B, ldb, transB, M, N, K, tma_shape, st, &op);
+    const int rc = choose_operands(A, lda, transA, B, ldb, transB, M, N, K, tma_shape, plain, st, &op);
     if (rc) return rc;
   }
   if (op.stream) {
@@ -1485,7 +1487,11 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
     const int grid = (int)std::min<long long>(num_sms(), units);
     const size_t part = align256(sizeof(float) * 2 * (size_t)grid * BM * bn);
     char* ws = static_cast<char*>(workspace(dev, st, part + op.pack_bytes, ws_lock));
-    if (!ws) return ci::set_last_error(CI_ERR_NOMEM, "ci_gemm_bf16: workspace");
+    if (!ws) {
+      ws_lock.unlock();
+      return gemm_bf16(A, lda, transA, B, ldb, transB, C, ldc, C_bf16, M, N, K, alpha, beta, bias,
+                       activation, d_error, stream, true);
+    }
     P.partial = reinterpret_cast<float*>(ws);
     if (!pack_operands(&op, ws + part, st))
       return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: packing launch failed");
@@ -1528,6 +1534,11 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   const size_t part = splits > 1 ? align256(sizeof(float) * (size_t)splits * M * N) : 0;
   if (part + op.pack_bytes) {
     char* ws = static_cast<char*>(workspace(dev, st, part + op.pack_bytes, ws_lock));
+    if (!ws && op.pack_bytes) {
+      ws_lock.unlock();
+      return gemm_bf16(A, lda, transA, B, ldb, transB, C, ldc, C_bf16, M, N, K, alpha, beta, bias,
+                       activation, d_error, stream, true);
+    }
     if (!ws) return ci::set_last_error(CI_ERR_NOMEM, "ci_gemm_bf16: workspace");
     if (splits > 1) partial = reinterpret_cast<float*>(ws);
     if (!pack_operands(&op, ws + part, st))
@@ -1575,4 +1586,14 @@ extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, i
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(e));
   return CI_OK;
+}
+
+}  // namespace
+
+extern "C" int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int transB,
+                            float* C, int ldc, void* C_bf16, int M, int N, int K, float alpha,
+                            float beta, const float* bias, int activation, int* d_error,
+                            void* stream) {
+  return gemm_bf16(A, lda, transA, B, ldb, transB, C, ldc, C_bf16, M, N, K, alpha, beta, bias,
+                   activation, d_error, stream, false);
 }
