@@ -470,7 +470,12 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
       if (threads[x] != threads[y]) return threads[x] > threads[y];
       return (long long)nsteps[x] * plans[x]->E > (long long)nsteps[y] * plans[y]->E;
     });
-    bool all_fit = true;
+    // tet10 of more than two windows of elements per CTA is faster with a launch per step (time of
+    // that over the resident form's, 4 to 58 cubes of 34,992 with 58 elements per chunk 1.03 to
+    // 1.11, of 24,576 with 41 1.10 to 1.19, with 64 0.74 to 0.79, with 160 0.36 to 0.46); tet4
+    // chunks of 34 to 320 elements 1.05 to 2.4
+    constexpr int kMaxResident10 = 60;
+    bool all_fit = npe == 4 || G.max_chunk_elems <= kMaxResident10;
     for (size_t i = 0; i < n_inst && all_fit;) {
       const int p = threads[by[i]], begin = (int)order.size();
       std::vector<ChunkInfo> ci;
