@@ -918,8 +918,8 @@ __device__ __forceinline__ void add_chunk_work(const FusedArgs& A, int c, float 
 // elements are sorted by colour, so the nodal sums do not depend on W.  The work sums would:
 // with W > 1 the factors of each element's work go through shared memory to the first BS
 // threads, which add them window by window.  A batch of 52 cubes of 10,368 elements (312
-// chunks, up to 138 steps) 5.12 -> 4.23 ms; a step of 384,000 elements in one mesh 19.7 -> 18.0
-// us, of 1,572,864 72.2 -> 56.8.  (A list of each node's elements to gather instead of the
+// chunks, up to 138 steps) 5.12 -> 4.16 ms; a step of 384,000 elements in one mesh 19.7 -> 17.1
+// us, of 1,572,864 72.2 -> 54.0.  (A list of each node's elements to gather instead of the
 // colours: 4.77 ms, 25.7 and 82 us.)
 struct StepPoint {  // a point's state read ahead
   float4 a;
@@ -947,7 +947,7 @@ inline size_t step_smem(int bs, int W, int max_local) {
 }
 
 template <int MODE, int BS, int W, bool BATCH = false>
-__global__ void __launch_bounds__(BS * W, BS * W > 256 ? 1 : 768 / (BS * W))
+__global__ void __launch_bounds__(BS * W, 1024 / (BS * W))
     k_step(FusedArgs A, ElemParams ep_arg, NodeParams np_arg) {
   constexpr int TH = BS * W;
   extern __shared__ float sm[];
@@ -1081,10 +1081,11 @@ inline StepKernel step_kernel(int bs, const StepForm& f) {
 }
 
 // The form for C chunks of at most max_local nodes and max_elems elements: as wide as all CTAs
-// still fit on the GPU together (768 threads or one wider CTA an SM).  Windows of 128, W = 1
-// against 2: a batch of 312 chunks of 1,980 elements 4.83 and 4.23 ms; 608 chunks of 630, which
-// take two rounds when twice as wide, 18.0 and 24.7 us per step.  Windows of 64, W = 1, 2, 4: a
-// batch of 162 chunks of 1,980 7.09, 4.42 and 3.33 ms.
+// still fit on the GPU together (1,024 threads of 64 registers an SM; with 768 of 80 the batch
+// below takes 4.20 ms, a mesh of 608 chunks of 630 elements 17.7 us per step instead of 17.1, and
+// blocks of 256 fit two or three on an SM instead of four, 162,000 elements 17.3 us instead of
+// 11.2).  Windows of 128, W = 1 against 2: a batch of 312 chunks of 1,980 elements 4.83 and 4.16
+// ms.  Windows of 64, W = 1, 2, 4: a batch of 162 chunks of 1,980 7.09, 4.42 and 3.32 ms.
 inline StepForm step_form(int C, int device, int bs, int max_local, int max_elems) {
   int sms = 0, smem_max = 0, smem_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -1096,7 +1097,7 @@ inline StepForm step_form(int C, int device, int bs, int max_local, int max_elem
   for (int W = 2; W <= 4 && W * bs <= 512 && W * bs / 2 < max_elems; W *= 2) {
     const size_t smem = step_smem(bs, W, max_local);
     if (smem + 1024 > (size_t)smem_max) break;
-    const int fit = std::min<int>(smem_sm / (smem + 2048), W * bs > 256 ? 1 : 768 / (W * bs));
+    const int fit = std::min<int>(smem_sm / (smem + 2048), 1024 / (W * bs));
     if (fit >= need) {
       best.W = W;
       best.smem = smem;
