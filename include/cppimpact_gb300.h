@@ -98,7 +98,8 @@ typedef struct ci_options {
   int step_kernel;    /* 0 = automatic (2 for four-lane tet10 meshes of more than 0.8 of a
                          round of fused CTAs, else 3), 1 = element + node kernels, 2 = persistent task
                          kernel (tet10, elem_lanes 4, block_threads 128: node and element
-                         tasks of all the call's steps), 3 = fused (one launch per step);
+                         tasks of all the call's steps), 3 = fused (one launch per step, or
+                         one per call where the chunks stay resident on the GPU);
                          0, 2 and 3 give the same bits */
   int block_threads;  /* threads per chunk CTA of the fused kernel: 64, 128 or 256; 0 = automatic */
   int elem_lanes;     /* tet10 fused kernel: 4 = one lane per Gauss point, 1 = one thread per
