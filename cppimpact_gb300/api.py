@@ -362,8 +362,8 @@ class Solver:
         return lib().ci_step_kernel(self._h)
 
     def debug_flow_stall(self, chunk: int, wait_seconds: float) -> None:
-        """Test hook (ci_debug_flow_stall): the next task-kernel launch never publishes
-        chunk `chunk`'s progress, so its waits give up after wait_seconds."""
+        """Test hook (ci_debug_flow_stall): the next task-kernel or resident launch never
+        publishes chunk `chunk`'s progress, so its waits give up after wait_seconds."""
         check(lib().ci_debug_flow_stall(self._h, int(chunk), float(wait_seconds)))
 
 

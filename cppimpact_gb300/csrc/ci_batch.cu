@@ -572,6 +572,7 @@ int enqueue_resident(Group& G, int total, const Snapshots& sn) {
     A.claim = G.claim.p;
     A.abort_flag = G.claim.p + 1;
     A.wait_ns = kFlowWaitNs;
+    A.stall_chunk = -1;
     A.tag0 = G.tag;
     A.nsteps = k;
     A.inst_ep = G.inst_ep.p;

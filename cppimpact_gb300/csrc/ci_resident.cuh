@@ -80,15 +80,17 @@ __device__ __forceinline__ bool res_sync_and(bool ok) {
   return __syncthreads_and(ok) != 0;
 }
 
-// One failed poll: every 64th looks at the abort flag and the clock; false = give up.
+// One failed poll: every 64th looks at the abort flag and the clock; false = give up, which
+// the status word always tells: a chunk that leaves has stored nothing.
 static __device__ __noinline__ bool res_patience(const ResidentArgs& A, unsigned spins,
                                           unsigned long long& t0) {
   if (spins >= 2) __nanosleep(32);
   if ((spins & 63u) != 63u) return true;
-  if (*(volatile int*)A.abort_flag) return false;
-  const unsigned long long t = global_ns();
-  if (t0 == 0) t0 = t;
-  if (t - t0 <= A.wait_ns) return true;
+  if (!*(volatile int*)A.abort_flag) {
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    if (t - t0 <= A.wait_ns) return true;
+  }
   atomicOr(A.status, (unsigned)ST_FLOW_TIMEOUT);
   atomicExch(A.abort_flag, 1);
   return false;
@@ -150,6 +152,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   constexpr int EPW = P / LN;            // elements per window
   constexpr int EU = NPE == 4 ? 8 : 4;   // a node's entries and slots loaded at once
   const int tid = threadIdx.x;
+  if (!BATCH && ci == A.stall_chunk) return false;
   const ChunkInfo ch = A.P.chunks[ci];
   // an instance's parameters are read where they are used (a copy per thread would take some
   // thirty registers), a single solve's come as constants

@@ -32,6 +32,7 @@ struct ResidentArgs {
   const uint32_t* node_slots;   // [Lt] begin | count << 16 of a boundary node's part of them
   int* abort_flag;
   unsigned long long wait_ns;  // a wait gives up after this long
+  int stall_chunk;             // test hook, single solves: this chunk leaves at once (-1: none)
   unsigned tag0;               // step k of the launch carries the tag tag0 + k
   int nsteps;                  // steps of this launch (batches: at most)
   ElemParams ep;

@@ -153,7 +153,7 @@ struct ci_solver {
   DBuf<int> d_flow_desc, d_flow_ctr;
   int flow_ctas = 0, flow_stride = 0, flow_lag = 0;
   unsigned long long flow_wait_ns = ci::kFlowWaitNs;
-  int flow_stall_chunk = -1;  // test hook, for the next task-kernel launch only
+  int flow_stall_chunk = -1;  // test hook, for the next task-kernel or resident launch only
   size_t flow_smem = 0;
   // resident form of the fused step (ci_resident.cuh), where the plan fits it: the kernel
   // and its tables, the tagged slot buffers, the abort flag and the next unused tag
@@ -419,10 +419,8 @@ int check_status(ci_solver* s) {
   const unsigned int st = s->d_status.read();
   if (st & ci::ST_DEGENERATE) return fail(CI_ERR_DEGENERATE, "an element has det J <= 0");
   if (st & ci::ST_NONFINITE) return fail(CI_ERR_NONFINITE, "non-finite nodal state");
-  if (st & ci::ST_FLOW_TIMEOUT) {
-    if (s->d_res_abort.p) CI_CUDA(cudaMemset(s->d_res_abort.p, 0, sizeof(int)));
-    return fail(CI_ERR_CUDA, "step task kernel: a task waited longer than its time limit");
-  }
+  if (st & ci::ST_FLOW_TIMEOUT)
+    return fail(CI_ERR_CUDA, "step kernel: a chunk waited longer than its time limit");
   return CI_OK;
 }
 
@@ -482,6 +480,8 @@ int reset_history(ci_solver* s) {
   CI_CUDA(cudaMemsetAsync(s->d_contact.p, 0, N, s->stream));
   CI_CUDA(cudaMemsetAsync(s->d_acc.p, 0, sizeof(float) * 3 * N, s->stream));
   CI_CUDA(cudaMemsetAsync(s->d_work.p, 0, sizeof(double) * 4 * s->C, s->stream));
+  // (the flag of a resident run that gave up lasts as long as the bit in the status word)
+  if (s->d_res_abort.p) CI_CUDA(cudaMemsetAsync(s->d_res_abort.p, 0, sizeof(int), s->stream));
   CI_CUDA(cudaStreamSynchronize(s->stream));
   s->d_status.clear();
   s->started = false;
@@ -766,7 +766,10 @@ cudaError_t enqueue_resident(ci_solver* s, int n) {
     A.node_ent = s->d_res_node_ent.p;
     A.ent = s->d_res_ent.p;
     A.abort_flag = s->d_res_abort.p;
-    A.wait_ns = ci::kFlowWaitNs;
+    A.wait_ns = s->flow_wait_ns;
+    A.stall_chunk = s->flow_stall_chunk;
+    s->flow_stall_chunk = -1;
+    s->flow_wait_ns = ci::kFlowWaitNs;
     A.tag0 = s->res_tag;
     A.nsteps = k;
     A.ep = s->elem_params((float)s->dt, true);
@@ -1832,7 +1835,8 @@ int ci_step_kernel(const ci_solver* s) { return s ? s->opt.step_kernel : -1; }
 
 int ci_debug_flow_stall(ci_solver* s, int chunk, double wait_seconds) {
   if (!s) return fail(CI_ERR_INVALID, "null solver");
-  if (s->opt.step_kernel != 2) return fail(CI_ERR_UNSUPPORTED, "the solver does not run the task kernel");
+  if (s->opt.step_kernel != 2 && !s->res.kernel)
+    return fail(CI_ERR_UNSUPPORTED, "the solver runs neither the task kernel nor the resident one");
   if (chunk < 0 || chunk >= s->C || !(wait_seconds > 0.0) || wait_seconds > 60.0)
     return fail(CI_ERR_INVALID, "bad chunk or wait");
   s->flow_stall_chunk = chunk;
