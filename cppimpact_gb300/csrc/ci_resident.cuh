@@ -19,9 +19,9 @@
 // elements' order in the chunk), so the results are the same bits.  Per step and chunk:
 //   0  positions of the next state and the wall's push (they need no forces), written to
 //      the other of two record buffers, so other warps may do the elements meanwhile
-//   1  element forces: on_chip form to a (corner, element) buffer in shared memory, from
-//      which each node then adds its entries in element order (no barrier per colour);
-//      otherwise colour by colour into the accumulators as the fused kernels do
+//   1  element forces to a (corner, element) buffer in shared memory, from which each node
+//      then adds its entries in element order (no barrier per colour, and an element may
+//      name a node twice)
 //   2  boundary nodes' partial forces to their slots; work sums
 //   3  every slot of the boundary nodes polled into shared memory, sums in slot order,
 //      velocities and increments
@@ -34,11 +34,11 @@
 // velocities 600 (an FP64 instruction takes a warp 64 cycles).  At 34,992 tet10 the node
 // updates, which every holder of a boundary node repeats, weigh as much as the elements.
 //
-// on_chip: stored stress, connectivity, entry and slot lists are in shared memory too (121 B
-// per local node, 112 B per tet4 and 312 B per tet10 element, 4 to 16 B per slot: up to
-// about 58 tet10 or 270 tet4 elements per chunk at four CTAs per SM).  The other form
-// (tet10 batches, chunks of up to 450 local nodes) reads them through the caches; for a
-// single solve it is no faster than a launch per step (48,000 tet10: 15.2 against 15.1).
+// Stored stress, connectivity, entry and slot lists are in shared memory too (121 B per local
+// node, 112 B per tet4 and 312 B per tet10 element, 4 to 16 B per slot: up to about 58 tet10
+// or 270 tet4 elements per chunk at four CTAs per SM).  Read through the caches instead,
+// for larger chunks, they made it no faster than a launch per step (48,000 tet10: 15.2
+// against 15.1).
 #pragma once
 #include "ci_resident.h"
 
@@ -144,7 +144,7 @@ struct ResidentParams {
   NodeParams np;
 };
 
-template <int NPE, int MODE, int P, bool CHIP, bool BATCH>
+template <int NPE, int MODE, int P, bool BATCH>
 __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* sm, int ci,
                                           float (*red)[2][P / 32], ResidentParams* par) {
   constexpr int NQ = Rule<NPE>::NQ;
@@ -176,50 +176,28 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   // shared memory (see resident_smem)
   double* su = reinterpret_cast<double*>(sm);
   double* sv = su + 3 * L;
-  double* sw;  // the wall's push on a node in contact
   // records, double-buffered by step parity: node_step's positions of S^{k+1} do not wait
   // for the elements of step k
   float4* const p0 = reinterpret_cast<float4*>(sv + 3 * L);  // [2][L]
-  int4* m1 = nullptr;     // CHIP: own slot, received slots, element entries, 1/m
-  float4* acc = nullptr;  // else: the force accumulator
-  float4* fbuf;  // CHIP: [NPE][ne] element forces
-  float* recv;   // [3][ns] the boundary nodes' slots (CHIP: in the place of fbuf)
-  int* sslot = nullptr;  // CHIP: their ids
+  int4* const m1 = reinterpret_cast<int4*>(p0 + 2 * L);  // own slot, received slots, element entries, 1/m
+  float4* const fbuf = reinterpret_cast<float4*>(m1 + L);  // [NPE][ne] element forces
+  float* const recv = reinterpret_cast<float*>(fbuf);  // [3][ns] the boundary nodes' slots, in its place
   DevState S;
-  float2* p1;
-  uint16_t* sconn = nullptr;
-  uint16_t* sent = nullptr;
-  unsigned char* flags;
   S.status = A.status;
-  if (CHIP) {
-    m1 = reinterpret_cast<int4*>(p0 + 2 * L);
-    fbuf = reinterpret_cast<float4*>(m1 + L);
-    recv = reinterpret_cast<float*>(fbuf);
-    S.sig_a = fbuf + resident_exchange(NPE, ne, ns) / 16;
-    p1 = reinterpret_cast<float2*>(S.sig_a + NQ * ne);
-    sw = reinterpret_cast<double*>(p1 + 2 * L);
-    S.sig_b = reinterpret_cast<float2*>(sw + L);
-    S.epbar = reinterpret_cast<float*>(S.sig_b + NQ * ne);
-    sslot = reinterpret_cast<int*>(S.epbar + NQ * ne);
-    sconn = reinterpret_cast<uint16_t*>(sslot + ns);
-    sent = sconn + NPE * ne;
-    flags = reinterpret_cast<unsigned char*>(sent + NPE * ne);
-  } else {
-    fbuf = nullptr;
-    S.sig_a = A.sig_a;
-    S.sig_b = A.sig_b;
-    S.epbar = A.epbar;
-    acc = p0 + 2 * L;
-    p1 = reinterpret_cast<float2*>(acc + L);
-    sw = reinterpret_cast<double*>(p1 + 2 * L);
-    recv = reinterpret_cast<float*>(sw + L);
-    flags = reinterpret_cast<unsigned char*>(recv + 3 * ns);
-  }
+  S.sig_a = fbuf + resident_exchange(NPE, ne, ns) / 16;
+  float2* const p1 = reinterpret_cast<float2*>(S.sig_a + NQ * ne);
+  double* const sw = reinterpret_cast<double*>(p1 + 2 * L);  // the wall's push on a node in contact
+  S.sig_b = reinterpret_cast<float2*>(sw + L);
+  S.epbar = reinterpret_cast<float*>(S.sig_b + NQ * ne);
+  int* const sslot = reinterpret_cast<int*>(S.epbar + NQ * ne);  // the boundary nodes' slots' ids
+  uint16_t* const sconn = reinterpret_cast<uint16_t*>(sslot + ns);
+  uint16_t* const sent = sconn + NPE * ne;
+  unsigned char* const flags = reinterpret_cast<unsigned char*>(sent + NPE * ne);
   auto tile = [&](int parity) {
     Tile T;
     T.p0 = p0 + parity * L;
     T.p1 = p1 + parity * L;
-    T.acc = acc;
+    T.acc = nullptr;
     return T;
   };
 
@@ -241,28 +219,22 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     store_record(tile(0), l, x0[0] + uf[0], x0[1] + uf[1], x0[2] + uf[2], ep.dt * vf[0],
                  ep.dt * vf[1], ep.dt * vf[2]);
     flags[l] = A.contact[g];
-    if (CHIP) {
-      m1[l] = make_int4(A.P.local_slot[lb], (int)A.node_slots[lb], (int)A.node_ent[lb],
-                        __float_as_int(__frcp_rn(A.mass[g])));
-    } else {
-      acc[l] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    m1[l] = make_int4(A.P.local_slot[lb], (int)A.node_slots[lb], (int)A.node_ent[lb],
+                      __float_as_int(__frcp_rn(A.mass[g])));
   }
-  if (CHIP) {
-    for (int i = tid; i < ne; i += P)
+  for (int i = tid; i < ne; i += P)
 #pragma unroll
-      for (int a = 0; a < NPE; a++)
-        sconn[a * ne + i] = A.P.conn_local[(size_t)a * E + ch.elem_begin + i];
-    for (int i = tid; i < ns; i += P) sslot[i] = A.slots[rc.slot_begin + i];
-    for (int i = tid; i < NPE * ne; i += P) sent[i] = A.ent[(size_t)NPE * ch.elem_begin + i];
-    if (MODE == EM_J2)
-      for (int i = tid; i < NQ * ne; i += P) {
-        const size_t qi = (size_t)NQ * ch.elem_begin + i;
-        S.sig_a[i] = A.sig_a[qi];
-        S.sig_b[i] = A.sig_b[qi];
-        S.epbar[i] = A.epbar[qi];
-      }
-  }
+    for (int a = 0; a < NPE; a++)
+      sconn[a * ne + i] = A.P.conn_local[(size_t)a * E + ch.elem_begin + i];
+  for (int i = tid; i < ns; i += P) sslot[i] = A.slots[rc.slot_begin + i];
+  for (int i = tid; i < NPE * ne; i += P) sent[i] = A.ent[(size_t)NPE * ch.elem_begin + i];
+  if (MODE == EM_J2)
+    for (int i = tid; i < NQ * ne; i += P) {
+      const size_t qi = (size_t)NQ * ch.elem_begin + i;
+      S.sig_a[i] = A.sig_a[qi];
+      S.sig_b[i] = A.sig_b[qi];
+      S.epbar[i] = A.epbar[qi];
+    }
   double w0 = 0.0, w1 = 0.0;  // thread 0: the chunk's running work sums
   if (tid == 0) {
     w0 = A.chunk_work[4 * (size_t)ci];
@@ -289,11 +261,6 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   };
   // this chunk's partial force of local node l
   auto own_force = [&](int l) {
-    if (!CHIP) {
-      const float4 f = acc[l];
-      acc[l] = make_float4(0.f, 0.f, 0.f, 0.f);
-      return f;
-    }
     const unsigned en = (unsigned)m1[l].z;
     const uint16_t* e = sent + (en & 0xffffu);
     const int c = (int)(en >> 16);
@@ -344,7 +311,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     flags[l] = fl;
   };
   auto push = [&](const Tile& T, int l, bool last, float fx, float fy, float fz) {
-    const float rm = CHIP ? __int_as_float(m1[l].w) : __frcp_rn(A.mass[gid(l)]);
+    const float rm = __int_as_float(m1[l].w);
     float a[3] = {__fadd_rn(__fmul_rn(-fx, rm), np.gf[0]), __fadd_rn(__fmul_rn(-fy, rm), np.gf[1]),
                   __fadd_rn(__fmul_rn(-fz, rm), np.gf[2])};
     double ad[3] = {f32_to_f64(a[0]), f32_to_f64(a[1]), f32_to_f64(a[2])};
@@ -390,12 +357,11 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
       const int ii = act ? i : 0;
       if (NPE == 10) {
         // a warp past the last element skips the window (its lanes have no part in the sums)
-        if (CHIP && w + (tid & ~31) / LN >= ne) break;
+        if (w + (tid & ~31) / LN >= ne) break;
         int ln[10];
 #pragma unroll
-        for (int a = 0; a < 10; a++)
-          ln[a] = CHIP ? sconn[a * ne + ii] : A.P.conn_local[(size_t)a * E + ch.elem_begin + ii];
-        const size_t qi = CHIP ? (size_t)ii * 4 + q : (size_t)(ch.elem_begin + ii) * 4 + q;
+        for (int a = 0; a < 10; a++) ln[a] = sconn[a * ne + ii];
+        const size_t qi = (size_t)ii * 4 + q;
         float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
         float2 s2 = make_float2(0.f, 0.f);
         float ep0 = 0.f;
@@ -415,33 +381,10 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
                            S.sig_b[qi] = a2;
                            S.epbar[qi] = epn;
                          });
-        if (CHIP) {
-          if (act) {
-            fbuf[q * ne + i] = make_float4(keep[0][0], keep[0][1], keep[0][2], 0.f);
-            fbuf[(q + 4) * ne + i] = make_float4(keep[1][0], keep[1][1], keep[1][2], 0.f);
-            if (q < 2) fbuf[(q + 8) * ne + i] = make_float4(keep[2][0], keep[2][1], keep[2][2], 0.f);
-          }
-        } else {
-          const int o0 = q == 0 ? ln[0] : q == 1 ? ln[1] : q == 2 ? ln[2] : ln[3];
-          const int o1 = q == 0 ? ln[4] : q == 1 ? ln[5] : q == 2 ? ln[6] : ln[7];
-          const int o2 = q == 0 ? ln[8] : ln[9];
-          const uint8_t* cl = A.P.color + ch.elem_begin;
-          const int col = act ? cl[i] : -1, c0 = cl[w], c1 = cl[min(w + EPW, ne) - 1];
-          for (int c = c0; c <= c1; c++) {
-            res_sync<P>();
-            if (col == c) {
-              auto add = [&](int o, const float (&f)[3]) {
-                float4 t = T.acc[o];
-                t.x += f[0];
-                t.y += f[1];
-                t.z += f[2];
-                T.acc[o] = t;
-              };
-              add(o0, keep[0]);
-              add(o1, keep[1]);
-              if (q < 2) add(o2, keep[2]);
-            }
-          }
+        if (act) {
+          fbuf[q * ne + i] = make_float4(keep[0][0], keep[0][1], keep[0][2], 0.f);
+          fbuf[(q + 4) * ne + i] = make_float4(keep[1][0], keep[1][1], keep[1][2], 0.f);
+          if (q < 2) fbuf[(q + 8) * ne + i] = make_float4(keep[2][0], keep[2][1], keep[2][2], 0.f);
         }
       } else {
         int ln[NPE];
@@ -450,7 +393,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
           float x[NPE][3], du[NPE][3];
 #pragma unroll
           for (int a = 0; a < NPE; a++) {
-            ln[a] = CHIP ? sconn[a * ne + i] : A.P.conn_local[(size_t)a * E + ch.elem_begin + i];
+            ln[a] = sconn[a * ne + i];
             float2 pr[3];
             load_pairs(T, ln[a], pr);
 #pragma unroll
@@ -459,27 +402,9 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
               du[a][c] = pr[c].y;
             }
           }
-          element_force<NPE, MODE>(ep, S, CHIP ? i : ch.elem_begin + i, x, du, f, wint, wp, vol);
-          if (CHIP)
+          element_force<NPE, MODE>(ep, S, i, x, du, f, wint, wp, vol);
 #pragma unroll
-            for (int a = 0; a < NPE; a++) fbuf[a * ne + i] = make_float4(f[a][0], f[a][1], f[a][2], 0.f);
-        }
-        if (!CHIP) {
-          const uint8_t* cl = A.P.color + ch.elem_begin;
-          const int col = act ? cl[i] : -1, c0 = cl[w], c1 = cl[min(w + EPW, ne) - 1];
-          for (int c = c0; c <= c1; c++) {
-            res_sync<P>();
-            if (col == c) {
-#pragma unroll
-              for (int a = 0; a < NPE; a++) {
-                float4 t = T.acc[ln[a]];
-                t.x += f[a][0];
-                t.y += f[a][1];
-                t.z += f[a][2];
-                T.acc[ln[a]] = t;
-              }
-            }
-          }
+          for (int a = 0; a < NPE; a++) fbuf[a * ne + i] = make_float4(f[a][0], f[a][1], f[a][2], 0.f);
         }
       }
     }
@@ -492,7 +417,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     for (int l = nd; l < L; l += P) {
       const float4 f = own_force(l);
       if (l >= ch.n_int) {
-        st_slot(halo + (CHIP ? m1[l].x : A.P.local_slot[ch.local_begin + l]), f.x, f.y, f.z, tag);
+        st_slot(halo + m1[l].x, f.x, f.y, f.z, tag);
       } else {  // kept in the next record's increments until the node's push
         float* r = reinterpret_cast<float*>(Tn.p0 + l);
         r[1] = f.x;
@@ -520,7 +445,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
         f[2] = __fadd_rn(0.f, Tn.p1[l].y);
         return;
       }
-      const unsigned sl = CHIP ? (unsigned)m1[l].y : A.node_slots[ch.local_begin + l];
+      const unsigned sl = (unsigned)m1[l].y;
       const float* r = recv + (sl & 0xffffu);
       const int cnt = (int)(sl >> 16);
       f[0] = f[1] = f[2] = 0.f;
@@ -555,7 +480,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
       w0 += (double)a;
       w1 += (double)b;
     }
-    const bool ok = res_receive<P>(A, halo, CHIP ? sslot : A.slots + rc.slot_begin, ns, tag, recv);
+    const bool ok = res_receive<P>(A, halo, sslot, ns, tag, recv);
     if (!res_sync_and<P>(ok)) return false;
     for (int l = early + nd; l < L; l += P) {
       float f[3];
@@ -582,7 +507,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     }
     A.contact[g] = flags[l];
   }
-  if (CHIP && MODE == EM_J2)
+  if (MODE == EM_J2)
     for (int i = tid; i < NQ * ne; i += P) {
       const size_t qi = (size_t)NQ * ch.elem_begin + i;
       A.sig_a[qi] = S.sig_a[i];
@@ -605,13 +530,13 @@ constexpr int resident_min_ctas(int npe, int p, bool batch) {
   return p == 64 ? 16 : 20;
 }
 
-template <int NPE, int MODE, int P, bool CHIP, bool BATCH>
+template <int NPE, int MODE, int P, bool BATCH>
 __global__ void __launch_bounds__(P, resident_min_ctas(NPE, P, BATCH))
     k_resident(const __grid_constant__ ResidentArgs A) {
   extern __shared__ __align__(16) unsigned char res_sm[];
   __shared__ float red[2][2][P / 32];
   if constexpr (!BATCH) {
-    res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, blockIdx.x, red, nullptr);
+    res_chunk<NPE, MODE, P, BATCH>(A, res_sm, blockIdx.x, red, nullptr);
   } else {
     // batches: chunks taken in order, an instance's chunks next to each other.  A CTA waits
     // only for chunks of its own instance; those before it in the order are running or
@@ -625,15 +550,15 @@ __global__ void __launch_bounds__(P, resident_min_ctas(NPE, P, BATCH))
       const int c = taken;
       res_sync<P>();
       if (c >= A.n_chunks) return;
-      if (!res_chunk<NPE, MODE, P, CHIP, BATCH>(A, res_sm, A.order[c], red, &par)) return;
+      if (!res_chunk<NPE, MODE, P, BATCH>(A, res_sm, A.order[c], red, &par)) return;
       res_sync<P>();
     }
   }
 }
 
-template <int NPE, int MODE, int P, bool CHIP, bool BATCH>
+template <int NPE, int MODE, int P, bool BATCH>
 const void* resident_fn() {
-  return reinterpret_cast<const void*>(&k_resident<NPE, MODE, P, CHIP, BATCH>);
+  return reinterpret_cast<const void*>(&k_resident<NPE, MODE, P, BATCH>);
 }
 
 }  // namespace ci

@@ -57,7 +57,6 @@ struct ResidentArgs {
 struct ResidentPick {
   const void* kernel = nullptr;
   int threads = 0;
-  bool on_chip = false;  // element tables, stress and node constants in shared memory too
   size_t smem = 0;
   int ctas = 0;  // co-resident on the whole GPU
 };
@@ -69,11 +68,10 @@ __host__ __device__ constexpr size_t resident_exchange(int npe, int ne, int ns) 
 }
 
 // Shared bytes of a chunk of `nl` local nodes, `ne` elements and `ns` boundary slots.
-__host__ __device__ constexpr size_t resident_smem(int npe, int nl, int ne, int ns, bool on_chip) {
+__host__ __device__ constexpr size_t resident_smem(int npe, int nl, int ne, int ns) {
   const int nq = npe == 4 ? 1 : 4;
-  return on_chip ? 121 * (size_t)nl + 28 * (size_t)(nq * ne) + 4 * (size_t)(npe * ne) +
-                       4 * (size_t)ns + resident_exchange(npe, ne, ns) + 64
-                 : 121 * (size_t)nl + 12 * (size_t)ns + 64;
+  return 121 * (size_t)nl + 28 * (size_t)(nq * ne) + 4 * (size_t)(npe * ne) + 4 * (size_t)ns +
+         resident_exchange(npe, ne, ns) + 64;
 }
 
 // Threads of the kernel for chunks of at most `elements` elements.  A single solve has SMs to

@@ -7,25 +7,24 @@ namespace ci {
 
 namespace {
 template <int MODE, bool BATCH>
-const void* pick(int threads, bool chip) {
+const void* pick(int threads) {
   if constexpr (BATCH)
-    if (threads == 32 && chip) return resident_fn<4, MODE, 32, true, BATCH>();
-  if (threads == 64 && chip) return resident_fn<4, MODE, 64, true, BATCH>();
-  if (threads == 128 && chip) return resident_fn<4, MODE, 128, true, BATCH>();
-  return nullptr;
+    if (threads == 32) return resident_fn<4, MODE, 32, BATCH>();
+  if (threads == 64) return resident_fn<4, MODE, 64, BATCH>();
+  return threads == 128 ? resident_fn<4, MODE, 128, BATCH>() : nullptr;
 }
 }  // namespace
 
-const void* resident_kernel_tet4(bool refcompat, bool batch, int threads, bool chip) {
-  if (batch) return refcompat ? nullptr : pick<EM_J2, true>(threads, chip);
-  return refcompat ? pick<EM_REFCOMPAT, false>(threads, chip) : pick<EM_J2, false>(threads, chip);
+const void* resident_kernel_tet4(bool refcompat, bool batch, int threads) {
+  if (batch) return refcompat ? nullptr : pick<EM_J2, true>(threads);
+  return refcompat ? pick<EM_REFCOMPAT, false>(threads) : pick<EM_J2, false>(threads);
 }
 
 }  // namespace ci
 
 namespace ci {
 
-const void* resident_kernel_tet10(bool refcompat, bool batch, int threads, bool chip);
+const void* resident_kernel_tet10(bool refcompat, bool batch, int threads);
 
 int resident_threads(int npe, bool batch, int elements) {
   if (npe == 10) return batch && elements <= 24 ? 64 : 128;
@@ -52,32 +51,27 @@ cudaError_t pick_resident(int npe, bool refcompat, bool batch, const std::vector
   if (energy_threads && threads != energy_threads &&
       (npe == 10 ? 4 : 1) * most > std::min(threads, energy_threads))
     return cudaSuccess;
-  for (const bool chip : {true, false}) {
-    const void* fn = npe == 4 ? resident_kernel_tet4(refcompat, batch, threads, chip)
-                              : resident_kernel_tet10(refcompat, batch, threads, chip);
-    if (!fn) continue;
-    size_t smem = 0;
-    bool fits = true;
-    for (size_t i = 0; i < chunks.size(); i++) {
-      const ChunkInfo& c = chunks[i];
-      const int ne = c.elem_end - c.elem_begin, ns = rchunks[i].n_slots;
-      smem = std::max(smem, resident_smem(npe, c.n_local, ne, ns, chip));
-      fits = fits && npe * ne <= 65535 && ns <= 65535;  // 16-bit positions
-    }
-    if (!fits || (long long)smem + 2048 > smem_max) continue;
-    // one limit for every solver (a smaller one set later would refuse this one's launch)
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 2048)))
-      return e;
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem))) return e;
-    if ((long long)per_sm * sms < need_ctas) continue;
-    out->kernel = fn;
-    out->threads = threads;
-    out->on_chip = chip;
-    out->smem = smem;
-    out->ctas = per_sm * sms;
-    return cudaSuccess;
+  const void* fn = npe == 4 ? resident_kernel_tet4(refcompat, batch, threads)
+                            : resident_kernel_tet10(refcompat, batch, threads);
+  if (!fn) return cudaSuccess;
+  size_t smem = 0;
+  for (size_t i = 0; i < chunks.size(); i++) {
+    const ChunkInfo& c = chunks[i];
+    const int ne = c.elem_end - c.elem_begin, ns = rchunks[i].n_slots;
+    if (npe * ne > 65535 || ns > 65535) return cudaSuccess;  // 16-bit positions
+    smem = std::max(smem, resident_smem(npe, c.n_local, ne, ns));
   }
+  if ((long long)smem + 2048 > smem_max) return cudaSuccess;
+  // one limit for every solver (a smaller one set later would refuse this one's launch)
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 2048)))
+    return e;
+  int per_sm = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem))) return e;
+  if ((long long)per_sm * sms < need_ctas) return cudaSuccess;
+  out->kernel = fn;
+  out->threads = threads;
+  out->smem = smem;
+  out->ctas = per_sm * sms;
   return cudaSuccess;
 }
 
