@@ -418,6 +418,8 @@ __global__ void __launch_bounds__(128, 1)
 // The epilogue of tile i overlaps the MMAs of tile i + 1.  Every wait is bounded; a role
 // that times out raises a shared abort flag so the others stop waiting, and the kernel
 // reports the error through *err.
+// CHAIN: an accumulator takes `chain` K steps, and the epilogue warps add the sums of a tile's
+// accumulators in registers, in K order: the sums of split K without its partial tiles.
 constexpr int GROUP_M = 16;
 
 __device__ __forceinline__ bool mbar_wait_abort(uint32_t bar, uint32_t phase, volatile int* abort) {
@@ -561,11 +563,11 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   nt = r / gm;
 }
 
-template <int BN, int STAGES, int EPW>
+template <int BN, int STAGES, int EPW, bool CHAIN>
 __global__ void __launch_bounds__(64 + 32 * EPW, 1)
     k_gemm_tma_pers(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     float* C, int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha,
-                    float beta, const float* __restrict__ bias, int act, int* err) {
+                    float beta, const float* __restrict__ bias, int act, int* err, int chain_steps) {
   constexpr int A_BYTES = BM * TBK * 2;
   constexpr int B_BYTES = BN * TBK * 2;
   constexpr uint32_t TCOLS = 2 * BN;  // two accumulators of BN FP32 columns
@@ -582,6 +584,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   const int tiles = tiles_m * tiles_n;
   const int ktiles = (K + TBK - 1) / TBK;
+  const int chain = CHAIN ? chain_steps : ktiles;  // K steps of an accumulator
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -641,43 +644,88 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
       const uint32_t idesc = instr_desc(BM, BN);
       long long it = 0;
       int j = 0;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, j++) {
-        const int b = j & 1;
-        if (j >= 2 && !mbar_wait_abort(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t acc_tmem = tmem + (uint32_t)(b * BN);
-        for (int kt = 0; kt < ktiles; kt++, it++) {
-          const int s = (int)(it % STAGES);
-          if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) {
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        for (int kc = 0; kc < ktiles && ok; kc += chain, j++) {
+          const int b = j & 1;
+          if (j >= 2 && !mbar_wait_abort(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint32_t acc_tmem = tmem + (uint32_t)(b * BN);
+          const int ke = min(ktiles, kc + chain);
+          for (int kt = kc; kt < ke; kt++, it++) {
+            const int s = (int)(it % STAGES);
+            if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) {
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-          for (int kk = 0; kk < TBK / 16; kk++) {
-            const uint64_t da = desc_sw128(smem_u32(sA + s * A_BYTES) + kk * 32);
-            const uint64_t db = desc_sw128(smem_u32(sB + s * B_BYTES) + kk * 32);
-            const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
+            for (int kk = 0; kk < TBK / 16; kk++) {
+              const uint64_t da = desc_sw128(smem_u32(sA + s * A_BYTES) + kk * 32);
+              const uint64_t db = desc_sw128(smem_u32(sB + s * B_BYTES) + kk * 32);
+              const uint32_t acc = (kt > kc || kk > 0) ? 1u : 0u;
+              asm volatile(
+                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                  " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc_tmem),
+                  "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                  : "memory");
+            }
             asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc_tmem),
-                "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                    smem_u32(&empty[s]))
                 : "memory");
           }
+          if (!ok) break;
+          // the accumulator is complete once every MMA issued so far has finished
           asm volatile(
               "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                  smem_u32(&empty[s]))
+                  smem_u32(&tfull[b]))
               : "memory");
         }
-        if (!ok) break;
-        // the accumulator is complete once every MMA issued so far has finished
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                smem_u32(&tfull[b]))
-            : "memory");
+      }
+    }
+  } else if constexpr (CHAIN) {
+    const int q = warp & 3;
+    constexpr int COLS = BN * 4 / EPW;
+    const int c_begin = (warp - 2) / 4 * COLS;
+    int j = 0;
+    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      float sum[COLS];
+      for (int kc = 0; kc < ktiles; kc += chain, j++) {
+        const int b = j & 1;
+        if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+        for (int n = 0; n < COLS; n += 32) {
+          uint32_t r[32];
+          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            sum[n + i] = kc == 0 ? __uint_as_float(r[i]) : sum[n + i] + __uint_as_float(r[i]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&tempty[b]))
+                       : "memory");
+      }
+      if (!ok) break;
+      int mt, nt;
+      tile_coords(t, tiles_m, tiles_n, mt, nt);
+      const int n0 = nt * BN + c_begin;
+#pragma unroll
+      for (int n = 0; n < COLS; n += 32) {
+        if (n0 + n >= N) break;
+        uint32_t r[32];
+#pragma unroll
+        for (int i = 0; i < 32; i++) r[i] = __float_as_uint(sum[n + i]);
+        epi_store(epi_buf[warp - 2], r, mt * BM + q * 32, M, n0 + n, N, C, ldc, Cb, alpha, beta,
+                  bias, act, lane);
       }
     }
   } else {
@@ -1209,24 +1257,24 @@ int num_sms() {
 // their buffers) keep more of them going than four.
 constexpr int kShortK = 512;
 
-template <int BN, int STAGES, int EPW>
+template <int BN, int STAGES, int EPW, bool CHAIN = false>
 cudaError_t launch_pers(const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t st, float* C,
                         int ldc, __nv_bfloat16* Cb, int M, int N, int K, float alpha, float beta,
-                        const float* bias, int act, int* err) {
+                        const float* bias, int act, int* err, int chain = 0) {
   static bool configured[64] = {};
   constexpr int smem = tma_smem_bytes<BN, STAGES>();
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     const cudaError_t e = cudaFuncSetAttribute(
-        k_gemm_tma_pers<BN, STAGES, EPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        k_gemm_tma_pers<BN, STAGES, EPW, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = std::min(tiles, num_sms());
-  return ci::launch_pdl(k_gemm_tma_pers<BN, STAGES, EPW>, grid, 64 + 32 * EPW, smem, st, ta, tb, C,
-                        ldc, Cb, M, N, K, alpha, beta, bias, act, err);
+  return ci::launch_pdl(k_gemm_tma_pers<BN, STAGES, EPW, CHAIN>, grid, 64 + 32 * EPW, smem, st, ta,
+                        tb, C, ldc, Cb, M, N, K, alpha, beta, bias, act, err, chain);
 }
 
 template <int BN>
@@ -1513,18 +1561,24 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
   const int bn_tma = N <= 64 ? 64 : N <= 128 ? 128 : 256;
   int bn = tma ? bn_tma : (N <= 64 ? 64 : 128);
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-  // Split K when the output has too few tiles to fill the GPU and K is long.  With more than
-  // half a tile per SM the split costs more than it gives (2,048 x 2,048 x 512, 128 tiles: 11.9
-  // us whole, 38.9 in two halves of K), but a longer chain of products loses accuracy, so only
-  // K up to 896 (1e-6 of the result) stays whole.
+  // Split K when the output has too few tiles to fill the GPU and K is long.
   int splits = 1;
-  const bool whole = tma && 2 * tiles > num_sms() && K <= 896;
-  if (!whole && tiles < 304 && K >= 8 * BK)
+  if (tiles < 304 && K >= 8 * BK)
     splits = std::min((304 + tiles - 1) / tiles, (K + 4 * BK - 1) / (4 * BK));
   splits = std::max(1, std::min(splits, 512));
   int k_chunk = (K + splits - 1) / splits;
   k_chunk = (k_chunk + BK - 1) / BK * BK;
   splits = (K + k_chunk - 1) / k_chunk;
+  // With more than half a tile per SM and a short K the partial tiles cost more than the CTAs give
+  // (4,096 x 1,024 x 512 39.2 us, 8,192 x 512 x 896 49.6), but one chain of products over all of K would lose accuracy
+  // (8,192 x 512 x 896: 8.6e-7, in chains of 320 products 2.7e-7): the same chains, one after
+  // the other in the persistent kernel (12.2 and 16.3 us; as one chain 11.4 and 14.9).
+  int chain = 0;
+  if (tma && splits > 1 && 2 * tiles > num_sms() && K <= 896) {
+    chain = k_chunk / BK;
+    splits = 1;
+    bn = std::min(bn, 128);  // (256 columns would be 128 sums a thread)
+  }
   // Narrower tiles while they leave the GPU half empty: 256 x 256 x 256, two tiles of 256
   // columns, 13.5 us, eight of 64 7.3 (cold, under a profiler).  The sums of an output do not
   // depend on its tile.
@@ -1550,7 +1604,13 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
     return ci::set_last_error(CI_ERR_CUDA, "ci_gemm_bf16: tensor map");
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, splits);
   cudaError_t le = cudaSuccess;
-  if (tma && splits == 1) {
+  if (tma && chain) {
+    le = bn == 64 ? launch_pers<64, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias,
+                                                      activation, d_error, chain)
+                  : launch_pers<128, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta,
+                                                       bias, activation, d_error, chain);
+    if (le != cudaSuccess) return ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(le));
+  } else if (tma && splits == 1) {
     if (bn == 64)
       le = launch_tma_pers<64>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias, activation, d_error);
     else if (bn == 128)

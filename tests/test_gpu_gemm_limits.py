@@ -1,0 +1,33 @@
+"""ci_gemm_bf16 where its kernels and copies meet their limits: length of the chains that the
+tensor core sums, sizes of launch grids, captured streams.  Operands and reference as in
+tests/test_gpu_gemm_shapes.py.
+
+The tensor core's FP32 sums lose about 1.1e-9 of the result per product of a chain (7.3e-6
+after 6,591 products), sums of a few chains add the rounding of one FP32 addition each,
+6e-8 at most: 1.2e-9 times the longest chain, and 2e-8, hold for chains of 192 products and
+more."""
+import numpy as np
+import pytest
+
+from test_gpu_gemm_shapes import product
+
+pytestmark = pytest.mark.gpu
+
+
+def error(c, ref):
+    return float(np.linalg.norm(c - ref) / np.linalg.norm(ref))
+
+
+@pytest.mark.parametrize("M,N,K,chain", [(2048, 2048, 512, 256), (4096, 1024, 704, 256),
+                                         (8192, 320, 896, 320), (10000, 64, 520, 192),
+                                         (9800, 100, 896, 320), (19000, 256, 640, 320),
+                                         (8190, 515, 521, 320)])
+@pytest.mark.parametrize("form", [dict(), dict(bias=True, act=1, alpha=0.02, copy=True, ldc_pad=3),
+                                  dict(beta=0.5, ldc_pad=4)])
+def test_chains_of_short_products(cilib, M, N, K, chain, form):
+    """Products of K from 512 to 896 whose tiles fill more than half of the GPU are summed in the
+    chains of split K (512 products in one chain would be 4.7e-7, 896 8.6e-7)."""
+    torch = pytest.importorskip("torch")
+    c, ref = product(cilib, torch, M, N, K, lda_pad=(-K) % 8 if N != 515 else 0,
+                     ldb_pad=(-K) % 8 if N != 515 else 0, seed=K, **form)
+    assert error(c, ref) <= 1.2e-9 * chain + 2e-8
