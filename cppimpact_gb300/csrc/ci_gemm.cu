@@ -793,10 +793,10 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
 // rate).
 //
 // Accuracy: the tensor core's FP32 sums lose about 1.1e-9 of the result per product in a chain
-// (measured: 7.3e-6 after 6,591, 2.9e-5 after 28,000; here 4.7e-7 for either).  A chain here is kChain K steps (512
-// products); the epilogue warps add the chains' sums in registers, rounded to nearest, while
-// the next chain runs in the other accumulator.
-constexpr int kChain = 8;
+// (measured: 7.3e-6 after 6,591, 2.9e-5 after 28,000).  A chain here is kChain K steps (256
+// products, the shortest that split K makes of a long K); the epilogue warps add the chains'
+// sums in registers, rounded to nearest, while the next chain runs in the other accumulator.
+constexpr int kChain = 4;
 constexpr int kMaxClasses = 8;
 
 struct StreamMaps {

@@ -31,3 +31,14 @@ def test_chains_of_short_products(cilib, M, N, K, chain, form):
     c, ref = product(cilib, torch, M, N, K, lda_pad=(-K) % 8 if N != 515 else 0,
                      ldb_pad=(-K) % 8 if N != 515 else 0, seed=K, **form)
     assert error(c, ref) <= 1.2e-9 * chain + 2e-8
+
+
+@pytest.mark.parametrize("M,N,K,form", [(8192, 96, 1031, dict()), (8192, 200, 1031, dict(ta=1)),
+                                        (4096, 16, 2048, dict()), (1024, 33, 4096, dict(tb=0)),
+                                        (8192, 256, 1024, dict()), (5000, 100, 1100, dict(bias=True))])
+def test_chains_of_streamed_products(cilib, M, N, K, form):
+    """The kernel that streams a long A past a narrow B sums chains of 256 products (of 512,
+    up to 3.8e-7 here)."""
+    torch = pytest.importorskip("torch")
+    c, ref = product(cilib, torch, M, N, K, seed=N, **form)
+    assert error(c, ref) <= 1.2e-9 * 256 + 2e-8
