@@ -1144,9 +1144,11 @@ __global__ void __launch_bounds__(256) k_pack_bf16(const PackArgs P) {
   }
 }
 
-// C = alpha sum_z partial[z] (z in order) + beta C + bias, then tanh; BF16 copy.  Latency bounds it:
-// ten parts are read at once (20 parts of 256 x 256, cold under a profiler: 7.2 us four at a time,
-// 4.5 so).
+// C = alpha sum_z partial[z] (z in order) + beta C + bias, then tanh; BF16 copy.  Latency bounds
+// it where many parts make a small output, so U parts are read at once: ten (20 parts of 256 x
+// 256, cold under a profiler: 7.2 us four at a time, 4.5 so), or two and four where there are no
+// more (8,192 x 1,024 x 2,048 in two parts, both kernels: 105.2 us with ten, 86.4 with two).
+template <int U>
 __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int ldc,
                                 __nv_bfloat16* Cb, int M, int N, float alpha, float beta,
                                 const float* bias, int act) {
@@ -1156,12 +1158,12 @@ __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int 
   if (i >= (long long)M * N) return;
   const int row = (int)(i / N), col = (int)(i % N);
   float acc = 0.f;
-  for (int z0 = 0; z0 < splits; z0 += 10) {
-    float v[10];
+  for (int z0 = 0; z0 < splits; z0 += U) {
+    float v[U];
 #pragma unroll
-    for (int j = 0; j < 10; j++) v[j] = partial[(size_t)min(z0 + j, splits - 1) * M * N + i];
+    for (int j = 0; j < U; j++) v[j] = partial[(size_t)min(z0 + j, splits - 1) * M * N + i];
 #pragma unroll
-    for (int j = 0; j < 10; j++)
+    for (int j = 0; j < U; j++)
       if (z0 + j < splits) acc += v[j];
   }
   float v = alpha * acc;
@@ -1640,8 +1642,11 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
   }
   if (splits > 1) {
     const long long mn = (long long)M * N;
-    ci::launch_pdl(k_splitk_reduce, (unsigned)((mn + 255) / 256), 256, 0, st, partial, splits, C, ldc,
-                   cb, M, N, alpha, beta, bias, activation);
+    ci::launch_pdl(splits == 2  ? k_splitk_reduce<2>
+                   : splits <= 4 ? k_splitk_reduce<4>
+                                 : k_splitk_reduce<10>,
+                   (unsigned)((mn + 255) / 256), 256, 0, st, partial, splits, C, ldc, cb, M, N, alpha,
+                   beta, bias, activation);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(e));
