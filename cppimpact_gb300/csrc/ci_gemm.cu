@@ -553,6 +553,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
+// 16 of them: sums over several accumulators leave no registers for more
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+      "%12, %13, %14, %15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& mt, int& nt) {
   const int per_group = GROUP_M * tiles_n;
   const int g = t / per_group;
@@ -692,7 +704,11 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
     const int c_begin = (warp - 2) / 4 * COLS;
     int j = 0;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      // (cleared, not set by the first chain: a choice between the two takes as many registers again)
       float sum[COLS];
+#pragma unroll
+      for (int n = 0; n < COLS; n++) sum[n] = 0.f;
+#pragma unroll 1
       for (int kc = 0; kc < ktiles; kc += chain, j++) {
         const int b = j & 1;
         if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
@@ -701,12 +717,11 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-        for (int n = 0; n < COLS; n += 32) {
-          uint32_t r[32];
-          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
+        for (int n = 0; n < COLS; n += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
 #pragma unroll
-          for (int i = 0; i < 32; i++)
-            sum[n + i] = kc == 0 ? __uint_as_float(r[i]) : sum[n + i] + __uint_as_float(r[i]);
+          for (int i = 0; i < 16; i++) sum[n + i] += __uint_as_float(r[i]);
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncwarp();
@@ -793,10 +808,9 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
 // rate).
 //
 // Accuracy: the tensor core's FP32 sums lose about 1.1e-9 of the result per product in a chain
-// (measured: 7.3e-6 after 6,591, 2.9e-5 after 28,000).  A chain here is kChain K steps (256
-// products, the shortest that split K makes of a long K); the epilogue warps add the chains'
-// sums in registers, rounded to nearest, while the next chain runs in the other accumulator.
-constexpr int kChain = 4;
+// (measured: 7.3e-6 after 6,591, 2.9e-5 after 28,000).  A chain here is 4 or 8 K steps
+// (stream_chain); the epilogue warps add the chains' sums in registers, rounded to nearest, while
+// the next chain runs in the other accumulator.
 constexpr int kMaxClasses = 8;
 
 struct StreamMaps {
@@ -816,6 +830,7 @@ struct StreamArgs {
   int p, b_copies;         // classes; 1 or p copies of B
   int delta[kMaxClasses];  // elements in front of the rows of a class
   int tm, tn, kt;          // row tiles per class, column tiles, K steps
+  int chain;               // K steps of an accumulator
 };
 
 // Unit range of CTA b of g: [units b / g, units (b + 1) / g)
@@ -846,6 +861,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chain = P.chain;
   const long long units = (long long)P.p * P.tm * P.tn * P.kt;
   const long long u0 = stream_begin(units, blockIdx.x, gridDim.x);
   const long long u1 = stream_begin(units, blockIdx.x + 1, gridDim.x);
@@ -917,7 +933,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
       int c, mt, nt;
       stream_tile(P, t, c, mt, nt);
       const int delta = P.delta[c];
-      for (int kc = k0; kc < k1 && ok; kc += kChain, j++) {
+      for (int kc = k0; kc < k1 && ok; kc += chain, j++) {
         const int b = j & 1;
         if (j >= 2 && !mbar_wait_abort(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
           ok = false;
@@ -925,7 +941,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t acc_tmem = tmem + (uint32_t)(b * BN);
-        const int ke = min(k1, kc + kChain);
+        const int ke = min(k1, kc + chain);
         for (int k = kc; k < ke; k++, it++) {
           const int s = (int)(it % STAGES);
           // every lane waits, so that the masking below is ordered after the TMA write
@@ -986,8 +1002,11 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
       const int k1 = (int)min((long long)P.kt, k0 + (u1 - u));
       int c, mt, nt;
       stream_tile(P, t, c, mt, nt);
-      float sum[COLS];
-      for (int kc = k0; kc < k1; kc += kChain, j++) {
+      float sum[COLS];  // (cleared as in k_gemm_tma_pers)
+#pragma unroll
+      for (int n = 0; n < COLS; n++) sum[n] = 0.f;
+#pragma unroll 1
+      for (int kc = k0; kc < k1; kc += chain, j++) {
         const int b = j & 1;
         if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
           ok = false;
@@ -995,12 +1014,11 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-        for (int n = 0; n < COLS; n += 32) {
-          uint32_t r[32];
-          tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
+        for (int n = 0; n < COLS; n += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c_begin + n), r);
 #pragma unroll
-          for (int i = 0; i < 32; i++)
-            sum[n + i] = kc == k0 ? __uint_as_float(r[i]) : sum[n + i] + __uint_as_float(r[i]);
+          for (int i = 0; i < 16; i++) sum[n + i] += __uint_as_float(r[i]);
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncwarp();
@@ -1013,23 +1031,25 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
       const int rows_c = (P.M - c + P.p - 1) / P.p;  // rows of the class
       const bool whole = k0 == 0 && k1 == P.kt;
       float4* part = reinterpret_cast<float4*>(P.partial) +
-                     ((size_t)(2 * blockIdx.x + (u == u0 ? 0 : 1)) * (BN / 4) + c_begin / 4) * 128;
+                     ((size_t)(2 * blockIdx.x + (u == u0 ? 0 : 1)) * (BN / 4) + c_begin / 4) * 128 +
+                     q * 32 + lane;
+      if (whole) {
 #pragma unroll
-      for (int n = 0; n < COLS; n += 32) {
-        if (n0 + n >= P.N) break;
-        if (whole) {
+        for (int n = 0; n < COLS; n += 32) {
+          if (n0 + n >= P.N) break;
           uint32_t r[32];
 #pragma unroll
           for (int i = 0; i < 32; i++) r[i] = __float_as_uint(sum[n + i]);
           epi_store(epi_buf[warp - 2], r, mt * BM + q * 32, rows_c, n0 + n, P.N,
-                    P.C + (size_t)c * P.ldc, P.p * P.ldc,
-                    P.Cb ? P.Cb + (size_t)c * P.ldc : nullptr, P.alpha, P.beta, P.bias, P.act, lane);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; i++)
-            part[(size_t)(n / 4 + i) * 128 + q * 32 + lane] = make_float4(
-                sum[n + 4 * i], sum[n + 4 * i + 1], sum[n + 4 * i + 2], sum[n + 4 * i + 3]);
+                          P.C + (size_t)c * P.ldc, P.p * P.ldc,
+                          P.Cb ? P.Cb + (size_t)c * P.ldc : nullptr, P.alpha, P.beta, P.bias, P.act,
+                          lane);
         }
+      } else {
+#pragma unroll
+        for (int n = 0; n < COLS; n += 4)
+          if (n0 + n < P.N)
+            part[n / 4 * 128] = make_float4(sum[n], sum[n + 1], sum[n + 2], sum[n + 3]);
       }
       u += k1 - k0;
     }
@@ -1049,59 +1069,73 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
                  : "memory");
 }
 
-// The tiles that range ends cut: their partial sums in K order (four contiguous runs of them by
-// four warps, then the runs in order), then the epilogue.  Block (range end, 4 columns, 32
-// rows); the first end inside a tile stands for the tile.
-__global__ void __launch_bounds__(128) k_stream_reduce(const StreamArgs P, int BN, int g) {
-  __shared__ float4 run[4][32];
+// The tiles that range ends cut: their partial sums in K order, then the epilogue.  Block (cut
+// tile, 16 columns, 32 rows): a warp adds the parts of 4 columns, lanes along the rows, eight
+// parts in flight; the sums go through shared memory, so that a row's 16 columns are written
+// together.  With fewer tiles than ranges (by_tile) the blocks count tiles, else range ends, of
+// which the one that begins a tile's second range stands for it: few blocks have nothing to do.
+// (One block per range end, 4 columns and 32 rows whatever the tiles, 1,024 x 64 x 16,384 with
+// the products 21.5 us; 13.5 so.)
+__global__ void __launch_bounds__(128) k_stream_reduce(const StreamArgs P, int BN, int g, int by_tile) {
+  __shared__ float4 sums[4][33];
   ci::pdl_next();
   ci::pdl_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int row = blockIdx.z * 32 + lane;
   const long long units = (long long)P.p * P.tm * P.tn * P.kt;
-  const int b0 = blockIdx.x;  // ranges b0 and b0 + 1 meet at u
-  const long long u = stream_begin(units, b0 + 1, g);
-  const int t = (int)(u / P.kt);
+  const int t = by_tile ? blockIdx.x : (int)(stream_begin(units, blockIdx.x + 1, g) / P.kt);
   const long long ut = (long long)t * P.kt;
-  if (u == ut || stream_begin(units, b0, g) > ut) return;
-  const int b1 = (int)(((ut + P.kt) * g - 1) / units);
-  const float4* part = reinterpret_cast<const float4*>(P.partial) + (size_t)blockIdx.y * 128 + row;
-  const int per = (b1 - b0 + 4) / 4, lo = b0 + w * per, hi = min(b1 + 1, lo + per);
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  // the ranges with the tile's first and last units
+  const int b0 = (int)(((ut + 1) * g - 1) / units), b1 = (int)(((ut + P.kt) * g - 1) / units);
+  if (b0 == b1 || (!by_tile && b0 != (int)blockIdx.x)) return;
+  const size_t stride = (size_t)(BN / 4) * 128;
+  const float4* part = reinterpret_cast<const float4*>(P.partial) +
+                       (size_t)(4 * blockIdx.y + w) * 128 + blockIdx.z * 32 + lane;
+  float4 s = part[(2 * b0 + (stream_begin(units, b0, g) == ut ? 0 : 1)) * stride];
 #pragma unroll 8
-  for (int b = lo; b < hi; b++) {
-    const int slot = 2 * b + (stream_begin(units, b, g) >= ut ? 0 : 1);
-    const float4 v = part[(size_t)slot * (BN / 4) * 128];
+  for (int b = b0 + 1; b <= b1; b++) {
+    const float4 v = part[2 * b * stride];
     s.x += v.x;
     s.y += v.y;
     s.z += v.z;
     s.w += v.w;
   }
-  run[w][lane] = s;
+  sums[w][lane] = s;
   __syncthreads();
   int c, mt, nt;
   stream_tile(P, t, c, mt, nt);
-  const int i = mt * BM + row, col = nt * BN + 4 * blockIdx.y;
-  if (w > 0 || i >= (P.M - c + P.p - 1) / P.p || col >= P.N) return;
-  for (int k = 1; k < 4; k++) {
-    const float4 v = run[k][lane];
-    s.x += v.x;
-    s.y += v.y;
-    s.z += v.z;
-    s.w += v.w;
-  }
-  const float acc[4] = {s.x, s.y, s.z, s.w};
+  const int r = threadIdx.x >> 2, i = mt * BM + blockIdx.z * 32 + r;
+  const int col = nt * BN + 16 * blockIdx.y + 4 * (threadIdx.x & 3);
+  if (i >= (P.M - c + P.p - 1) / P.p || col >= P.N) return;
+  s = sums[threadIdx.x & 3][r];
   const size_t at = ((size_t)i * P.p + c) * P.ldc + col;
+  float v[4] = {P.alpha * s.x, P.alpha * s.y, P.alpha * s.z, P.alpha * s.w};
+  const bool vec = col + 4 <= P.N && (reinterpret_cast<uintptr_t>(P.C + at) & 15) == 0;
+  float old[4] = {0.f, 0.f, 0.f, 0.f};
+  if (P.beta != 0.f) {
+    if (vec)
+      *reinterpret_cast<float4*>(old) = *reinterpret_cast<const float4*>(P.C + at);
+    else
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (col + j < P.N) old[j] = P.C[at + j];
+  }
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    if (col + j >= P.N) break;
-    float v = P.alpha * acc[j];
-    if (P.beta != 0.f) v += P.beta * P.C[at + j];
-    if (P.bias) v += P.bias[col + j];
-    if (P.act == 1) v = tanhf(v);
-    P.C[at + j] = v;
-    if (P.Cb) P.Cb[at + j] = __float2bfloat16(v);
+    if (P.beta != 0.f) v[j] += P.beta * old[j];
+    if (P.bias && col + j < P.N) v[j] += P.bias[col + j];
+    if (P.act == 1) v[j] = tanhf(v[j]);
   }
+  if (vec) {
+    *reinterpret_cast<float4*>(P.C + at) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (col + j < P.N) P.C[at + j] = v[j];
+  }
+  if (P.Cb)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (col + j < P.N) P.Cb[at + j] = __float2bfloat16(v[j]);
 }
 
 // Operand copies that TMA can address: out [copies][rows][ld] with ld a multiple of 8 (the
@@ -1304,8 +1338,10 @@ cudaError_t launch_stream(const StreamMaps& maps, const StreamArgs& P, int grid,
                                        maps, P);
   if (e != cudaSuccess) return e;
   if (grid == 1) return cudaSuccess;
-  const int cols = std::min(BN, P.N);
-  return ci::launch_pdl(k_stream_reduce, dim3(grid - 1, (cols + 3) / 4, BM / 32), 128, 0, st, P, BN, grid);
+  const int cols = std::min(BN, P.N), tiles = P.p * P.tm * P.tn;
+  const bool by_tile = tiles < grid - 1;
+  return ci::launch_pdl(k_stream_reduce, dim3(by_tile ? tiles : grid - 1, (cols + 15) / 16, BM / 32), 128,
+                        0, st, P, BN, grid, (int)by_tile);
 }
 
 inline size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
@@ -1367,6 +1403,30 @@ void* workspace(int dev, cudaStream_t st, size_t need, std::unique_lock<std::mut
     w.size = need;
   }
   return w.p;
+}
+
+// Parts of K, multiples of a stage, where the output has too few tiles to fill the GPU and K is
+// long.
+struct SplitK {
+  int splits, k_chunk;
+};
+SplitK split_k(int tiles, int K) {
+  int splits = 1;
+  if (tiles < 304 && K >= 8 * BK)
+    splits = std::min((304 + tiles - 1) / tiles, (K + 4 * BK - 1) / (4 * BK));
+  splits = std::max(1, std::min(splits, 512));
+  int k_chunk = (K + splits - 1) / splits;
+  k_chunk = (k_chunk + BK - 1) / BK * BK;
+  return {(K + k_chunk - 1) / k_chunk, k_chunk};
+}
+
+// K steps of an accumulator of the streaming products: 256 products where K is short or split K
+// would make chains of less than 512, so that none is less exact than it, else 512, which costs
+// the epilogue warps half as much (40,000 x 32 x 20,480: 271 and 256 us; error against 64 bits
+// 2.5e-7 and 4.7e-7, of one chain 2.2e-5).
+int stream_chain(int M, int N, int K) {
+  const int bn = N <= 64 ? 64 : N <= 128 ? 128 : 256;
+  return K > 2048 && split_k((M + BM - 1) / BM * ((N + bn - 1) / bn), K).k_chunk >= 512 ? 8 : 4;
 }
 
 // How a product's operands reach the tensor-core kernels.
@@ -1514,6 +1574,20 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
     const int rc = choose_operands(A, lda, transA, B, ldb, transB, M, N, K, tma_shape, plain, st, &op);
     if (rc) return rc;
   }
+  int chain = 0;  // K steps of an accumulator of the persistent kernel (0: all)
+  // A streamed product of many tiles goes to the persistent kernel, in the same chains of K, where
+  // the SMs' idle time in its last round (0.37 us a K step: 16 KB of A at an SM's share of HBM)
+  // is below what cut tiles cost (a launch, and partial sums of BN columns).  65,536 x 256 x 1,024
+  // 65.4 us cut, 52.7 so; 65,536 x 64 x 1,024 36.7 and 31.6.
+  if (op.stream && op.p == 1 && op.max_delta == 0) {
+    const int w = N <= 64 ? 64 : N <= 128 ? 128 : 256, sms = num_sms();
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + w - 1) / w);
+    const double idle = (double)(((tiles + sms - 1) / sms) * sms - tiles) / sms * ((K + TBK - 1) / TBK);
+    if (tiles >= 2 * sms && 0.37 * idle <= 5.0 + 0.04 * N) {
+      op.stream = false;
+      chain = stream_chain(M, N, K);
+    }
+  }
   if (op.stream) {
     const int bn = N <= 64 ? 64 : N <= 96 ? 96 : N <= 128 ? 128 : 256;
     StreamArgs P{};
@@ -1533,6 +1607,7 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
     P.tm = ((M + op.p - 1) / op.p + BM - 1) / BM;
     P.tn = (N + bn - 1) / bn;
     P.kt = (K + op.max_delta + TBK - 1) / TBK;
+    P.chain = stream_chain(M, N, K);
     const long long units = (long long)P.p * P.tm * P.tn * P.kt;
     const int grid = (int)std::min<long long>(num_sms(), units);
     const size_t part = align256(sizeof(float) * 2 * (size_t)grid * BM * bn);
@@ -1563,24 +1638,19 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
   const int bn_tma = N <= 64 ? 64 : N <= 128 ? 128 : 256;
   int bn = tma ? bn_tma : (N <= 64 ? 64 : 128);
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-  // Split K when the output has too few tiles to fill the GPU and K is long.
-  int splits = 1;
-  if (tiles < 304 && K >= 8 * BK)
-    splits = std::min((304 + tiles - 1) / tiles, (K + 4 * BK - 1) / (4 * BK));
-  splits = std::max(1, std::min(splits, 512));
-  int k_chunk = (K + splits - 1) / splits;
-  k_chunk = (k_chunk + BK - 1) / BK * BK;
-  splits = (K + k_chunk - 1) / k_chunk;
+  SplitK cut = split_k(tiles, K);
+  if (chain) cut = {1, K};
   // With more than half a tile per SM and a short K the partial tiles cost more than the CTAs give
-  // (4,096 x 1,024 x 512 39.2 us, 8,192 x 512 x 896 49.6), but one chain of products over all of K would lose accuracy
+  // (4,096 x 1,024 x 512 39.2 us, 8,192 x 512 x 896 49.6), but one chain of products over all of K
+  // would lose accuracy
   // (8,192 x 512 x 896: 8.6e-7, in chains of 320 products 2.7e-7): the same chains, one after
-  // the other in the persistent kernel (12.2 and 16.3 us; as one chain 11.4 and 14.9).
-  int chain = 0;
-  if (tma && splits > 1 && 2 * tiles > num_sms() && K <= 896) {
-    chain = k_chunk / BK;
-    splits = 1;
-    bn = std::min(bn, 128);  // (256 columns would be 128 sums a thread)
+  // the other in the persistent kernel (12.2 and 15.6 us; as one chain 11.4 and 14.9).
+  if (tma && cut.splits > 1 && 2 * tiles > num_sms() && K <= 896) {
+    chain = cut.k_chunk / BK;
+    cut = {1, K};
+    bn = std::min(bn, 128);  // (8,192 x 1,024 x 512 18.5 us, with 256 columns 19.6)
   }
+  const int splits = cut.splits, k_chunk = cut.k_chunk;
   // Narrower tiles while they leave the GPU half empty: 256 x 256 x 256, two tiles of 256
   // columns, 13.5 us, eight of 64 7.3 (cold, under a profiler).  The sums of an output do not
   // depend on its tile.
@@ -1607,10 +1677,15 @@ int gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int tr
   dim3 grid((M + BM - 1) / BM, (N + bn - 1) / bn, splits);
   cudaError_t le = cudaSuccess;
   if (tma && chain) {
-    le = bn == 64 ? launch_pers<64, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias,
-                                                      activation, d_error, chain)
-                  : launch_pers<128, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta,
-                                                       bias, activation, d_error, chain);
+    if (bn == 64)
+      le = launch_pers<64, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias,
+                                             activation, d_error, chain);
+    else if (bn == 128)
+      le = launch_pers<128, TSTAGES, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias,
+                                              activation, d_error, chain);
+    else
+      le = launch_pers<256, 3, 8, true>(ta, tb, st, C, ldc, cb, M, N, K, alpha, beta, bias, activation,
+                                        d_error, chain);
     if (le != cudaSuccess) return ci::set_last_error(CI_ERR_CUDA, cudaGetErrorString(le));
   } else if (tma && splits == 1) {
     if (bn == 64)

@@ -42,3 +42,19 @@ def test_chains_of_streamed_products(cilib, M, N, K, form):
     torch = pytest.importorskip("torch")
     c, ref = product(cilib, torch, M, N, K, seed=N, **form)
     assert error(c, ref) <= 1.2e-9 * 256 + 2e-8
+
+
+@pytest.mark.parametrize("M,N,K", [(25001, 40, 1031), (25000, 72, 1024), (40000, 32, 1024),
+                                   (39001, 100, 1096), (39000, 200, 1032), (1024, 256, 4160),
+                                   (1030, 130, 6600), (300, 48, 20000), (4224, 97, 1024)])
+@pytest.mark.parametrize("form", [dict(), dict(bias=True, act=1, alpha=0.02, copy=True, ldc_pad=3),
+                                  dict(beta=0.5, ldc_pad=(4), c_off=4)])
+def test_streamed_tiles(cilib, M, N, K, form):
+    """Long products in whole tiles (304 tiles and more), in ranges that cut them, with fewer and
+    with more tiles than ranges, column tiles of 64 to 256.  Beside the chains of at most 512 the
+    sums of K / 256 of them round in FP32, 3e-8 of the result each, at random."""
+    torch = pytest.importorskip("torch")
+    c, ref = product(cilib, torch, M, N, K, seed=M, **form)
+    assert error(c, ref) <= 1.2e-9 * 512 + 3e-8 * (K / 256) ** 0.5
+    again, _ = product(cilib, torch, M, N, K, seed=M, **form)
+    assert np.array_equal(c, again)
