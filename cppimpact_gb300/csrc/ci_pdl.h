@@ -27,7 +27,9 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
   a.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &a;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by a later call
+  return e;
 }
 
 }  // namespace ci

@@ -58,3 +58,24 @@ def test_streamed_tiles(cilib, M, N, K, form):
     assert error(c, ref) <= 1.2e-9 * 512 + 3e-8 * (K / 256) ** 0.5
     again, _ = product(cilib, torch, M, N, K, seed=M, **form)
     assert np.array_equal(c, again)
+
+
+@pytest.mark.parametrize("M,N,K,ta,tb", [(2097121, 20, 12, 0, 1), (2200000, 8, 48, 1, 1),
+                                         (8, 2200000, 10, 0, 0), (1, 9, 8400000, 1, 0)])
+def test_copies_of_many_rows(cilib, M, N, K, ta, tb):
+    """Operands to be copied with more than 32 * 65,535 rows, and more than 128 * 65,535 columns,
+    checked in 64 bits on the device."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn((K, M) if ta else (M, K), generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn((N, K) if tb else (K, N), generator=g, device="cuda").to(torch.bfloat16)
+    c = torch.full((M, N), float("nan"), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rc = cilib.lib().ci_gemm_bf16(a.data_ptr(), a.shape[1], ta, b.data_ptr(), b.shape[1], tb,
+                                  c.data_ptr(), N, None, M, N, K, 1.0, 0.0, None, 0,
+                                  err.data_ptr(), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, cilib.lib().ci_last_error()
+    assert int(err.item()) == 0
+    ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    assert float((c.double() - ref).norm() / ref.norm()) <= 1e-5
