@@ -438,6 +438,12 @@ __device__ __forceinline__ bool mbar_wait_abort(uint32_t bar, uint32_t phase, vo
   return false;
 }
 
+// The same by a whole warp, with one outcome for its lanes: a lane that gave up by itself would
+// leave the others waiting for it at their next warp-wide instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t phase, volatile int* abort) {
+  return __all_sync(0xffffffffu, mbar_wait_abort(bar, phase, abort));
+}
+
 // Epilogue of 32 x 32 accumulators by one warp, turned through shared memory (buf, 32 rows
 // of EPI_LD floats): r holds lane's row, the stores go out row by row, 128 contiguous bytes
 // at a time (16-byte stores where C's rows allow it).  A lane storing its own row touches 32
@@ -711,7 +717,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
 #pragma unroll 1
       for (int kc = 0; kc < ktiles; kc += chain, j++) {
         const int b = j & 1;
-        if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
+        if (!mbar_wait_warp(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
           ok = false;
           break;
         }
@@ -751,7 +757,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
     int j = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, j++) {
       const int b = j & 1;
-      if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
+      if (!mbar_wait_warp(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
         ok = false;
         break;
       }
@@ -935,7 +941,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
       const int delta = P.delta[c];
       for (int kc = k0; kc < k1 && ok; kc += chain, j++) {
         const int b = j & 1;
-        if (j >= 2 && !mbar_wait_abort(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
+        if (j >= 2 && !mbar_wait_warp(smem_u32(&tempty[b]), (uint32_t)((j >> 1) - 1) & 1u, abort)) {
           ok = false;
           break;
         }
@@ -945,8 +951,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
         for (int k = kc; k < ke; k++, it++) {
           const int s = (int)(it % STAGES);
           // every lane waits, so that the masking below is ordered after the TMA write
-          if (!mbar_wait_abort(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) ok = false;
-          if (!__all_sync(0xffffffffu, ok)) {
+          if (!mbar_wait_warp(smem_u32(&full[s]), (uint32_t)(it / STAGES) & 1u, abort)) {
             ok = false;
             break;
           }
@@ -1008,7 +1013,7 @@ __global__ void __launch_bounds__(64 + 32 * EPW, 1)
 #pragma unroll 1
       for (int kc = k0; kc < k1; kc += chain, j++) {
         const int b = j & 1;
-        if (!mbar_wait_abort(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
+        if (!mbar_wait_warp(smem_u32(&tfull[b]), (uint32_t)(j >> 1) & 1u, abort)) {
           ok = false;
           break;
         }
