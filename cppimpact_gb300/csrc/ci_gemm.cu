@@ -39,6 +39,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/cppimpact_gb300.h"
 #include "ci_pdl.h"
@@ -1220,14 +1222,18 @@ __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int 
 // that do share one).  At most kMaxWorkspaces are kept per device; a new stream beyond
 // that frees the device's others first.  A caller holds g_ws_mu from the lookup until
 // its kernels are enqueued, and cudaFree synchronises the device, so no workspace is
-// freed while a call still uses it.
+// freed while a call still uses it.  One that a call used while its stream was captured is
+// never freed: the graph's replays use it whenever they run.
 struct Workspace {
   float* p = nullptr;
   size_t size = 0;
+  bool captured = false;
 };
 constexpr size_t kMaxWorkspaces = 32;
 std::mutex g_ws_mu;
 std::map<std::pair<int, cudaStream_t>, Workspace> g_ws;
+// outgrown while their stream was captured, where nothing may be freed
+std::vector<std::pair<int, void*>> g_ws_later;
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -1380,16 +1386,37 @@ __global__ void __launch_bounds__(256) k_gemm_small(const __nv_bfloat16* A, int 
   if (Cb) Cb[(size_t)row * ldc + col] = __float2bfloat16(v);
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;  // the legacy stream while another one is captured
+}
+
+// Empties a workspace; cudaFree synchronises the device, so no call still uses it.
+void release(Workspace& w) {
+  if (w.p && !w.captured) cudaFree(w.p);
+  w = Workspace();
+}
+
 // The stream's workspace, grown to `need` bytes (null: no memory); takes the lock.
 void* workspace(int dev, cudaStream_t st, size_t need, std::unique_lock<std::mutex>& lock) {
   lock.lock();
-  if (!g_ws.count({dev, st})) {
+  const bool cap = capturing(st);
+  if (!cap) {
+    for (size_t i = 0; i < g_ws_later.size();)
+      if (g_ws_later[i].first == dev) {
+        cudaFree(g_ws_later[i].second);
+        g_ws_later.erase(g_ws_later.begin() + i);
+      } else {
+        i++;
+      }
     size_t on_dev = 0;
     for (const auto& kv : g_ws) on_dev += kv.first.first == dev;
-    if (on_dev >= kMaxWorkspaces)
+    if (!g_ws.count({dev, st}) && on_dev >= kMaxWorkspaces)
       for (auto it = g_ws.begin(); it != g_ws.end();) {
         if (it->first.first == dev) {
-          if (it->second.p) cudaFree(it->second.p);
+          release(it->second);
           it = g_ws.erase(it);
         } else {
           ++it;
@@ -1398,17 +1425,18 @@ void* workspace(int dev, cudaStream_t st, size_t need, std::unique_lock<std::mut
   }
   Workspace& w = g_ws[{dev, st}];
   if (w.size < need) {
-    if (w.p) cudaFree(w.p);  // synchronises the device: no call still reads it
-    w.p = nullptr;
-    w.size = 0;
+    if (!cap) release(w);
     void* p = nullptr;
     if (cudaMalloc(&p, need) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
+    if (w.p && !w.captured) g_ws_later.push_back({dev, w.p});
+    w = Workspace();
     w.p = static_cast<float*>(p);
     w.size = need;
   }
+  w.captured = w.captured || cap;
   return w.p;
 }
 
@@ -1478,13 +1506,9 @@ int choose_operands(const void* A, int lda, int transA, const void* B, int ldb, 
   }
   // A of 8 MB or more read once past a B of at most 256 rows, K long enough to cut
   const bool streams = N <= 256 && (long long)M * K >= (1 << 22) && K >= 1024;
-  if (!tma_shape || streams) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      op->tma = tma_shape;
-      return CI_OK;
-    }
+  if ((!tma_shape || streams) && capturing(st)) {
+    op->tma = tma_shape;
+    return CI_OK;
   }
   if (!tma_shape) {
     if ((transA ? lda < M : lda < K) || (transB ? ldb < K : ldb < N)) return CI_OK;

@@ -79,3 +79,56 @@ def test_copies_of_many_rows(cilib, M, N, K, ta, tb):
     assert int(err.item()) == 0
     ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
     assert float((c.double() - ref).norm() / ref.norm()) <= 1e-5
+
+
+def test_captured_workspace_outlives_larger_calls(cilib):
+    """A graph keeps the partial sums' address of its split product: a later call on the same
+    stream that needs more memory must leave that memory alone.  (This one also captures behind
+    a copy and behind a joined stream.)"""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    s, side = torch.cuda.Stream(), torch.cuda.Stream()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def call(a, b, c, tb=1):
+        rc = cilib.lib().ci_gemm_bf16(a.data_ptr(), a.shape[1], 0, b.data_ptr(), b.shape[1], tb,
+                                      c.data_ptr(), c.shape[1], None, a.shape[0], c.shape[1],
+                                      a.shape[1], 1.0, 0.0, None, 0, err.data_ptr(),
+                                      C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, cilib.lib().ci_last_error()
+
+    a, b = rand(256, 2048), rand(300, 2048)
+    a2, c, d = torch.empty_like(a), *(torch.empty((256, 300), device="cuda") for _ in range(2))
+    big_a, big_b = rand(2000, 8008), rand(8008, 500)
+    big_c = torch.empty((2000, 500), device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        call(a, b, c)   # the workspace exists before the capture
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        a2.copy_(a)
+        call(a2, b, c)
+        side.wait_stream(s)
+        with torch.cuda.stream(side):
+            e = c + 0.0
+        call(a2, b, d)
+        s.wait_stream(side)
+        call(a2, b, d)
+        graph.capture_end()
+        ref = a.double() @ b.double().t()
+        for _ in range(3):
+            call(big_a, big_b, big_c, tb=0)
+            torch.cuda.synchronize()
+            # whatever was freed is somebody else's now
+            other = [torch.zeros(1 << 20, device="cuda") for _ in range(64)]
+            c.zero_(), d.zero_(), a2.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            for x in (c, d, e):
+                assert float((x.double() - ref).norm() / ref.norm()) <= 1e-6
+            assert all(not bool(o.any()) for o in other)
+    big = big_a.double() @ big_b.double()
+    assert float((big_c.double() - big).norm() / big.norm()) <= 1e-6 and int(err.item()) == 0
