@@ -1224,12 +1224,19 @@ __global__ void k_splitk_reduce(const float* partial, int splits, float* C, int 
 // its kernels are enqueued, and cudaFree synchronises the device, so no workspace is
 // freed while a call still uses it.  One that a call used while its stream was captured is
 // never freed: the graph's replays use it whenever they run.
+// Operand copies make workspaces of up to some 300 MB, so together a device's hold kMaxKept at
+// most (beyond it, and where an allocation fails, the others are freed), and one of more than
+// kKeepBytes goes back when kIdleCalls calls in a row needed less than half of it.
 struct Workspace {
   float* p = nullptr;
   size_t size = 0;
   bool captured = false;
+  int idle = 0;  // calls in a row that needed less than half
 };
 constexpr size_t kMaxWorkspaces = 32;
+constexpr size_t kMaxKept = (size_t)512 << 20;
+constexpr size_t kKeepBytes = (size_t)64 << 20;
+constexpr int kIdleCalls = 64;
 std::mutex g_ws_mu;
 std::map<std::pair<int, cudaStream_t>, Workspace> g_ws;
 // outgrown while their stream was captured, where nothing may be freed
@@ -1424,10 +1431,31 @@ void* workspace(int dev, cudaStream_t st, size_t need, std::unique_lock<std::mut
       }
   }
   Workspace& w = g_ws[{dev, st}];
+  w.idle = need < w.size / 2 ? w.idle + 1 : 0;
+  if (!cap && w.size > kKeepBytes && w.idle >= kIdleCalls) release(w);
   if (w.size < need) {
-    if (!cap) release(w);
+    auto release_others = [&](size_t keep) {  // until they hold `keep` bytes
+      size_t held = 0;
+      for (const auto& kv : g_ws)
+        if (kv.first.first == dev && &kv.second != &w) held += kv.second.size;
+      for (auto& kv : g_ws)
+        if (kv.first.first == dev && &kv.second != &w && !kv.second.captured && held > keep) {
+          held -= kv.second.size;
+          release(kv.second);
+        }
+    };
+    if (!cap) {
+      release(w);
+      release_others(need < kMaxKept ? kMaxKept - need : 0);
+    }
     void* p = nullptr;
-    if (cudaMalloc(&p, need) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&p, need);
+    if (e != cudaSuccess && !cap) {
+      cudaGetLastError();
+      release_others(0);
+      e = cudaMalloc(&p, need);
+    }
+    if (e != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }

@@ -132,3 +132,42 @@ def test_captured_workspace_outlives_larger_calls(cilib):
             assert all(not bool(o.any()) for o in other)
     big = big_a.double() @ big_b.double()
     assert float((big_c.double() - big).norm() / big.norm()) <= 1e-6 and int(err.item()) == 0
+
+
+def test_workspaces_are_bounded_and_given_back(cilib):
+    """Copies of 126 MB on eight streams hold 512 MB together, not 1 GB; a stream that goes on
+    with small split products gives its 130 MB back."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a = torch.randn((327680, 96), generator=g, device="cuda").to(torch.bfloat16)
+    sa, sb = (torch.randn((256, 2048), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    c, d = torch.empty((96, 96), device="cuda"), torch.empty((256, 256), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(8)]
+    L = cilib.lib()
+
+    def big(s):
+        assert L.ci_gemm_bf16(a.data_ptr(), 96, 1, a.data_ptr(), 96, 0, c.data_ptr(), 96, None, 96, 96,
+                              327680, 1.0, 0.0, None, 0, err.data_ptr(), C.c_void_p(s.cuda_stream)) == 0
+        torch.cuda.synchronize()
+
+    def small(s):
+        assert L.ci_gemm_bf16(sa.data_ptr(), 2048, 0, sb.data_ptr(), 2048, 1, d.data_ptr(), 256, None,
+                              256, 256, 2048, 1.0, 0.0, None, 0, err.data_ptr(),
+                              C.c_void_p(s.cuda_stream)) == 0
+        torch.cuda.synchronize()
+
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for s in streams:
+        big(s)
+    ref = a.double().t() @ a.double()
+    assert float((c.double() - ref).norm() / ref.norm()) <= 1e-6
+    assert free0 - torch.cuda.mem_get_info()[0] <= 600 << 20
+    big(streams[0])
+    held = torch.cuda.mem_get_info()[0]
+    for _ in range(70):
+        small(streams[0])
+    assert torch.cuda.mem_get_info()[0] - held >= 100 << 20
+    assert int(err.item()) == 0
