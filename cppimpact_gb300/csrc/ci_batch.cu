@@ -444,7 +444,8 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   CB_CUDA(G.sig_b.alloc(E * G.nq));
   CB_CUDA(G.epbar.alloc(E * G.nq));
   CB_CUDA(G.work.alloc(4 * (size_t)G.C));
-  CB_CUDA(G.status.alloc(1));
+  CB_CUDA(G.status.alloc(kStatusWords));
+  CB_CUDA(cudaMemsetAsync(G.status.p, 0, sizeof(unsigned int) * kStatusWords, st));  // no copy in host memory
   CB_CUDA(G.step_ctr.alloc(1));
   CB_CUDA(G.peak.alloc(G.insts.size()));
   CB_CUDA(npe == 4 ? configure<4>((int)G.smem) : configure<10>((int)G.smem));

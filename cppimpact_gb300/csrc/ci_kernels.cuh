@@ -32,6 +32,19 @@ enum ElemMode { EM_J2 = 0, EM_REFCOMPAT = 1, EM_MASS_ROWSUM = 2, EM_MASS_HRZ = 3
 
 enum StatusBits { ST_DEGENERATE = 1u, ST_NONFINITE = 2u, ST_FLOW_TIMEOUT = 8u };
 
+// A status block on the device: the bits, and in words 2 and 3 the address of a copy of them
+// in host memory (null: none).  A lane looks before it writes, so that a run in which every
+// element or node reports costs reads of the L2 cache, and the host's copy, a trip over the bus
+// for every write, is written once a bit.  (20 steps of 384,000 tet4 without a finite node: 3.2
+// ms with the word in host memory alone, 0.52 in device memory alone, 0.43 so.)
+constexpr int kStatusWords = 4;
+__device__ __forceinline__ void report(unsigned int* status, unsigned int bit) {
+  if (*static_cast<volatile unsigned int*>(status) & bit) return;
+  if (atomicOr(status, bit) & bit) return;
+  unsigned int* const host = *reinterpret_cast<unsigned int**>(status + 2);
+  if (host) atomicOr_system(host, bit);
+}
+
 struct DevPlan {
   const ChunkInfo* chunks;
   const uint16_t* conn_local;  // [npe][E]
@@ -268,7 +281,7 @@ __device__ __forceinline__ void element_force_on(const ElemParams& p, const Stat
         for (int j = 0; j < 3; j++) J[3 * a + j] = fmaf(x[i][a], G[i][j], J[3 * a + j]);
     float Ji[9];
     const float detJ = inv3f(J, Ji);
-    if (!(detJ > 0.f)) atomicOr(S.status, (unsigned)ST_DEGENERATE);
+    if (!(detJ > 0.f)) report(S.status, ST_DEGENERATE);
     const float wd = R::W * detJ;
     vol += wd;
     ve += wd;
@@ -516,7 +529,7 @@ __global__ void __launch_bounds__(256) k_node(NodeArrays A, NodeParams p) {
     if (!INIT) A.u[k][n] = un[k];
     if (STORE_ACC) A.acc[k][n] = (float)a[k];
   }
-  if (!finite) atomicOr(A.status, (unsigned)ST_NONFINITE);
+  if (!finite) report(A.status, ST_NONFINITE);
 }
 
 // ---------------------------------------------------------------------------
@@ -673,7 +686,7 @@ __device__ __forceinline__ void store_node(const FusedArgs& A, double* const (&u
     finite = finite && isfinite(vf[k]);
     if (store_acc) A.acc[k][g] = a[k];
   }
-  if (!finite) atomicOr(A.status, (unsigned)ST_NONFINITE);
+  if (!finite) report(A.status, ST_NONFINITE);
   const unsigned char flag = in_contact ? 3 : (old & 2);
   if (flag != old) A.contact[g] = flag;
 }
@@ -1294,7 +1307,7 @@ __device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& 
   }
   float Ji[9];
   const float detJ = inv3f(J, Ji);
-  if (act && !(detJ > 0.f)) atomicOr(status, (unsigned)ST_DEGENERATE);
+  if (act && !(detJ > 0.f)) report(status, ST_DEGENERATE);
   const float wd = act ? W * detJ : 0.f;
   float Lg[9];
 #pragma unroll
@@ -1630,7 +1643,7 @@ __device__ __forceinline__ bool flow_wait(const FlowArgs& F, const int* ctr, con
         const unsigned long long t = global_ns();
         if (t0 == 0) t0 = t;
         if (t - t0 > F.wait_ns) {
-          atomicOr(F.A[0].status, (unsigned)ST_FLOW_TIMEOUT);
+          report(F.A[0].status, ST_FLOW_TIMEOUT);
           atomicExch(F.abort_flag, 1);
           ok = false;
           break;
@@ -1996,7 +2009,7 @@ __device__ __forceinline__ void tet10_bary_element(const ElemParams& ep, const F
     }
     float Ji[9];
     const float detJ = inv3f<false>(J, Ji);
-    if (!(detJ > 0.f)) atomicOr(A.status, (unsigned)ST_DEGENERATE);
+    if (!(detJ > 0.f)) report(A.status, ST_DEGENERATE);
     const float wd = W * detJ;
     float Lg[9];
 #pragma unroll
@@ -2189,7 +2202,7 @@ __global__ void __launch_bounds__(256) k_node_init(NodeArrays A, NodeParams p_ar
     A.acc[k][n] = (float)ad[k];
   }
   A.contact[n] = flag;
-  if (!finite) atomicOr(A.status, (unsigned)ST_NONFINITE);
+  if (!finite) report(A.status, ST_NONFINITE);
 }
 
 // Adds n to the batched step counter (after each captured block of steps).

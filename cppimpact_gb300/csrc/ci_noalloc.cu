@@ -42,7 +42,7 @@ constexpr unsigned int kBadIndex = 4u;  // beside ci::ST_DEGENERATE (1) and ST_N
 
 // per-block partial (energy, volume) of one call: block b writes entries 2b and 2b + 1
 static __device__ __align__(256) double g_partials[2 * kMaxBlocks];
-static __device__ __align__(256) unsigned int g_status;
+static __device__ __align__(256) unsigned int g_status[ci::kStatusWords];
 
 std::mutex g_mu;
 double* g_partials_ptr[kMaxDevices] = {};
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kThreads) k_energy_partials(const double* __re
       n[a] = conn[(size_t)NPE * e + a];
       ok = ok && (unsigned)n[a] < (unsigned)N;
     }
-    if (!ok) atomicOr(status, kBadIndex);
+    if (!ok) ci::report(status, kBadIndex);
   }
   if (ok) {
     float xe[NPE][3], ue[NPE][3];

@@ -91,7 +91,7 @@ static __device__ __noinline__ bool res_patience(const ResidentArgs& A, unsigned
     if (t0 == 0) t0 = t;
     if (t - t0 <= A.wait_ns) return true;
   }
-  atomicOr(A.status, (unsigned)ST_FLOW_TIMEOUT);
+  report(A.status, ST_FLOW_TIMEOUT);
   atomicExch(A.abort_flag, 1);
   return false;
 }
@@ -336,7 +336,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     r[1] = ep.dt * vf[0];
     r[3] = ep.dt * vf[1];
     T.p1[l].y = ep.dt * vf[2];
-    if (!finite) atomicOr(A.status, (unsigned)ST_NONFINITE);
+    if (!finite) report(A.status, ST_NONFINITE);
     if (last && l < ch.n_own)
 #pragma unroll
       for (int c = 0; c < 3; c++) A.acc[c][ch.own_begin + l] = a[c];
