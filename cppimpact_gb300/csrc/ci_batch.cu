@@ -241,10 +241,10 @@ cudaError_t prepare_step(Group& G) {
   const int bs = G.block_threads;
   if (G.npe == 4) {
     G.step = step_form(G.C, device, bs, G.max_local, G.max_chunk_elems);
-    return configure_step_kernel(step_kernel<EM_J2, true>(bs, G.step), device);
+    return raise_smem(step_kernel<EM_J2, true>(bs, G.step), device);
   }
   G.step10 = step_form10(G.C, device, bs, G.max_local, G.max_chunk_elems);
-  return configure_step_kernel(kernel10(G), device);
+  return raise_smem(kernel10(G), device);
 }
 
 cudaError_t launch_batch(Group& G, const FusedArgs& F) {
@@ -254,16 +254,6 @@ cudaError_t launch_batch(Group& G, const FusedArgs& F) {
                       G.stream, F, ElemParams{}, NodeParams{});
   return launch_pdl(kernel10(G), G.C, one_lane(G) ? bs : G.step10.threads,
                     one_lane(G) ? G.smem : G.step10.smem, G.stream, F, ElemParams{}, NodeParams{});
-}
-
-template <int NPE>
-cudaError_t configure(int bytes) {
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_elem<NPE, EM_MASS_HRZ, 256>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  return cudaFuncSetAttribute(k_elem<NPE, EM_MASS_ROWSUM, 256>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 // Build one element-type group from its instances.
@@ -448,7 +438,8 @@ int build_group(ci_batch* b, Group& G, const ci_instance* in, const ci_options& 
   CB_CUDA(cudaMemsetAsync(G.status.p, 0, sizeof(unsigned int) * kStatusWords, st));  // no copy in host memory
   CB_CUDA(G.step_ctr.alloc(1));
   CB_CUDA(G.peak.alloc(G.insts.size()));
-  CB_CUDA(npe == 4 ? configure<4>((int)G.smem) : configure<10>((int)G.smem));
+  CB_CUDA(npe == 4 ? raise_smem(k_elem<4, EM_MASS_HRZ, 256>, b->device, G.smem)
+                   : raise_smem(k_elem<10, EM_MASS_HRZ, 256>, b->device, G.smem));
   // the resident form, where every instance's chunks fit the GPU together: a launch for the
   // instances of each CTA size (resident_threads)
   G.res.clear();

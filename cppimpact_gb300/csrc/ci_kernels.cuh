@@ -1074,6 +1074,21 @@ __global__ void __launch_bounds__(BS * W, 1024 / (BS * W))
 
 using StepKernel = void (*)(FusedArgs, ElemParams, NodeParams);
 
+// A kernel's dynamic shared-memory limit is one for the process: it is raised to all that the
+// device offers, whatever a solver needs (need bytes, checked), as a smaller limit set for the
+// next solver would refuse this one's launches.  Not inside a stream capture.
+template <class... A>
+cudaError_t raise_smem(void (*kernel)(A...), int device, size_t need = 0) {
+  int smem_max = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  cudaFuncAttributes fa;
+  if (!e) e = cudaFuncGetAttributes(&fa, kernel);
+  if (e) return e;
+  const int limit = smem_max - (int)fa.sharedSizeBytes;
+  if (need > (size_t)limit) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
 // Form of the tet4 step kernel: windows at a time, shared memory.
 struct StepForm {
   int W = 1;
@@ -1117,18 +1132,6 @@ inline StepForm step_form(int C, int device, int bs, int max_local, int max_elem
     }
   }
   return best;
-}
-
-// Its shared-memory limit is the device's, whatever a solver needs: several solvers share it.
-inline cudaError_t configure_step_kernel(StepKernel k, int device) {
-  int smem_max = 0;
-  cudaError_t e =
-      cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  cudaFuncAttributes fa;
-  if (!e) e = cudaFuncGetAttributes(&fa, k);
-  if (e) return e;
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              smem_max - (int)fa.sharedSizeBytes);
 }
 
 // ---------------------------------------------------------------------------

@@ -301,39 +301,23 @@ cudaError_t launch_elem(ci_solver* s, const ci::DevState& D, const ci::ElemParam
   return cudaGetLastError();
 }
 
-template <int BS>
-cudaError_t configure_step10(int bytes) {
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_J2, BS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  if ((e = cudaFuncSetAttribute(ci::k_step_t10<ci::EM_REFCOMPAT, BS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  return cudaSuccess;
-}
-
-// Raise the dynamic shared-memory limit of the element kernels once per solver (not
-// inside stream capture).
+// Raise the dynamic shared-memory limits of the element kernels and the one-lane step kernels.
 template <int NPE>
-cudaError_t configure_npe(int bytes) {
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_J2, kBS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  if ((e = cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_REFCOMPAT, kBS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
-  if ((e = cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_MASS_ROWSUM, kBS>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-    return e;
+cudaError_t configure_npe(const ci_solver* s) {
+  const int d = s->device;
+  const size_t b = s->smem_bytes;
+  cudaError_t e = ci::raise_smem(ci::k_elem<NPE, ci::EM_J2, kBS>, d, b);
+  if (!e) e = ci::raise_smem(ci::k_elem<NPE, ci::EM_REFCOMPAT, kBS>, d, b);
+  if (!e) e = ci::raise_smem(ci::k_elem<NPE, ci::EM_MASS_ROWSUM, kBS>, d, b);
+  if (!e) e = ci::raise_smem(ci::k_elem<NPE, ci::EM_MASS_HRZ, kBS>, d, b);
   if (NPE == 10) {
-    if ((e = configure_step10<64>(bytes))) return e;
-    if ((e = configure_step10<128>(bytes))) return e;
-    if ((e = configure_step10<256>(bytes))) return e;
+    for (const ci::StepKernel k :
+         {ci::k_step_t10<ci::EM_J2, 64>, ci::k_step_t10<ci::EM_J2, 128>, ci::k_step_t10<ci::EM_J2, 256>,
+          ci::k_step_t10<ci::EM_REFCOMPAT, 64>, ci::k_step_t10<ci::EM_REFCOMPAT, 128>,
+          ci::k_step_t10<ci::EM_REFCOMPAT, 256>})
+      if (!e) e = ci::raise_smem(k, d, b);
   }
-  return cudaFuncSetAttribute(ci::k_elem<NPE, ci::EM_MASS_HRZ, kBS>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e;
 }
 
 template <int BS>
@@ -618,7 +602,7 @@ int setup_flow(ci_solver* s) {
   CI_CUDA(s->d_flow_ctr.alloc(2 * (size_t)C + 2));
   auto kern = s->opt.mode != CI_MODE_REFCOMPAT ? ci::k_flow_qp10<ci::EM_J2, 128>
                                                : ci::k_flow_qp10<ci::EM_REFCOMPAT, 128>;
-  CI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->flow_smem));
+  CI_CUDA(ci::raise_smem(kern, s->device, s->flow_smem));
   int per_sm = 0, sms = 0;
   CI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, s->flow_smem));
   CI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
@@ -728,12 +712,12 @@ int setup_step(ci_solver* s) {
   const bool j2 = s->opt.mode != CI_MODE_REFCOMPAT;
   if (s->npe == 4) {
     s->step = ci::step_form(s->C, s->device, bs, P.max_local, P.max_chunk_elems);
-    CI_CUDA(ci::configure_step_kernel(j2 ? ci::step_kernel<ci::EM_J2, false>(bs, s->step)
+    CI_CUDA(ci::raise_smem(j2 ? ci::step_kernel<ci::EM_J2, false>(bs, s->step)
                                          : ci::step_kernel<ci::EM_REFCOMPAT, false>(bs, s->step),
                                       s->device));
   } else {
     s->step10 = ci::step_form10(s->C, s->device, bs, P.max_local, P.max_chunk_elems);
-    CI_CUDA(ci::configure_step_kernel(j2 ? ci::step_kernel10<ci::EM_J2, false>(bs, s->step10)
+    CI_CUDA(ci::raise_smem(j2 ? ci::step_kernel10<ci::EM_J2, false>(bs, s->step10)
                                          : ci::step_kernel10<ci::EM_REFCOMPAT, false>(bs, s->step10),
                                       s->device));
   }
@@ -1147,7 +1131,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   s->X = s->X0;
   s->vel0.assign(3, 0.0);
 
-  CI_CUDA(s->npe == 4 ? configure_npe<4>((int)s->smem_bytes) : configure_npe<10>((int)s->smem_bytes));
+  CI_CUDA(s->npe == 4 ? configure_npe<4>(s.get()) : configure_npe<10>(s.get()));
   if (s->plan.repeats && s->opt.step_kernel != 1) s->opt.step_kernel = 3;  // not the task kernel
   if (s->opt.step_kernel == 0) {
     // automatic: the task kernel when the chunks of a four-lane tet10 mesh need more than
@@ -1169,7 +1153,7 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
     // L1 for the read-only connectivity and index loads (shell: 98 against 107 us per
     // step with the 896-node default, which suits the fused kernel)
     if ((rc = make_plan(kTaskChunkNodes))) return rc;
-    CI_CUDA(configure_npe<10>((int)s->smem_bytes));
+    CI_CUDA(configure_npe<10>(s.get()));
   }
   const ci::Plan& P = s->plan;
   CI_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
