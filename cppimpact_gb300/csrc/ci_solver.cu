@@ -1142,8 +1142,9 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
     s->opt.step_kernel = 3;
     if (s->npe == 10 && s->opt.elem_lanes == 4 && s->opt.block_threads == 128) {
       int per_sm = 0, sms = 0;
-      CI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, ci::k_step_qp10<ci::EM_J2, 128, 128>, 128, s->smem_bytes));
+      const ci::StepKernel fused = ci::k_step_qp10<ci::EM_J2, 128, 128>;
+      CI_CUDA(ci::raise_smem(fused, s->device, s->smem_bytes));  // else no CTA of more than 48 KB fits
+      CI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused, 128, s->smem_bytes));
       CI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
       if (5LL * s->C > 4LL * per_sm * sms) s->opt.step_kernel = 2;
     }

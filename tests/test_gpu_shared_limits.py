@@ -68,3 +68,19 @@ def test_a_smaller_batch_comes_second(cilib, order):
             c.close()
     for k in ("x", "v", "epbar", "contact"):
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+def test_automatic_kernel_of_the_first_solver(cilib):
+    """The automatic choice asks how many chunks fit an SM.  In a process of its own: the first
+    solver, with chunks beyond the 48 KB that a kernel has by default, takes the kernel that
+    any later one does (few chunks: the fused one)."""
+    code = ("import sys; sys.path.insert(0, %r)\n"
+            "from cppimpact_gb300 import api, meshgen as mg\n"
+            "m = mg.cube(10, 2)\n"
+            "k = [api.Solver(m.xloc, m.conn, E=1e9, nu=0.3, rho=1e3, chunk_nodes=n, chunk_elements=4096)"
+            ".step_kernel() for n in (1400, 512, 1400)]\n"
+            "print(k)\n" % ROOT)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ))
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split("\n")[0] == "[3, 3, 3]"
