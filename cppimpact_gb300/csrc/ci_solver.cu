@@ -3,6 +3,7 @@
 // Host orchestration: preprocessing (ci_plan.cpp), device buffers, the one-time
 // lumped mass and initial half step, graph-captured stepping, read-back in the
 // caller's node/element order, one-shot kernels for parity checks.
+#include <cuda.h>  // pointer attributes; the function is fetched at run time
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1279,17 +1280,41 @@ int ci_steps_done(const ci_solver* s, long long* nsteps) {
 }
 
 // The device's address of a caller's array of n doubles that lies whole in page-locked host
-// memory, else null.
+// memory, else null: every allocation or registration it runs through is asked for its end, as
+// the first and the last may be page-locked and what lies between them not.
 static double* mapped_address(const double* p, size_t n) {
-  if (!p || reinterpret_cast<size_t>(p) % sizeof(double)) return nullptr;
-  cudaPointerAttributes a, b;
-  if (cudaPointerGetAttributes(&a, p) || cudaPointerGetAttributes(&b, p + n - 1)) {
-    cudaGetLastError();
-    return nullptr;
+  typedef CUresult (*RangeFn)(void*, CUpointer_attribute, CUdeviceptr);
+  static const RangeFn attribute = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &q) ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<RangeFn>(fn);
+  }();
+  if (!p || !attribute || reinterpret_cast<size_t>(p) % sizeof(double)) return nullptr;
+  const char *begin = reinterpret_cast<const char*>(p), *end = begin + sizeof(double) * n, *at = begin;
+  char* dev = nullptr;
+  while (at < end) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, at)) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+    char* const d = static_cast<char*>(a.devicePointer);
+    if (at == begin) dev = d;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr here = reinterpret_cast<CUdeviceptr>(d);
+    if (d - dev != at - begin || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, here) ||
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, here) || start + size <= here)
+      return nullptr;
+    at += start + size - here;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-  double* d = static_cast<double*>(a.devicePointer);
-  return static_cast<double*>(b.devicePointer) == d + n - 1 ? d : nullptr;
+  return reinterpret_cast<double*>(dev);
 }
 
 int ci_get_state(ci_solver* s, double* x, double* v, double* mass, float* sigma, float* epbar,
