@@ -1343,51 +1343,46 @@ int ci_get_state(ci_solver* s, double* x, double* v, double* mass, float* sigma,
       CI_CUDA(cudaMemcpyAsync(v, s->d_vc.p, sizeof(double) * 3 * (size_t)N, cudaMemcpyDeviceToHost,
                               s->stream));
   }
-  std::vector<float> hm, hep;
-  std::vector<float4> hsa;
-  std::vector<float2> hsb;
-  std::vector<unsigned char> hc;
-  if (mass) {
-    hm.resize(N);
-    CI_CUDA(cudaMemcpyAsync(hm.data(), s->d_mass.p, sizeof(float) * N, cudaMemcpyDeviceToHost,
+  // (plain arrays: a vector would be cleared first)
+  const size_t Q = (size_t)E * nq;
+  std::unique_ptr<float[]> hm(mass ? new float[N] : nullptr), hep(epbar ? new float[Q] : nullptr);
+  std::unique_ptr<float4[]> hsa(sigma ? new float4[Q] : nullptr);
+  std::unique_ptr<float2[]> hsb(sigma ? new float2[Q] : nullptr);
+  std::unique_ptr<unsigned char[]> hc(contact ? new unsigned char[N] : nullptr);
+  if (mass)
+    CI_CUDA(cudaMemcpyAsync(hm.get(), s->d_mass.p, sizeof(float) * N, cudaMemcpyDeviceToHost,
+                            s->stream));
+  if (sigma) {
+    CI_CUDA(cudaMemcpyAsync(hsa.get(), s->d_sig_a.p, sizeof(float4) * Q, cudaMemcpyDeviceToHost,
+                            s->stream));
+    CI_CUDA(cudaMemcpyAsync(hsb.get(), s->d_sig_b.p, sizeof(float2) * Q, cudaMemcpyDeviceToHost,
                             s->stream));
   }
+  if (epbar)
+    CI_CUDA(cudaMemcpyAsync(hep.get(), s->d_epbar.p, sizeof(float) * Q, cudaMemcpyDeviceToHost,
+                            s->stream));
+  if (contact)
+    CI_CUDA(cudaMemcpyAsync(hc.get(), s->d_contact.p, N, cudaMemcpyDeviceToHost, s->stream));
+  CI_CUDA(cudaStreamSynchronize(s->stream));
+  const int* const node = P.node_orig.data();
+  const int* const elem = P.elem_orig.data();
+  if (mass)
+    for (int i = 0; i < N; i++) mass[node[i]] = hm[i];
+  if (contact)
+    for (int i = 0; i < N; i++) contact[node[i]] = hc[i];
   if (sigma) {
-    hsa.resize((size_t)E * nq);
-    hsb.resize((size_t)E * nq);
-    CI_CUDA(cudaMemcpyAsync(hsa.data(), s->d_sig_a.p, sizeof(float4) * hsa.size(),
-                            cudaMemcpyDeviceToHost, s->stream));
-    CI_CUDA(cudaMemcpyAsync(hsb.data(), s->d_sig_b.p, sizeof(float2) * hsb.size(),
-                            cudaMemcpyDeviceToHost, s->stream));
+    const float4* a = hsa.get();
+    const float2* b = hsb.get();
+    for (int pe = 0; pe < E; pe++) {
+      float* d = sigma + 6 * (size_t)elem[pe] * nq;
+      for (int q = 0; q < nq; q++, a++, b++, d += 6) {
+        d[0] = a->x; d[1] = a->y; d[2] = a->z; d[3] = a->w; d[4] = b->x; d[5] = b->y;
+      }
+    }
   }
   if (epbar) {
-    hep.resize((size_t)E * nq);
-    CI_CUDA(cudaMemcpyAsync(hep.data(), s->d_epbar.p, sizeof(float) * hep.size(),
-                            cudaMemcpyDeviceToHost, s->stream));
-  }
-  if (contact) {
-    hc.resize(N);
-    CI_CUDA(cudaMemcpyAsync(hc.data(), s->d_contact.p, N, cudaMemcpyDeviceToHost, s->stream));
-  }
-  CI_CUDA(cudaStreamSynchronize(s->stream));
-  if (mass || contact)
-    for (int i = 0; i < N; i++) {
-      const int n = P.node_orig[i];
-      if (mass) mass[n] = hm[i];
-      if (contact) contact[n] = hc[i];
-    }
-  for (int pe = 0; pe < E; pe++) {
-    const int oe = P.elem_orig[pe];
-    for (int q = 0; q < nq; q++) {
-      const size_t qi = (size_t)pe * nq + q, o = (size_t)oe * nq + q;
-      if (sigma) {
-        const float4 a = hsa[qi];
-        const float2 b = hsb[qi];
-        float* d = sigma + 6 * o;
-        d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w; d[4] = b.x; d[5] = b.y;
-      }
-      if (epbar) epbar[o] = hep[qi];
-    }
+    const float* e = hep.get();
+    for (int pe = 0; pe < E; pe++, e += nq) std::copy(e, e + nq, epbar + (size_t)elem[pe] * nq);
   }
   return CI_OK;
 }
