@@ -468,9 +468,12 @@ def study(cfg: Config, plain_sample: int = 4, audit_fail_fraction: float = 0.1) 
     out = {"config": dataclasses.asdict(cfg), "mesh": {"elements": mesh.num_elements,
                                                        "nodes": mesh.num_nodes}}
     # tile shapes for big batches (training and evaluation runs) and for fallback-sized
-    # ones, each picked by the autotuner on a batch of that size (one-off)
+    # ones, each picked by the autotuner on a batch of that size (one-off).  The re-runs are the
+    # audited share and some 3 % flagged: for a shape, fewer runs than it was picked for never
+    # take longer, more can need a second round of CTAs (picked for 36 runs, 87 ms, 44 took 129;
+    # picked for 47, 92.1)
     t0 = time.perf_counter()
-    n_fb = max(1, int(math.ceil((cfg.audit_fraction + 0.02) * cfg.n_test)))
+    n_fb = max(1, int(math.ceil((cfg.audit_fraction + 0.04) * cfg.n_test)))
     shape_big = tune_shape(ptr[:min(len(ptr), 256)], cfg, mesh)
     shape_fb = tune_shape(pte[:n_fb], cfg, mesh)
     out["tuning"] = {"big": shape_big, "fallback": shape_fb, "fallback_batch": n_fb,
