@@ -87,13 +87,17 @@ __global__ void __launch_bounds__(256) k_mse_loss(const float* Y, const float* T
   if (lane == 0) part[w] = s[0];
 }
 
-// The passes over a [rows x cols] gradient between two products, CB columns and all rows per
-// CTA of 8 CB threads (thread: column tx, row group g): the value of entry (r, c) from `value`,
-// its BF16 copy in row order (vb, may be null) and transposed (vT, may be null), and the column
-// sums (group g of 8 sums rows r = g, g + 8, ... in order, then the 8 partial sums in group
-// order).  Products and sums are rounded one by one.  What bounds it is latency: 32 rows of a
-// thread are in flight at once (256 x 5,120, cold under a profiler: 8 behind branches about 25 us,
-// 14.4 so), and narrow gradients take 8 columns per CTA.
+// The passes over a [rows x cols] gradient between two products, CB columns and kPassRows rows
+// per CTA of 8 CB threads (thread: column tx, row group g): the value of entry (r, c) from
+// `value`, its BF16 copy in row order (vb, may be null) and transposed (vT, may be null), and the
+// column sums (group g of 8 sums rows r = g, g + 8, ... in order, then the 8 partial sums in group
+// order), those of the blocks of rows one after the other in colsum.  Products and sums are
+// rounded one by one.  What bounds it is latency: 32 rows of a thread are in flight at once (256 x
+// 5,120, cold under a profiler: 8 behind branches about 25 us, 14.4 so), narrow gradients take 8
+// columns per CTA, and tall ones several CTAs a column (gradients of 60,000 rows, 40 -> 64 -> 64 ->
+// 64: 2.50 ms with one CTA over all rows, 1.01 so).
+constexpr int kPassRows = 16384;
+
 template <int CB, class Value>
 __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* vT, float* colsum,
                                             Value value) {
@@ -104,16 +108,17 @@ __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* 
   __shared__ float part[8][CB];
   const int tx = threadIdx.x % CB, g = threadIdx.x / CB;
   const int c0 = blockIdx.x * CB, c = c0 + tx;
+  const int begin = blockIdx.y * kPassRows, end = min(rows, begin + kPassRows);
   float s = 0.f;
-  for (int r0 = 0; r0 < rows; r0 += TR) {
+  for (int r0 = begin; r0 < end; r0 += TR) {
     // (indices past the end load the last entry, so that no branch holds a load back)
     float v[U];
 #pragma unroll
-    for (int i = 0; i < U; i++) v[i] = value(min(r0 + g + 8 * i, rows - 1), min(c, cols - 1));
+    for (int i = 0; i < U; i++) v[i] = value(min(r0 + g + 8 * i, end - 1), min(c, cols - 1));
 #pragma unroll
     for (int i = 0; i < U; i++) {
       const int r = r0 + g + 8 * i;
-      if (r < rows && c < cols) {
+      if (r < end && c < cols) {
         s = __fadd_rn(s, v[i]);
         const bf16 h = __float2bfloat16(v[i]);
         if (vb) vb[(size_t)r * cols + c] = h;
@@ -124,7 +129,7 @@ __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* 
       __syncthreads();
       for (int i = threadIdx.x; i < CB * TR; i += 8 * CB) {
         const int k = i / TR, r = i % TR;
-        if (c0 + k < cols && r0 + r < rows) vT[(size_t)(c0 + k) * rows + r0 + r] = tile[k][r];
+        if (c0 + k < cols && r0 + r < end) vT[(size_t)(c0 + k) * rows + r0 + r] = tile[k][r];
       }
       __syncthreads();
     }
@@ -134,8 +139,19 @@ __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* 
   if (g == 0 && c < cols) {
     float t = part[0][tx];
     for (int k = 1; k < 8; k++) t += part[k][tx];
-    colsum[c] = t;
+    colsum[(size_t)blockIdx.y * cols + c] = t;
   }
+}
+
+// gb = the sums of the blocks of rows, in order
+__global__ void k_add_colsums(const float* colsum, int blocks, int cols, float* gb) {
+  ci::pdl_next();
+  ci::pdl_wait();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  float s = colsum[c];
+  for (int b = 1; b < blocks; b++) s = __fadd_rn(s, colsum[(size_t)b * cols + c]);
+  gb[c] = s;
 }
 
 // dY = scale (Y - T) (scale = 2 / (rows * cols)) for row r, whose targets are row idx[r] of T
@@ -364,6 +380,7 @@ struct ci_mlp {
   DBuf<bf16> Xb, H1b, H2b, dYb, dZ2b, dZ1b;
   DBuf<bf16> H1bT, H2bT, dYbT, dZ2bT, dZ1bT;  // transposes [cols x rows] for the weight gradients
   DBuf<double> part;
+  DBuf<float> colpart;  // column sums by blocks of kPassRows rows, where there are several
   DBuf<int> idx;
 };
 
@@ -389,6 +406,7 @@ int ensure_cap(ci_mlp* M, int rows) {
   CM_CUDA(M->dZ2bT.alloc(r * M->H));
   CM_CUDA(M->dZ1bT.alloc(r * M->H));
   CM_CUDA(M->part.alloc(r * nb(M->n_out)));
+  CM_CUDA(M->colpart.alloc(rows > kPassRows ? (r + kPassRows - 1) / kPassRows * std::max(M->H, M->n_out) : 0));
   CM_CUDA(M->idx.alloc(r));
   M->cap = rows;
   return CI_OK;
@@ -458,26 +476,35 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
   // layer 3: gW3 = H2^T dY as (H2^T) (dY^T)^T
   const float scale = 2.0f / (float)ny;
   const bool wide = M->n_out > 2048;
+  const unsigned blocks = (rows + kPassRows - 1) / kPassRows;
+  auto sums = [&](float* gb) { return blocks > 1 ? M->colpart.p : gb; };
+  auto add_sums = [&](int cols, float* gb) {
+    return blocks > 1 ? ci::launch_pdl(k_add_colsums, nb(cols), 256, 0, st, M->colpart.p, (int)blocks, cols, gb)
+                      : cudaSuccess;
+  };
   CM_CUDA(ci::launch_pdl(wide ? k_mse_grad<32> : k_mse_grad<8>,
-                         wide ? (M->n_out + 31) / 32 : (M->n_out + 7) / 8, wide ? 256 : 64, 0, st,
-                         M->Y.p, T, idx, rows, M->n_out, scale, M->dYb.p, M->dYbT.p, gb3));
+                         dim3(wide ? (M->n_out + 31) / 32 : (M->n_out + 7) / 8, blocks), wide ? 256 : 64,
+                         0, st, M->Y.p, T, idx, rows, M->n_out, scale, M->dYb.p, M->dYbT.p, sums(gb3)));
+  CM_CUDA(add_sums(M->n_out, gb3));
   CM_OK(gemm(M, M->H2bT.p, rows, 0, M->dYbT.p, rows, 1, gW3, M->n_out, nullptr, M->H, M->n_out,
              rows, 0.f, nullptr, 0, st));
   CM_OK(gemm(M, M->dYb.p, M->n_out, 0, W3, M->n_out, 1, M->dH2.p, M->H, nullptr, rows, M->H,
              M->n_out, 0.f, nullptr, 0, st));
   // layer 2: gW2 = H1^T dZ2 as (H1^T) (dZ2^T)^T; Z2 holds tanh(Z2) = H2 (the GEMM wrote the
   // activated values)
-  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, (M->H + 7) / 8, 64, 0, st, M->dH2.p, M->Z2.p, rows, M->H, M->dZ2b.p,
-                                               M->dZ2bT.p, gb2));
+  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH2.p, M->Z2.p,
+                         rows, M->H, M->dZ2b.p, M->dZ2bT.p, sums(gb2)));
+  CM_CUDA(add_sums(M->H, gb2));
   CM_OK(gemm(M, M->H1bT.p, rows, 0, M->dZ2bT.p, rows, 1, gW2, M->H, nullptr, M->H, M->H, rows, 0.f,
              nullptr, 0, st));
   CM_OK(gemm(M, M->dZ2b.p, M->H, 0, W2, M->H, 1, M->dH1.p, M->H, nullptr, rows, M->H, M->H, 0.f,
              nullptr, 0, st));
   // layer 1
   const bool small = M->n_in < 16;
-  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, (M->H + 7) / 8, 64, 0, st, M->dH1.p, M->Z1.p, rows, M->H,
-                                               small ? nullptr : M->dZ1b.p,
-                                               small ? M->dZ1bT.p : nullptr, gb1));
+  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH1.p, M->Z1.p,
+                         rows, M->H, small ? nullptr : M->dZ1b.p, small ? M->dZ1bT.p : nullptr,
+                         sums(gb1)));
+  CM_CUDA(add_sums(M->H, gb1));
   if (small) {
     CM_CUDA(ci::launch_pdl(k_layer1_wgrad, nb(32LL * M->n_in * M->H), 256, 0, st, X, idx, M->dZ1bT.p, rows, M->n_in,
                                                                M->H, gW1));
