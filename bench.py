@@ -349,7 +349,8 @@ def run_ours(args, rank, world):
     en = s.energy()
     # fused path: one step kernel per step + the end-of-call completion per window; task
     # kernel: one launch per window
-    launches = (1 if sk == 2 else s.launches_per_step() * args.steps + 1) * len(reps)
+    launches = (1 if sk == 2 or s.debug_resident() else
+                s.launches_per_step() * args.steps + 1) * len(reps)
     s.close()
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,

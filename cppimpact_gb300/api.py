@@ -102,6 +102,7 @@ EXPORTS = {
     "ci_launches_per_step": (C.c_int, [C.c_void_p]),
     "ci_step_kernel": (C.c_int, [C.c_void_p]),
     "ci_debug_flow_stall": (C.c_int, [C.c_void_p, C.c_int, C.c_double]),
+    "ci_debug_resident": (C.c_int, [C.c_void_p, C.c_int]),
     "ci_mesh_load_inp": (C.c_int, [C.c_char_p, C.c_int, C.POINTER(CiMesh)]),
     "ci_mesh_free": (None, [C.POINTER(CiMesh)]),
     "ci_plan_stats": (C.c_int, [C.POINTER(CiMesh), C.c_int, C.c_int, C.POINTER(C.c_longlong),
@@ -365,6 +366,13 @@ class Solver:
         """Test hook (ci_debug_flow_stall): the next task-kernel or resident launch never
         publishes chunk `chunk`'s progress, so its waits give up after wait_seconds."""
         check(lib().ci_debug_flow_stall(self._h, int(chunk), float(wait_seconds)))
+
+    def debug_resident(self, use: int = -1) -> bool:
+        """Whether the fused kernel holds its chunks on the GPU for all steps of a call
+        (ci_debug_resident); test hook: use=0 launches every step, use=1 allows it again."""
+        rc = lib().ci_debug_resident(self._h, int(use))
+        check(min(rc, CI_OK))
+        return rc == 1
 
 
 class Batch:

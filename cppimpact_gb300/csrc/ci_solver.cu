@@ -176,6 +176,8 @@ struct ci_solver {
   DBuf<float4> d_res_halo;  // [2][S]
   DBuf<int> d_res_abort;
   unsigned res_tag = 1;
+  bool launches_only = false;  // test hook
+  bool resident() const { return res.kernel && !launches_only; }
   bool xc_stale = true;  // X changed since d_Xc was uploaded
   // nodal strain/stress output: last element (caller order) of every node, and the plan
   // position of every caller element (built on first use)
@@ -786,7 +788,7 @@ int enqueue_steps(ci_solver* s, int n) {
     s->steps_done += n;
     return CI_OK;
   }
-  if (s->res.kernel) {
+  if (s->resident()) {
     CI_CUDA(enqueue_resident(s, n));
     s->steps_done += n;
     return CI_OK;
@@ -1784,10 +1786,10 @@ int ci_time_kernels(ci_solver* s, int nsteps, float* out_ms) {
   std::vector<cudaEvent_t> ev(3 * nsteps);
   for (auto& e : ev) CI_CUDA(cudaEventCreate(&e));
   double te = 0, tn = 0;
-  if (s->opt.step_kernel == 2 || s->res.kernel) {
+  if (s->opt.step_kernel == 2 || s->resident()) {
     // one launch runs all the steps: out[0] = its duration per step, out[1] = 0
     CI_CUDA(cudaEventRecord(ev[0], s->stream));
-    CI_CUDA(s->res.kernel ? enqueue_resident(s, nsteps) : enqueue_flow(s, nsteps));
+    CI_CUDA(s->resident() ? enqueue_resident(s, nsteps) : enqueue_flow(s, nsteps));
     CI_CUDA(cudaEventRecord(ev[1], s->stream));
     CI_CUDA(cudaEventSynchronize(ev[1]));
     float a;
@@ -1849,7 +1851,7 @@ int ci_step_kernel(const ci_solver* s) { return s ? s->opt.step_kernel : -1; }
 
 int ci_debug_flow_stall(ci_solver* s, int chunk, double wait_seconds) {
   if (!s) return fail(CI_ERR_INVALID, "null solver");
-  if (s->opt.step_kernel != 2 && !s->res.kernel)
+  if (s->opt.step_kernel != 2 && !s->resident())
     return fail(CI_ERR_UNSUPPORTED, "the solver runs neither the task kernel nor the resident one");
   if (chunk < 0 || chunk >= s->C || !(wait_seconds > 0.0) || wait_seconds > 60.0)
     return fail(CI_ERR_INVALID, "bad chunk or wait");
@@ -1858,8 +1860,15 @@ int ci_debug_flow_stall(ci_solver* s, int chunk, double wait_seconds) {
   return CI_OK;
 }
 
+int ci_debug_resident(ci_solver* s, int use) {
+  if (!s) return fail(CI_ERR_INVALID, "null solver");
+  if (use >= 0) s->launches_only = use == 0;
+  return s->resident() ? 1 : 0;
+}
+
 int ci_launches_per_step(const ci_solver* s) {
-  // the task kernel launches once per call of any length (and per 65,536 steps)
+  // the task kernel launches once per call of any length (and per 65,536 steps), the resident
+  // form of the fused one too (and per 16,384)
   return s ? (s->opt.step_kernel == 1 ? 2 : 1) : 0;
 }
 

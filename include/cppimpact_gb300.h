@@ -325,7 +325,8 @@ int ci_time_steps(ci_solver* s, int nsteps, float* ms);
  * kernel, out[1] = node kernel. */
 int ci_time_kernels(ci_solver* s, int nsteps, float* out_ms);
 /* Kernel launches one step issues (for launch accounting; the task kernel launches once
- * per call of up to 65,536 steps). */
+ * per call of up to 65,536 steps, the resident form of the fused kernel, see
+ * ci_debug_resident, once per 16,384). */
 int ci_launches_per_step(const ci_solver* s);
 /* The step kernel a solver runs (ci_options::step_kernel with 0 resolved), -1 for NULL. */
 int ci_step_kernel(const ci_solver* s);
@@ -338,6 +339,11 @@ int ci_step_kernel(const ci_solver* s);
  * its calls fail until ci_start or ci_solve starts again.  CI_ERR_UNSUPPORTED unless the solver
  * runs one of the two. */
 int ci_debug_flow_stall(ci_solver* s, int chunk, double wait_seconds);
+
+/* Whether the fused kernel steps in its resident form (chunks stay on the GPU for all steps of
+ * a call): 1 or 0, negative for NULL.  Test hook: use = 0 makes the solver launch every step
+ * from now on, 1 lets it step resident again where its plan fits, -1 changes nothing. */
+int ci_debug_resident(ci_solver* s, int use);
 
 /* ---- mesh utilities (host only) ---- */
 /* Mesh::load_mesh (include/mesh.h:57-267): parse an Abaqus/CalculiX .inp file.
