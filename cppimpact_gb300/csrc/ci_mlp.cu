@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) k_mse_loss(const float* Y, const float* T
 // 64: 2.50 ms with one CTA over all rows, 1.01 so).
 constexpr int kPassRows = 16384;
 
-template <int CB, class Value>
+template <int CB, bool BLOCKS, class Value>
 __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* vT, float* colsum,
                                             Value value) {
   ci::pdl_next();
@@ -108,7 +108,9 @@ __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* 
   __shared__ float part[8][CB];
   const int tx = threadIdx.x % CB, g = threadIdx.x / CB;
   const int c0 = blockIdx.x * CB, c = c0 + tx;
-  const int begin = blockIdx.y * kPassRows, end = min(rows, begin + kPassRows);
+  // (BLOCKS false, one block: the arithmetic of the bounds alone cost 4 % of a training epoch)
+  const int begin = BLOCKS ? blockIdx.y * kPassRows : 0;
+  const int end = BLOCKS ? min(rows, begin + kPassRows) : rows;
   float s = 0.f;
   for (int r0 = begin; r0 < end; r0 += TR) {
     // (indices past the end load the last entry, so that no branch holds a load back)
@@ -139,7 +141,7 @@ __device__ __forceinline__ void column_pass(int rows, int cols, bf16* vb, bf16* 
   if (g == 0 && c < cols) {
     float t = part[0][tx];
     for (int k = 1; k < 8; k++) t += part[k][tx];
-    colsum[(size_t)blockIdx.y * cols + c] = t;
+    colsum[(BLOCKS ? (size_t)blockIdx.y * cols : 0) + c] = t;
   }
 }
 
@@ -156,22 +158,22 @@ __global__ void k_add_colsums(const float* colsum, int blocks, int cols, float* 
 
 // dY = scale (Y - T) (scale = 2 / (rows * cols)) for row r, whose targets are row idx[r] of T
 // (row r when idx is null): BF16 in both orders, and gb = its column sums
-template <int CB>
+template <int CB, bool BLOCKS>
 __global__ void __launch_bounds__(8 * CB) k_mse_grad(const float* __restrict__ Y,
                                                      const float* __restrict__ T,
                                                      const int* __restrict__ idx, int rows, int cols,
                                                      float scale, bf16* dYb, bf16* dYbT, float* gb) {
-  column_pass<CB>(rows, cols, dYb, dYbT, gb, [&](int r, int c) {
+  column_pass<CB, BLOCKS>(rows, cols, dYb, dYbT, gb, [&](int r, int c) {
     return __fmul_rn(scale, Y[(size_t)r * cols + c] - T[(size_t)(idx ? idx[r] : r) * cols + c]);
   });
 }
 
 // dZ = dH (1 - H^2): BF16 in row order and transposed (either may be null), and gb
-template <int CB>
+template <int CB, bool BLOCKS>
 __global__ void __launch_bounds__(8 * CB) k_tanh_back(const float* __restrict__ dH,
                                                       const float* __restrict__ H, int rows,
                                                       int cols, bf16* dZb, bf16* dZbT, float* gb) {
-  column_pass<CB>(rows, cols, dZb, dZbT, gb, [&](int r, int c) {
+  column_pass<CB, BLOCKS>(rows, cols, dZb, dZbT, gb, [&](int r, int c) {
     const size_t i = (size_t)r * cols + c;
     const float h = H[i];
     return __fmul_rn(dH[i], __fmaf_rn(-h, h, 1.f));
@@ -482,7 +484,8 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
     return blocks > 1 ? ci::launch_pdl(k_add_colsums, nb(cols), 256, 0, st, M->colpart.p, (int)blocks, cols, gb)
                       : cudaSuccess;
   };
-  CM_CUDA(ci::launch_pdl(wide ? k_mse_grad<32> : k_mse_grad<8>,
+  CM_CUDA(ci::launch_pdl(blocks > 1 ? (wide ? k_mse_grad<32, true> : k_mse_grad<8, true>)
+                                    : (wide ? k_mse_grad<32, false> : k_mse_grad<8, false>),
                          dim3(wide ? (M->n_out + 31) / 32 : (M->n_out + 7) / 8, blocks), wide ? 256 : 64,
                          0, st, M->Y.p, T, idx, rows, M->n_out, scale, M->dYb.p, M->dYbT.p, sums(gb3)));
   CM_CUDA(add_sums(M->n_out, gb3));
@@ -492,7 +495,7 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
              M->n_out, 0.f, nullptr, 0, st));
   // layer 2: gW2 = H1^T dZ2 as (H1^T) (dZ2^T)^T; Z2 holds tanh(Z2) = H2 (the GEMM wrote the
   // activated values)
-  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH2.p, M->Z2.p,
+  CM_CUDA(ci::launch_pdl(blocks > 1 ? k_tanh_back<8, true> : k_tanh_back<8, false>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH2.p, M->Z2.p,
                          rows, M->H, M->dZ2b.p, M->dZ2bT.p, sums(gb2)));
   CM_CUDA(add_sums(M->H, gb2));
   CM_OK(gemm(M, M->H1bT.p, rows, 0, M->dZ2bT.p, rows, 1, gW2, M->H, nullptr, M->H, M->H, rows, 0.f,
@@ -501,7 +504,7 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
              nullptr, 0, st));
   // layer 1
   const bool small = M->n_in < 16;
-  CM_CUDA(ci::launch_pdl(k_tanh_back<8>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH1.p, M->Z1.p,
+  CM_CUDA(ci::launch_pdl(blocks > 1 ? k_tanh_back<8, true> : k_tanh_back<8, false>, dim3((M->H + 7) / 8, blocks), 64, 0, st, M->dH1.p, M->Z1.p,
                          rows, M->H, small ? nullptr : M->dZ1b.p, small ? M->dZ1bT.p : nullptr,
                          sums(gb1)));
   CM_CUDA(add_sums(M->H, gb1));
