@@ -38,9 +38,9 @@ enum StatusBits { ST_DEGENERATE = 1u, ST_NONFINITE = 2u, ST_FLOW_TIMEOUT = 8u };
 // for every write, is written once a bit.  (20 steps of 384,000 tet4 without a finite node: 3.2
 // ms with the word in host memory alone, 0.52 in device memory alone, 0.43 so.)
 constexpr int kStatusWords = 4;
-__device__ __forceinline__ void report(unsigned int* status, unsigned int bit) {
-  if (*static_cast<volatile unsigned int*>(status) & bit) return;
-  if (atomicOr(status, bit) & bit) return;
+__device__ __forceinline__ void report(unsigned int* status, unsigned int bit) {  // or several
+  if ((*static_cast<volatile unsigned int*>(status) & bit) == bit) return;
+  if ((atomicOr(status, bit) & bit) == bit) return;
   unsigned int* const host = *reinterpret_cast<unsigned int**>(status + 2);
   if (host) atomicOr_system(host, bit);
 }
@@ -80,6 +80,7 @@ struct DevState {
   unsigned int* status;
   const ElemParams* inst_ep;  // per-instance parameters of a batched solve (else null)
 
+  __device__ __forceinline__ void flag(unsigned int bit) const { report(status, bit); }
   __device__ __forceinline__ void load(size_t q, float4& a, float2& b, float& e) const {
     a = sig_a[q];
     b = sig_b[q];
@@ -281,7 +282,7 @@ __device__ __forceinline__ void element_force_on(const ElemParams& p, const Stat
         for (int j = 0; j < 3; j++) J[3 * a + j] = fmaf(x[i][a], G[i][j], J[3 * a + j]);
     float Ji[9];
     const float detJ = inv3f(J, Ji);
-    if (!(detJ > 0.f)) report(S.status, ST_DEGENERATE);
+    if (!(detJ > 0.f)) S.flag(ST_DEGENERATE);
     const float wd = R::W * detJ;
     vol += wd;
     ve += wd;
@@ -373,8 +374,8 @@ __device__ __forceinline__ void element_force_on(const ElemParams& p, const Stat
   }
 }
 
-template <int NPE, int MODE>
-__device__ __forceinline__ void element_force(const ElemParams& p, const DevState& S, int e,
+template <int NPE, int MODE, class State>
+__device__ __forceinline__ void element_force(const ElemParams& p, const State& S, int e,
                                               const float (&x)[NPE][3], const float (&du)[NPE][3],
                                               float (&f)[NPE][3], float& wint, float& wp,
                                               float& vol) {
@@ -942,6 +943,7 @@ struct StepPoint {  // a point's state read ahead
   float2* sig_b;
   float* epbar;
   unsigned int* status;
+  __device__ __forceinline__ void flag(unsigned int bit) const { report(status, bit); }
   __device__ __forceinline__ void load(size_t, float4& sa, float2& sb, float& e) const {
     sa = a;
     sb = b;
@@ -1283,10 +1285,10 @@ __device__ __forceinline__ void tet10_rs_slot(const Tet10QP& t, const float (&Pm
 // records, the stress update from the stored stress (s4, s2: xx yy zz xy, yz xz) and
 // plastic strain ep0, which an active lane passes updated to put(), the work terms, and in
 // keep the element force on the nodes this lane owns (q, q + 4 and, for q < 2, q + 8).
-template <int MODE, class Work, class Put>
+template <int MODE, class Flag, class Work, class Put>
 __device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& t, int q,
                                            const Tile& T, const int (&ln)[10], bool act, float4 s4,
-                                           float2 s2, float ep0, unsigned* status, Work work,
+                                           float2 s2, float ep0, Flag flag, Work work,
                                            float (&keep)[3][3], Put put) {
   constexpr float W = 1.0f / 24.0f;
   float2 JG[9];
@@ -1310,7 +1312,7 @@ __device__ __forceinline__ void qp10_point(const ElemParams& ep, const Tet10QP& 
   }
   float Ji[9];
   const float detJ = inv3f(J, Ji);
-  if (act && !(detJ > 0.f)) report(status, ST_DEGENERATE);
+  if (act && !(detJ > 0.f)) flag(ST_DEGENERATE);
   const float wd = act ? W * detJ : 0.f;
   float Lg[9];
 #pragma unroll
@@ -1452,7 +1454,8 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
         if (MODE == EM_J2) wp = fmaf(hp, wdp, wp);
       }
     };
-    qp10_point<MODE>(ep, t, q, T, ln, act, s4, s2, ep0, A.status, work, keep,
+    auto flag = [&](unsigned bit) { report(A.status, bit); };
+    qp10_point<MODE>(ep, t, q, T, ln, act, s4, s2, ep0, flag, work, keep,
                      [&](float4 a4, float2 a2, float epn) {
                        A.sig_a[qi] = a4;
                        A.sig_b[qi] = a2;

@@ -144,6 +144,40 @@ struct ResidentParams {
   NodeParams np;
 };
 
+// A status bit: to the status word at once, or kept by the thread until it is done with its
+// chunk.  Which of the two leaves the better code differs.  us per step, elements' bit kept or
+// not and nodes' bit kept or not (-- neither): 34,992 tet10 8.71 with the elements' kept, 8.74
+// --, 8.90 both; 6,000 tet4 3.54 with the nodes' kept, 3.58 --, 3.56 both; mixed batch of 24 cubes
+// 81.1 ms both, 83.2 --.
+template <bool KEEP>
+__device__ __forceinline__ void res_flag(unsigned* status, unsigned& bits, unsigned bit) {
+  if (KEEP)
+    bits |= bit;
+  else
+    report(status, bit);
+}
+
+// The chunk's stress and plastic strain in shared memory.
+template <bool KEEP>
+struct ResidentState {
+  float4* sig_a;
+  float2* sig_b;
+  float* epbar;
+  unsigned* status;
+  unsigned* bits;
+  __device__ __forceinline__ void flag(unsigned bit) const { res_flag<KEEP>(status, *bits, bit); }
+  __device__ __forceinline__ void load(size_t q, float4& a, float2& b, float& e) const {
+    a = sig_a[q];
+    b = sig_b[q];
+    e = epbar[q];
+  }
+  __device__ __forceinline__ void store(size_t q, float4 a, float2 b, float e) const {
+    sig_a[q] = a;
+    sig_b[q] = b;
+    epbar[q] = e;
+  }
+};
+
 template <int NPE, int MODE, int P, bool BATCH>
 __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* sm, int ci,
                                           float (*red)[2][P / 32], ResidentParams* par) {
@@ -182,8 +216,11 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   int4* const m1 = reinterpret_cast<int4*>(p0 + 2 * L);  // own slot, received slots, element entries, 1/m
   float4* const fbuf = reinterpret_cast<float4*>(m1 + L);  // [NPE][ne] element forces
   float* const recv = reinterpret_cast<float*>(fbuf);  // [3][ns] the boundary nodes' slots, in its place
-  DevState S;
+  constexpr bool KEEP_E = BATCH || NPE == 10, KEEP_N = BATCH || NPE == 4;  // res_flag
+  unsigned bits = 0;
+  ResidentState<KEEP_E> S;
   S.status = A.status;
+  S.bits = &bits;
   S.sig_a = fbuf + resident_exchange(NPE, ne, ns) / 16;
   float2* const p1 = reinterpret_cast<float2*>(S.sig_a + NQ * ne);
   double* const sw = reinterpret_cast<double*>(p1 + 2 * L);  // the wall's push on a node in contact
@@ -336,7 +373,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
     r[1] = ep.dt * vf[0];
     r[3] = ep.dt * vf[1];
     T.p1[l].y = ep.dt * vf[2];
-    if (!finite) report(A.status, ST_NONFINITE);
+    if (!finite) res_flag<KEEP_N>(A.status, bits, ST_NONFINITE);
     if (last && l < ch.n_own)
 #pragma unroll
       for (int c = 0; c < 3; c++) A.acc[c][ch.own_begin + l] = a[c];
@@ -375,7 +412,8 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
           wint = fmaf(h, wd, wint);
           if (MODE == EM_J2) wp = fmaf(hp, wdp, wp);
         };
-        qp10_point<MODE>(ep, t10, q, T, ln, act, s4, s2, ep0, A.status, work, keep,
+        auto flag = [&](unsigned bit) { S.flag(bit); };
+        qp10_point<MODE>(ep, t10, q, T, ln, act, s4, s2, ep0, flag, work, keep,
                          [&](float4 a4, float2 a2, float epn) {
                            S.sig_a[qi] = a4;
                            S.sig_b[qi] = a2;
@@ -481,7 +519,10 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
       w1 += (double)b;
     }
     const bool ok = res_receive<P>(A, halo, sslot, ns, tag, recv);
-    if (!res_sync_and<P>(ok)) return false;
+    if (!res_sync_and<P>(ok)) {
+      if (bits) report(A.status, bits);
+      return false;
+    }
     for (int l = early + nd; l < L; l += P) {
       float f[3];
       total(l, f);
@@ -497,6 +538,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   if (snaps)
     for (int si = (A.step0 + n) / A.every; si < A.snap_end; si++) snapshot(si);
 
+  if (bits) report(A.status, bits);
   // ---- store the owned nodes' state, the stress and the work sums
   for (int l = tid; l < ch.n_own; l += P) {
     const int g = ch.own_begin + l;
