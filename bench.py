@@ -309,7 +309,7 @@ def run_ours(args, rank, world):
     kname = {0: "k_step (fused element force + J2 + assembly + node update)",
              1: "k_elem (element force + J2 + colour assembly)",
              2: "k_flow_qp10 (persistent task kernel: node and element tasks of every step)"}
-    kname[3] = kname[0]
+    kname[3] = "k_resident (the fused step, chunks on the SMs)" if s.debug_resident() else kname[0]
     roofline = {"bound": "hbm", "kernel": kname[sk],
                 "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "peak_source": peak_src,

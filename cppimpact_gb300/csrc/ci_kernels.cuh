@@ -1410,7 +1410,6 @@ __device__ __forceinline__ void qp10_element_loop(const FusedArgs& A, const Elem
   const DevPlan& P = A.P;
   const int q = tid & 3;
   const Tet10QP t = tet10_qp(q);
-  const int E = P.E;
   wint = 0.f;
   wp = 0.f;
   constexpr int EPW = BS / 4;  // elements per window
@@ -2211,7 +2210,6 @@ __global__ void __launch_bounds__(256) k_node_init(NodeArrays A, NodeParams p_ar
   if (!finite) report(A.status, ST_NONFINITE);
 }
 
-// Adds n to the batched step counter (after each captured block of steps).
 // conn_local [10][E] and the colours as records (DevPlan::conn8, conn2).
 static __global__ void k_pack_conn10(const uint16_t* conn, const uint8_t* color, int E, uint4* c8,
                                      uint2* c2) {
@@ -2225,6 +2223,7 @@ static __global__ void k_pack_conn10(const uint16_t* conn, const uint8_t* color,
   c2[e] = make_uint2(w[4], color[e]);
 }
 
+// Adds n to the batched step counter (after each captured block of steps).
 static __global__ void k_tick(int* step_ctr, int n) { *step_ctr += n; }
 
 // Peak |u| over a node range since the last reset (one FP32 max per block, fixed order).

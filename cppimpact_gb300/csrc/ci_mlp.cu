@@ -477,6 +477,8 @@ int backward(ci_mlp* M, const float* X, const float* T, const int* idx, int rows
   }
   // layer 3: gW3 = H2^T dY as (H2^T) (dY^T)^T
   const float scale = 2.0f / (float)ny;
+  // (an epoch of 4,096 rows, 8 and 32 columns per CTA: 1,536 outputs 1,114 and 1,132 us, 2,048 1,124 and
+  // 1,123, 2,560 1,172 and 1,154, 5,120 1,429 and 1,315)
   const bool wide = M->n_out > 2048;
   const unsigned blocks = (rows + kPassRows - 1) / kPassRows;
   auto sums = [&](float* gb) { return blocks > 1 ? M->colpart.p : gb; };

@@ -37,8 +37,7 @@
 // Stored stress, connectivity, entry and slot lists are in shared memory too (121 B per local
 // node, 112 B per tet4 and 312 B per tet10 element, 4 to 16 B per slot: up to about 58 tet10
 // or 270 tet4 elements per chunk at four CTAs per SM).  Read through the caches instead,
-// for larger chunks, they made it no faster than a launch per step (48,000 tet10: 15.2
-// against 15.1).
+// for larger chunks, they made it slower than a launch per step (48,000 tet10: 15.2 and 14.5).
 #pragma once
 #include "ci_resident.h"
 

@@ -682,8 +682,8 @@ cudaError_t enqueue_flow(ci_solver* s, int n) {
 // chunks the GPU holds all at once with their tables on chip, whatever the number of steps:
 // one launch instead of a graph of steps and the completion kernel (a call of one step and
 // the state read back, 6,000 tet4: 60.9 -> 52.1 us; times per step in ci_resident.cuh).
-// Larger plans keep a launch per step: 48,000 tet10 took 15.2 us per step resident with
-// the tables read through the caches against 15.1, 86,400 tet10 20.1 against 20.2.
+// Larger plans keep a launch per step: with the tables read through the caches 48,000 tet10
+// took 15.2 us per step resident, 86,400 20.1, by launches now 14.5 and 16.7.
 int setup_resident(ci_solver* s) {
   const ci::Plan& P = s->plan;
   if (s->npe == 10 && s->opt.elem_lanes != 4) return CI_OK;
@@ -1139,9 +1139,10 @@ int ci_create(const ci_mesh* mesh, const ci_material* mat, const ci_wall* wall,
   if (s->opt.step_kernel == 0) {
     // automatic: the task kernel when the chunks of a four-lane tet10 mesh need more than
     // 0.8 of a round of the fused kernel's resident CTAs -- meshes whose chunks are cut by
-    // the local-node budget -- else the fused kernel (measured: the 604,800-element shell,
-    // 1.9 rounds, 98.0 against 121.9 us per step; half of it, 0.95 rounds, 58.1 against
-    // 63.4; the quad cube, 0.66 rounds of small chunks, 19.4 against 14.9).
+    // the local-node budget -- else the fused kernel.  us per step, task against fused kernel,
+    // by rounds of CTAs: 604,800-element shell, 1.9, 94.4 and 122.3; parts of it, 0.94, 56.3 and
+    // 60.6, 0.81, 53.1 and 51.3, 0.68, 49.4 and 45.8; cubes of 384,000, 279,936 and 196,608, 1.1, 70.9
+    // and 97.7, 0.78, 61.6 and 61.4, 0.67, 50.3 and 34.0.
     s->opt.step_kernel = 3;
     if (s->npe == 10 && s->opt.elem_lanes == 4 && s->opt.block_threads == 128) {
       int per_sm = 0, sms = 0;

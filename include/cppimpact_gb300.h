@@ -262,11 +262,11 @@ int ci_batch_run_peaks(ci_batch* b, int every, int max_snaps, float* peak_disp, 
  * multiply-adds (M N K <= 1048576) outside the form A B^T with 16-byte rows run on the CUDA
  * cores, one thread per output summing the BF16 products in FP32 in K order; all others on
  * the tensor cores.  A workspace per device and stream (grown by cudaMalloc on first need,
- * at most 32 streams' kept per device) holds the FP32 partial sums of products whose K is
- * cut across CTAs, added in a fixed order so that results are deterministic, and aligned
+ * at most 32 streams' and 512 MB kept per device) holds the FP32 partial sums of products whose
+ * K is cut across CTAs, added in a fixed order so that results are deterministic, and aligned
  * copies (at most 256 MB per call) of operands that the tensor kernels cannot read in
  * place; calls on different streams may run concurrently.  While `stream` is being captured
- * no copies are made. */
+ * no copies are made, and the workspace that the captured calls use is kept for good. */
 int ci_gemm_bf16(const void* A, int lda, int transA, const void* B, int ldb, int transB, float* C,
                  int ldc, void* C_bf16, int M, int N, int K, float alpha, float beta,
                  const float* bias, int activation, int* d_error, void* stream);
