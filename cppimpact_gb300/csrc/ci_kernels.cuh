@@ -44,6 +44,11 @@ __device__ __forceinline__ void report(unsigned int* status, unsigned int bit) {
   unsigned int* const host = *reinterpret_cast<unsigned int**>(status + 2);
   if (host) atomicOr_system(host, bit);
 }
+// The same as a call: where a node's update ends, beside an element loop that needs the
+// registers (604,800 tet10 93.37 us per step inlined, 93.20 so; in the element loop itself 94.0).
+static __device__ __noinline__ void report_call(unsigned int* status, unsigned int bit) {
+  report(status, bit);
+}
 
 struct DevPlan {
   const ChunkInfo* chunks;
@@ -530,7 +535,7 @@ __global__ void __launch_bounds__(256) k_node(NodeArrays A, NodeParams p) {
     if (!INIT) A.u[k][n] = un[k];
     if (STORE_ACC) A.acc[k][n] = (float)a[k];
   }
-  if (!finite) report(A.status, ST_NONFINITE);
+  if (!finite) report_call(A.status, ST_NONFINITE);
 }
 
 // ---------------------------------------------------------------------------
@@ -687,7 +692,7 @@ __device__ __forceinline__ void store_node(const FusedArgs& A, double* const (&u
     finite = finite && isfinite(vf[k]);
     if (store_acc) A.acc[k][g] = a[k];
   }
-  if (!finite) report(A.status, ST_NONFINITE);
+  if (!finite) report_call(A.status, ST_NONFINITE);
   const unsigned char flag = in_contact ? 3 : (old & 2);
   if (flag != old) A.contact[g] = flag;
 }
@@ -2207,7 +2212,7 @@ __global__ void __launch_bounds__(256) k_node_init(NodeArrays A, NodeParams p_ar
     A.acc[k][n] = (float)ad[k];
   }
   A.contact[n] = flag;
-  if (!finite) report(A.status, ST_NONFINITE);
+  if (!finite) report_call(A.status, ST_NONFINITE);
 }
 
 // conn_local [10][E] and the colours as records (DevPlan::conn8, conn2).
