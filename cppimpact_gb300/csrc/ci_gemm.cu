@@ -1148,8 +1148,8 @@ __global__ void __launch_bounds__(128) k_stream_reduce(const StreamArgs P, int B
 // Operand copies that TMA can address: out [copies][rows][ld] with ld a multiple of 8 (the
 // columns up to ld zero), copy c shifted by delta[c] zeros; the source [rows x K], or
 // [K x rows] when trans.  32 x 32 tiles through shared memory, so both sides are read and
-// written along their rows.  Blocks of 32 rows x 128 columns are counted on grid.x, whose
-// limit neither many rows nor many columns reach.
+// written along their rows.  A block has 128 columns and every gridDim.y-th 32 rows (grid.y counts
+// to 65,535 only).
 struct PackArgs {
   const __nv_bfloat16* in;
   __nv_bfloat16* out;
@@ -1161,27 +1161,28 @@ __global__ void __launch_bounds__(256) k_pack_bf16(const PackArgs P) {
   ci::pdl_next();
   ci::pdl_wait();
   __shared__ __nv_bfloat16 tile[32][34];
-  const int d = P.delta[blockIdx.y];
+  const int d = P.delta[blockIdx.z];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const __nv_bfloat16 zero = __float2bfloat16(0.f);
-  __nv_bfloat16* out = P.out + (size_t)blockIdx.y * P.rows * P.ld;
-  const int nx = (P.ld + 127) / 128, bx = blockIdx.x % nx;
-  const int r0 = (blockIdx.x / nx) * 32;
-  for (int x0 = bx * 128; x0 < min(P.ld, (bx + 1) * 128); x0 += 32) {
-    if (P.trans) {
-      for (int k = ty; k < 32; k += 8) {
-        const int x = x0 + k - d, r = r0 + tx;
-        tile[k][tx] = (x >= 0 && x < P.K && r < P.rows) ? P.in[(size_t)x * P.ld_in + r] : zero;
-      }
-      __syncthreads();
-      for (int k = ty; k < 32; k += 8)
-        if (r0 + k < P.rows && x0 + tx < P.ld) out[(size_t)(r0 + k) * P.ld + x0 + tx] = tile[tx][k];
-      __syncthreads();
-    } else {
-      for (int k = ty; k < 32; k += 8) {
-        const int x = x0 + tx - d, r = r0 + k;
-        if (r < P.rows && x0 + tx < P.ld)
-          out[(size_t)r * P.ld + x0 + tx] = (x >= 0 && x < P.K) ? P.in[(size_t)r * P.ld_in + x] : zero;
+  __nv_bfloat16* out = P.out + (size_t)blockIdx.z * P.rows * P.ld;
+  const int x_end = min(P.ld, (int)(blockIdx.x + 1) * 128);
+  for (int r0 = blockIdx.y * 32; r0 < P.rows; r0 += gridDim.y * 32) {
+    for (int x0 = blockIdx.x * 128; x0 < x_end; x0 += 32) {
+      if (P.trans) {
+        for (int k = ty; k < 32; k += 8) {
+          const int x = x0 + k - d, r = r0 + tx;
+          tile[k][tx] = (x >= 0 && x < P.K && r < P.rows) ? P.in[(size_t)x * P.ld_in + r] : zero;
+        }
+        __syncthreads();
+        for (int k = ty; k < 32; k += 8)
+          if (r0 + k < P.rows && x0 + tx < P.ld) out[(size_t)(r0 + k) * P.ld + x0 + tx] = tile[tx][k];
+        __syncthreads();
+      } else {
+        for (int k = ty; k < 32; k += 8) {
+          const int x = x0 + tx - d, r = r0 + k;
+          if (r < P.rows && x0 + tx < P.ld)
+            out[(size_t)r * P.ld + x0 + tx] = (x >= 0 && x < P.K) ? P.in[(size_t)r * P.ld_in + x] : zero;
+        }
       }
     }
   }
@@ -1581,7 +1582,7 @@ bool pack_operands(Operands* op, char* at, cudaStream_t st) {
   auto run = [&](PackArgs& a, int copies) {
     a.out = reinterpret_cast<__nv_bfloat16*>(at);
     at += align256(sizeof(__nv_bfloat16) * (size_t)copies * a.rows * a.ld);
-    const dim3 grid((unsigned)((a.ld + 127) / 128) * (unsigned)((a.rows + 31) / 32), copies);
+    const dim3 grid((a.ld + 127) / 128, std::min((a.rows + 31) / 32, 65535), copies);
     return ci::launch_pdl(k_pack_bf16, grid, 256, 0, st, a) == cudaSuccess;
   };
   if (op->do_a) {
