@@ -144,10 +144,10 @@ struct ResidentParams {
 };
 
 // A status bit: to the status word at once, or kept by the thread until it is done with its
-// chunk.  Which of the two leaves the better code differs.  us per step, elements' bit kept or
-// not and nodes' bit kept or not (-- neither): 34,992 tet10 8.71 with the elements' kept, 8.74
-// --, 8.90 both; 6,000 tet4 3.54 with the nodes' kept, 3.58 --, 3.56 both; mixed batch of 24 cubes
-// 81.1 ms both, 83.2 --.
+// chunk.  Which of the two leaves the better code differs.  us per step with the elements' bit
+// kept, the nodes', both, neither: 34,992 tet10 8.71, 8.95, 8.90, 8.74; 6,000 tet4 (CTAs of 64
+// threads) 3.60, 3.52, 3.55, 3.56; 48,000 tet4 (128) 5.02, 4.96, 4.99, 4.89; mixed batch of 24 cubes
+// both 81.1 ms, neither 83.2.
 template <bool KEEP>
 __device__ __forceinline__ void res_flag(unsigned* status, unsigned& bits, unsigned bit) {
   if (KEEP)
@@ -215,7 +215,7 @@ __device__ __forceinline__ bool res_chunk(const ResidentArgs& A, unsigned char* 
   int4* const m1 = reinterpret_cast<int4*>(p0 + 2 * L);  // own slot, received slots, element entries, 1/m
   float4* const fbuf = reinterpret_cast<float4*>(m1 + L);  // [NPE][ne] element forces
   float* const recv = reinterpret_cast<float*>(fbuf);  // [3][ns] the boundary nodes' slots, in its place
-  constexpr bool KEEP_E = BATCH || NPE == 10, KEEP_N = BATCH || NPE == 4;  // res_flag
+  constexpr bool KEEP_E = BATCH || NPE == 10, KEEP_N = BATCH || (NPE == 4 && P == 64);  // res_flag
   unsigned bits = 0;
   ResidentState<KEEP_E> S;
   S.status = A.status;
